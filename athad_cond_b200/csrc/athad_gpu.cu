@@ -154,12 +154,12 @@ athad_status athad_create(const athad_grid* grid, const athad_params* params, at
     c->polar_passes = (int*)take((size_t)jm * sizeof(int));
     c->turb_lev = (TurbLevel*)take((size_t)im * sizeof(TurbLevel));
     if (params->precision == ATHAD_PRECISION_MIXED) {
-        const size_t fb = L.field_elems * sizeof(float);
-        for (int n = 0; n < kNY; n++) c->mA[n] = (float*)take(fb);
-        for (int n = 0; n < kNY; n++) c->mB[n] = (float*)take(fb);
-        for (int n = 0; n < kNY; n++) c->mK[n] = (float*)take(fb);
-        for (int n = 0; n < kNY; n++) c->mYn[n] = (float*)take(fb);
-        for (int f = 0; f < ATHAD_MF_COUNT; f++) c->mF[f] = (float*)take(fb);
+        const size_t fb = L.field_elems * sizeof(float4);
+        for (int n = 0; n < kMixedGroups; n++) c->mA[n] = (float4*)take(fb);
+        for (int n = 0; n < kMixedGroups; n++) c->mB[n] = (float4*)take(fb);
+        for (int n = 0; n < kMixedGroups; n++) c->mK[n] = (float4*)take(fb);
+        for (int n = 0; n < kMixedGroups; n++) c->mYn[n] = (float4*)take(fb);
+        for (int f = 0; f < kMixedForcing; f++) c->mF[f] = (float4*)take(fb);
         c->geof = (GeoF*)take((size_t)im * jm * sizeof(GeoF));
     }
     if ((size_t)(q - c->slab) > L.bytes) {
@@ -549,7 +549,8 @@ athad_status athad_rk4_step(athad_ctx* ctx, const athad_step_scalars* s)
         g.nontrad = p.coriolis_nontrad;
         g.flags = s->write_diagnostics & 3;
         for (int n = 0; n < kNY; n++) {
-            if (ctx->p.precision == ATHAD_PRECISION_MIXED) g.Y32[n] = ctx->mA[n];
+            const int G = rk4m_field_group(n), q = rk4m_field_place(n);
+            if (ctx->p.precision == ATHAD_PRECISION_MIXED) g.Y32[n] = (const float*)ctx->mA[G] + q;
             else g.Y64[n] = ctx->stA[n];
         }
         launch_rhs_diagnostics(g, ctx->stream);
@@ -636,10 +637,12 @@ void athad::mixed_args(athad_ctx* ctx, const athad_step_scalars* s, RK4MArgs& a)
     for (int n = 0; n < kNY; n++) {
         a.Y[n] = ctx->field[ATHAD_T + n];
         a.Yn[n] = ctx->field[ATHAD_TN + n];
-        a.Yn32[n] = ctx->mYn[n];
-        a.K[n] = ctx->mK[n];
     }
-    for (int f = 0; f < ATHAD_MF_COUNT; f++) a.F[f] = ctx->mF[f];
+    for (int G = 0; G < kMixedGroups; G++) {
+        a.Yn32[G] = ctx->mYn[G];
+        a.K[G] = ctx->mK[G];
+    }
+    for (int f = 0; f < kMixedForcing; f++) a.F[f] = ctx->mF[f];
     double** F = ctx->field;
     a.p_dyn = F[ATHAD_P_DYN]; a.nue = F[ATHAD_NUE]; a.t_eq = F[ATHAD_T_EQ]; a.p_stat = F[ATHAD_P_STAT];
     a.r_humid = F[ATHAD_R_HUMID];
@@ -689,7 +692,7 @@ static athad_status rk4_step_mixed(athad_ctx* ctx, const athad_step_scalars* s)
     RK4MArgs a;
     mixed_args(ctx, s, a);
     for (int stage = 1; stage <= 4; stage++) {
-        for (int n = 0; n < kNY; n++) {
+        for (int n = 0; n < kMixedGroups; n++) {
             a.Yin[n] = (stage == 3) ? ctx->mB[n] : ctx->mA[n];
             a.Yout[n] = (stage == 1 || stage == 3) ? ctx->mA[n] : ctx->mB[n];
             a.Ybnd[n] = ctx->mB[n];

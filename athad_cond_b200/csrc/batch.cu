@@ -212,11 +212,11 @@ athad_status athad_batch_create(athad_ctx* const* members, int32_t n_members, co
         athad_ctx* c = members[q];
         athad_step_scalars sc{step->dt, step->diffusion_ramp, 1.0, 0, 0};
         mixed_args(c, &sc, args[q]);
-        for (int f = 0; f < kNY; f++) {
+        for (int f = 0; f < kMixedGroups; f++) {
             args[q].Yout[f] = c->mA[f];      // stage buffer A
             args[q].Ybnd[f] = c->mB[f];      // stage buffer B
-            args[q].Yn_store[f] = c->field[ATHAD_TN + f];
         }
+        for (int f = 0; f < kNY; f++) args[q].Yn_store[f] = c->field[ATHAD_TN + f];
         args[q].store_n = 1;
         BatchStep& s = steps[q];
         std::memset(&s, 0, sizeof s);

@@ -28,9 +28,9 @@ constexpr int kInternal3D = 3 * kNY + 2;
 
 inline size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// FP32 buffers of the mixed-precision RK4 step: stage A, stage B, accumulator K, level n
-// (11 each) and the packed forcing
-constexpr int kMixed32 = 4 * kNY + ATHAD_MF_COUNT;
+// float4 buffers of the mixed-precision RK4 step: stage A, stage B, accumulator K, level n
+// (three groups each) and the packed forcing
+constexpr int kMixed128 = 4 * kMixedGroups + kMixedForcing;
 
 inline Layout make_layout(const athad_grid& g, int precision)
 {
@@ -54,7 +54,7 @@ inline Layout make_layout(const athad_grid& g, int precision)
     b += round_up((size_t)g.jm * sizeof(int), 256);                                   // polar passes
     b += round_up((size_t)g.im * sizeof(TurbLevel), 256);                             // turbulence levels
     if (precision == ATHAD_PRECISION_MIXED) {
-        b += (size_t)kMixed32 * round_up(L.field_elems * sizeof(float), 256);
+        b += (size_t)kMixed128 * round_up(L.field_elems * sizeof(float4), 256);
         b += round_up((size_t)g.im * g.jm * sizeof(GeoF), 256);
     }
     L.bytes = b;
@@ -79,11 +79,11 @@ struct athad_ctx {
     double* stK[kNY] = {};
     double* src = nullptr;
     double* upload_stage = nullptr;   // im*jm*km packed doubles
-    float* mA[kNY] = {};              // mixed precision: FP32 stage buffers, accumulator,
-    float* mB[kNY] = {};              // level n and packed forcing; FP32 geometry
-    float* mK[kNY] = {};
-    float* mYn[kNY] = {};
-    float* mF[ATHAD_MF_COUNT] = {};
+    float4* mA[kMixedGroups] = {};    // mixed precision: FP32 stage buffers, accumulator,
+    float4* mB[kMixedGroups] = {};    // level n and packed forcing; FP32 geometry
+    float4* mK[kMixedGroups] = {};
+    float4* mYn[kMixedGroups] = {};
+    float4* mF[kMixedForcing] = {};
     GeoF* geof = nullptr;
     double* f2d[ATHAD_NFIELDS2D] = {};
     double* prof[ATHAD_NPROFILES] = {};

@@ -14,6 +14,10 @@ namespace athad {
 
 namespace {
 
+// values between consecutive cells: the FP32 stage buffers hold four fields per cell
+template <typename TY> constexpr int kStep = 1;
+template <> constexpr int kStep<float> = 4;
+
 template <typename TY>
 struct StarD {
     double c, ip, im, jp, jm, kp, km;
@@ -23,10 +27,11 @@ template <typename TY>
 __device__ __forceinline__ StarD<TY> star(const TY* __restrict__ F, long long c, long long sI, long long sJ)
 {
     StarD<TY> s;
-    s.c = (double)F[c];
-    s.ip = (double)F[c + sI]; s.im = (double)F[c - sI];
-    s.jp = (double)F[c + sJ]; s.jm = (double)F[c - sJ];
-    s.kp = (double)F[c + 1];  s.km = (double)F[c - 1];
+    constexpr int S = kStep<TY>;
+    s.c = (double)F[S * c];
+    s.ip = (double)F[S * (c + sI)]; s.im = (double)F[S * (c - sI)];
+    s.jp = (double)F[S * (c + sJ)]; s.jm = (double)F[S * (c - sJ)];
+    s.kp = (double)F[S * (c + 1)];  s.km = (double)F[S * (c - 1)];
     return s;
 }
 
@@ -54,8 +59,8 @@ __global__ void __launch_bounds__(128) rhs_diag_kernel(const RhsDiagArgs a)
     const double inv_rm2sinthe2 = G.inv_rm2sinthe2, cos_rm2sin = G.costhe_inv_rm2sinthe;
     const double sinthe = G.sinthe, costhe = G.costhe;
 
-    const double t_ijk = (double)ycol<TY>(a, 0)[c], u_ijk = (double)ycol<TY>(a, 1)[c], v_ijk = (double)ycol<TY>(a, 2)[c];
-    const double w_ijk = (double)ycol<TY>(a, 3)[c], c_ijk = (double)ycol<TY>(a, 4)[c];
+    const double t_ijk = (double)ycol<TY>(a, 0)[kStep<TY> * c], u_ijk = (double)ycol<TY>(a, 1)[kStep<TY> * c], v_ijk = (double)ycol<TY>(a, 2)[kStep<TY> * c];
+    const double w_ijk = (double)ycol<TY>(a, 3)[kStep<TY> * c], c_ijk = (double)ycol<TY>(a, 4)[kStep<TY> * c];
     const double u_exp = u_ijk * exp_rm, v_invrm = v_ijk * inv_rm, w_invrs = w_ijk * inv_rmsinthe;
     const double dpdr = (a.p_dyn[c + sI] - a.p_dyn[c - sI]) * a.inv_2dr;
     const double dpdthe = (a.p_dyn[c + sJ] - a.p_dyn[c - sJ]) * a.inv_2dthe;

@@ -57,8 +57,8 @@ struct RhsDiagArgs {
     const GeoIJ* geo;
     const double* t_ref;
     const double* p_dyn; const double* nue; const double* MC_v; const double* MC_w;
-    const double* Y64[11];      // the state read: FP64 (Y32[0] null) or FP32 stage buffers
-    const float* Y32[11];
+    const double* Y64[11];      // the state read: FP64 (Y32[0] null) or the FP32 stage buffers,
+    const float* Y32[11];       // four values per cell: consecutive cells four floats apart
     double* out[17];
     double inv_2dr, inv_2dthe, inv_2dphi, inv_dr2, inv_dthe2, inv_dphi2;
     double coeff_Coriolis, coeff_buoy, coeff_u_p, coeff_L, coeff_S, t_0;
@@ -77,20 +77,15 @@ struct GeoF {
     float exp_rm, exp_2_rm, sinthe, costhe, inv_rm, inv_rm2, inv_rmsinthe, inv_rm2sinthe,
           inv_rm2sinthe2, costhe_inv_rm2sinthe, two_over_rm_exp, v_metric, cos4lat, pad;
 };
-enum {
-    ATHAD_MF_P = 0,   // p_dyn (read as a stencil)
-    ATHAD_MF_NUE,     // nue
-    ATHAD_MF_QT,      // moist-convective and latent heating of t
-    ATHAD_MF_KT,      // Held-Suarez rate k_T * L_atm / u_0
-    ATHAD_MF_TEQ,     // t_eq
-    ATHAD_MF_QC,      // sources of c, cloud, ice, gr (consecutive)
-    ATHAD_MF_QCL,
-    ATHAD_MF_QI,
-    ATHAD_MF_QG,
-    ATHAD_MF_MV,      // moist-convective momentum sources of v and w
-    ATHAD_MF_MW,
-    ATHAD_MF_COUNT
-};
+constexpr int kMixedGroups = 3;    // groups of four values per cell (k_rk4m.cu)
+constexpr int kMixedForcing = 2;   // groups of packed forcing
+// group and place of field n (0 t, 1 u, 2 v, 3 w, 4 c, 5 cloud, 6 ice, 7 gr, 8 co2, 9 tke,
+// 10 dis): (u, v, w, p_dyn), (tke, dis, t, c), (cloud, ice, gr, co2)
+ATHAD_HD constexpr int rk4m_field_group(int n) { return (n >= 1 && n <= 3) ? 0 : (n >= 5 && n <= 8) ? 2 : 1; }
+ATHAD_HD constexpr int rk4m_field_place(int n)
+{
+    return (n >= 1 && n <= 3) ? n - 1 : (n >= 5 && n <= 8) ? n - 5 : n == 0 ? 2 : n == 4 ? 3 : n - 9;
+}
 struct RK4MArgs {
     Dims d;
     const GeoF* geo;
@@ -101,12 +96,12 @@ struct RK4MArgs {
     const double* p_dyn; const double* nue; const double* t_eq; const double* p_stat; const double* r_humid;
     const double* S_c; const double* S_r; const double* S_i; const double* S_s; const double* S_g; const double* S_v;
     const double* MC_t; const double* MC_q; const double* MC_v; const double* MC_w;
-    const float* Yin[11];       // FP32 stage state read (stages 2-4)
-    float* Yout[11];            // FP32 stage state written (stages 1-3)
-    float* Ybnd[11];            // stage 1: second stage buffer that receives the boundary
-    float* Yn32[11];            // FP32 time level n (written by stage 1, read by 2-3)
-    float* K[11];               // FP32 accumulator
-    float* F[ATHAD_MF_COUNT];   // packed forcing
+    const float4* Yin[kMixedGroups];   // FP32 stage state read (stages 2-4)
+    float4* Yout[kMixedGroups];        // FP32 stage state written (stages 1-3)
+    float4* Ybnd[kMixedGroups];        // stage 1: second stage buffer that receives the boundary
+    float4* Yn32[kMixedGroups];        // FP32 time level n (written by stage 1, read by 2-3)
+    float4* K[kMixedGroups];           // FP32 accumulator
+    float4* F[kMixedForcing];          // packed forcing: (MC_w, q_t, k_T, t_eq), (q_c, q_cloud, q_ice, q_gr)
     double* Yn_store[11];       // store_n: stage 4 also writes the new time level n here
     double* aux_u; double* aux_v; double* aux_w;
     double* prod; double* tke_source; double* dis_source;
