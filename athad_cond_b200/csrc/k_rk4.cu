@@ -115,48 +115,56 @@ __device__ __forceinline__ double ar(const Star& s, const RK4Args& a) { return m
 __device__ __forceinline__ double at(const Star& s, const RK4Args& a) { return minmod(s.c - s.jm, s.jp - s.c) * (2.0 * a.inv_2dthe); }
 __device__ __forceinline__ double ap(const Star& s, const RK4Args& a) { return minmod(s.c - s.km, s.kp - s.c) * (2.0 * a.inv_2dphi); }
 
-// Stage update of one field (RungeKutta_Atm_Turb.cpp:167-182, 199-209, 226-236, 253-263).
-// Field n: 0 t, 1 u, 2 v, 3 w, 4 c, 5 cloud, 6 ice, 7 gr, 8 co2, 9 tke, 10 dis.
-// single-use operands (time level n, accumulator) with the streaming hint
-// (ATHAD_RK4_STREAM_LOADS), so they do not displace the stencil fields' lines from L1:
-// 1.745 -> 1.717 ms per FP64 step at 41x181x361 (the mixed step, whose single-use operands
-// are FP32, runs 2 % slower with it and keeps plain loads)
-#ifndef ATHAD_RK4_STREAM_LOADS
-#define ATHAD_RK4_STREAM_LOADS 1
+#ifndef ATHAD_RK4_MIN_BLOCKS
+#define ATHAD_RK4_MIN_BLOCKS 4   // 128 registers per thread, 4 CTAs of 128 threads per SM
 #endif
-__device__ __forceinline__ double ld_once(const double* p)
+#ifndef ATHAD_RK4_BX
+#define ATHAD_RK4_BX 32          // CTA: BX longitudes x BY rows of one level (61x181x361: 2161 us per step with
+#endif                           // 32 x 4 at 4 CTAs; at 5, 2202 with 32 x 4, 2216 with 64 x 2, 2268 with 128 x 1)
+#ifndef ATHAD_RK4_BY
+#define ATHAD_RK4_BY 4
+#endif
+constexpr int kThreads = ATHAD_RK4_BX * ATHAD_RK4_BY;
+
+// The operands that a stage reads once per cell (the accumulator, time level n and 13 of the
+// forcing fields) come through shared memory: each thread starts the asynchronous copies of
+// its own cell's values before its first stencil load and waits for them before the first
+// stage update.  Read where they are used, they were 35 of the loads that a thread waited
+// for one after another (the accumulator's cannot pass the stores of the fields before it,
+// and 72 registers hold few loads in flight: long-scoreboard stalls 10.6 of 15.2 cycles per
+// issue); now the whole cell's DRAM traffic is in flight at once.  A thread reads only what
+// it copied, so no barrier is needed.  61x181x361 per step: 2551 -> 2161 us at 4 CTAs per SM
+// (128 registers, hardly a spill), 2202 at 5, 2439 at 3; 6 CTAs (2969) leave the stencil too
+// little L1.  Accumulator and level n alone in shared memory: 2355-2414.  16-byte copies by
+// half warps: 2195.  Asking the L2 for the tile's rows instead (k_rk4m.cu): 2770.
+constexpr int kForcingSlots = 13;   // t_eq, p_stat, r_humid, S_c, S_r, S_i, S_s, S_g, S_v, MC_t, MC_q, MC_v, MC_w
+constexpr int kSlotYn = kForcingSlots, kSlotK = kSlotYn + 11;
+static_assert(ATHAD_MC_W - ATHAD_T_EQ + 1 == kForcingSlots, "the forcing fields are consecutive in the slab");
+template <int STAGE> constexpr int kSlots = (STAGE == 1) ? kSlotK : kSlotK + 11;
+
+__device__ __forceinline__ void copy_async(double* dst, const double* src)
 {
-#if ATHAD_RK4_STREAM_LOADS
-    return __ldcs(p);
-#else
-    return __ldg(p);
-#endif
-}
-// the same for the accumulator, which the launch also writes (same thread, same cell): a
-// coherent load either way
-__device__ __forceinline__ double ld_acc(const double* p)
-{
-#if ATHAD_RK4_STREAM_LOADS
-    return __ldcs(p);
-#else
-    return *p;
-#endif
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(__cvta_generic_to_global(src)) : "memory");
 }
 
+// Stage update of one field (RungeKutta_Atm_Turb.cpp:167-182, 199-209, 226-236, 253-263).
+// Field n: 0 t, 1 u, 2 v, 3 w, 4 c, 5 cloud, 6 ice, 7 gr, 8 co2, 9 tke, 10 dis.  once: the
+// thread's slots in shared memory.
 template <int STAGE>
-__device__ __forceinline__ void stage_update(const RK4Args& a, int n, long long c, double kn)
+__device__ __forceinline__ void stage_update(const RK4Args& a, int n, long long c, double kn, const double* once)
 {
-    const double yn = ld_once(a.Yn[n] + c);
+    const double yn = once[(kSlotYn + n) * kThreads];
     double kk, coef;
     if (STAGE == 1) {
         a.K[n][c] = kn;
         kk = kn; coef = a.half_dt;
     } else if (STAGE < 4) {
-        const double acc = ld_acc(a.K[n] + c) + 2.0 * kn;
+        const double acc = once[(kSlotK + n) * kThreads] + 2.0 * kn;
         a.K[n][c] = acc;
         kk = kn; coef = (STAGE == 3) ? a.dt : a.half_dt;
     } else {
-        kk = ld_acc(a.K[n] + c) + kn; coef = a.dt_sixth;
+        kk = once[(kSlotK + n) * kThreads] + kn; coef = a.dt_sixth;
     }
     const double y = yn + kk * coef;
     double out;
@@ -172,57 +180,9 @@ __device__ __forceinline__ void stage_update(const RK4Args& a, int n, long long 
 // values live (turbulence, momentum, temperature, tracers), each term with the operation
 // order of RHS_Atm_Turb.cpp; stencil values a later phase needs again are re-read, which
 // hits L1.
-#ifndef ATHAD_RK4_MIN_BLOCKS
-#define ATHAD_RK4_MIN_BLOCKS 7   // 72 registers per thread, 7 CTAs of 128 threads per SM
-#endif
-
-#ifndef ATHAD_RK4_BX
-#define ATHAD_RK4_BX 32          // CTA: BX longitudes x BY rows of one level
-#endif
-#ifndef ATHAD_RK4_BY
-#define ATHAD_RK4_BY 4
-#endif
-
-// Shared-memory staging of the stencil tiles (ATHAD_RK4_SMEM=1): the CTA's BY x BX cells of
-// level i with a one-cell ring in j and k, for the 11 stage fields and p_dyn, loaded once
-// per launch; the centre, meridional and zonal neighbours then come from shared memory and
-// only the radial neighbours (levels i +- 1) from global memory (L1/L2).  Same results bit
-// for bit.  Off: measured at 41x181x361 (FP64 step, reference initial state) 1.743 ms
-// against 1.744 ms without it at 32 x 4 and 7 CTAs per SM, 1.76 ms at 6 CTAs, 1.94 ms with
-// 32 x 8 tiles (a third less halo, half the CTAs per SM): the DRAM traffic is already
-// 1.17x the algorithmic bytes, the neighbours the tiles would serve hit L1/L2 today, and
-// the staging adds a barrier and its own loads.
-#ifndef ATHAD_RK4_SMEM
-#define ATHAD_RK4_SMEM 0
-#endif
-constexpr int kTileJ = ATHAD_RK4_BY + 2, kTileK = ATHAD_RK4_BX + 2, kTileFields = 12;
-constexpr int kTileCells = kTileJ * kTileK;
-
 __device__ __forceinline__ const double* stage_field(const RK4Args& a, int n)
 {
     return (n < 11) ? a.Yin[n] : a.p_dyn;
-}
-
-// every thread of the CTA takes part (before any thread returns); levels 0 and im-1 hold
-// boundary cells only and stage nothing
-__device__ __forceinline__ void stage_tiles(const RK4Args& a, double (*tile)[kTileJ][kTileK], int i)
-{
-    const Dims& d = a.d;
-    if (i <= 0 || i >= d.im - 1) return;
-    const int j0 = blockIdx.y * ATHAD_RK4_BY - 1, k0 = blockIdx.x * ATHAD_RK4_BX - 1;
-    const int tid = threadIdx.y * ATHAD_RK4_BX + threadIdx.x;
-    constexpr int kThreads = ATHAD_RK4_BX * ATHAD_RK4_BY;
-#pragma unroll
-    for (int e0 = 0; e0 < kTileCells; e0 += kThreads) {
-        const int e = e0 + tid;
-        if (e >= kTileCells) break;
-        const int tj = e / kTileK, tk = e - tj * kTileK;
-        const int jj = j0 + tj, kk = k0 + tk;
-        if (jj < 0 || jj >= d.jm || kk < 0 || kk >= d.km) continue;
-        const long long g = idx3(d, i, jj, kk);
-#pragma unroll
-        for (int n = 0; n < kTileFields; n++) tile[n][tj][tk] = __ldg(stage_field(a, n) + g);
-    }
 }
 
 #ifndef ATHAD_RK4_TRACER_UNROLL
@@ -231,7 +191,7 @@ __device__ __forceinline__ void stage_tiles(const RK4Args& a, double (*tile)[kTi
 constexpr int kTracerUnroll64 = ATHAD_RK4_TRACER_UNROLL;
 
 template <int STAGE>
-__global__ void __launch_bounds__(ATHAD_RK4_BX * ATHAD_RK4_BY, ATHAD_RK4_MIN_BLOCKS * 128 / (ATHAD_RK4_BX * ATHAD_RK4_BY))
+__global__ void __launch_bounds__(kThreads, ATHAD_RK4_MIN_BLOCKS * 128 / kThreads)
 rk4_stage_kernel(const RK4Args a)
 {
     pdl_trigger();
@@ -244,11 +204,6 @@ rk4_stage_kernel(const RK4Args a)
     const int i = (STAGE % 2 == 0) ? d.im - 1 - (int)blockIdx.z : (int)blockIdx.z;
 #else
     const int i = blockIdx.z;
-#endif
-#if ATHAD_RK4_SMEM
-    __shared__ double tile[kTileFields][kTileJ][kTileK];
-    stage_tiles(a, tile, i);
-    __syncthreads();
 #endif
     if (k >= d.km || j >= d.jm) return;
     const long long c = idx3(d, i, j, k);
@@ -271,22 +226,19 @@ rk4_stage_kernel(const RK4Args a)
         return;
     }
     const long long sI = d.plane, sJ = d.pitch;
+    __shared__ double slots[kSlots<STAGE> * kThreads];
+    double* once = slots + threadIdx.y * ATHAD_RK4_BX + threadIdx.x;
+#pragma unroll
+    for (int n = 0; n < 11; n++) {
+        copy_async(once + (kSlotYn + n) * kThreads, a.Yn[n] + c);
+        if (STAGE > 1) copy_async(once + (kSlotK + n) * kThreads, a.K[n] + c);
+    }
+#pragma unroll
+    for (int f = 0; f < kForcingSlots; f++) copy_async(once + f * kThreads, a.t_eq + c + f * d.fstride);
+    auto forcing = [&](int f) { return once[(f - ATHAD_T_EQ) * kThreads]; };
     const GeoIJ* G = a.geo + (i * d.jm + j);
     const double exp_rm = G->exp_rm, inv_rm = G->inv_rm, inv_rmsinthe = G->inv_rmsinthe;
-#if ATHAD_RK4_SMEM
-    const int ty = threadIdx.y + 1, tx = threadIdx.x + 1;
-    auto star = [&](int n) {
-        Star s;
-        s.c = tile[n][ty][tx];
-        s.jp = tile[n][ty + 1][tx]; s.jm = tile[n][ty - 1][tx];
-        s.kp = tile[n][ty][tx + 1]; s.km = tile[n][ty][tx - 1];
-        const double* F = stage_field(a, n);
-        s.ip = __ldg(F + c + sI); s.im = __ldg(F + c - sI);
-        return s;
-    };
-#else
     auto star = [&](int n) { return load_star(stage_field(a, n), c, sI, sJ); };
-#endif
 
     const double u_ijk = __ldg(a.Yin[1] + c), v_ijk = __ldg(a.Yin[2] + c), w_ijk = __ldg(a.Yin[3] + c);
     const double nue_ijk = __ldg(a.nue + c);
@@ -395,8 +347,9 @@ rk4_stage_kernel(const RK4Args a)
             + d2t(TK, a) * inv_rm2 + dtkedthe * cos_rm2sin + d2p(TK, a) * inv_rm2sinthe2) * diffusion_tke_re;
         const double diffusion_dis = (d2r(DI, a) * exp_2_rm + ddisdr * two_over_rm_exp
             + d2t(DI, a) * inv_rm2 + ddisdthe * cos_rm2sin + d2p(DI, a) * inv_rm2sinthe2) * diffusion_dis_re;
-        stage_update<STAGE>(a, 9, c, -tr_tke + diffusion_tke + tke_source);
-        stage_update<STAGE>(a, 10, c, -tr_dis + diffusion_dis + dis_source);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        stage_update<STAGE>(a, 9, c, -tr_tke + diffusion_tke + tke_source, once);
+        stage_update<STAGE>(a, 10, c, -tr_dis + diffusion_dis + dis_source, once);
         if (STAGE == 4 && a.write_diag) {
             a.prod[c] = prod;
             a.tke_source[c] = tke_source;
@@ -436,7 +389,7 @@ rk4_stage_kernel(const RK4Args a)
             const double rhs_u = -dpdr_exp - tr_u + diffusion_u
                 + a.buoy_pref * (t_ijk - __ldg(a.t_ref + i))
                 + 1.0 * a.force_nd * coriolis_rad;
-            stage_update<STAGE>(a, 1, c, rhs_u);
+            stage_update<STAGE>(a, 1, c, rhs_u, once);
             if (STAGE == 4) a.aux_u[c] = rhs_u + dpdr_exp;
         }
         {   // v: every term but the w-shear one, which closes the sum below
@@ -455,9 +408,9 @@ rk4_stage_kernel(const RK4Args a)
             const double coriolis_the = 2.0 * costhe * w_ijk;
             const double rhs_v = -dpdthe_invrm - tr_v + diffusion_v
                 + 1.0 * a.force_nd * coriolis_the
-                + a.coeff_MC_vel * __ldg(a.MC_v + c)
+                + a.coeff_MC_vel * forcing(ATHAD_MC_V)
                 - surf_drag * v_ijk;
-            stage_update<STAGE>(a, 2, c, rhs_v);
+            stage_update<STAGE>(a, 2, c, rhs_v, once);
             if (STAGE == 4) a.aux_v[c] = rhs_v + dpdthe_invrm;
         }
         {   // w
@@ -472,33 +425,33 @@ rk4_stage_kernel(const RK4Args a)
             const double coriolis_phi = -2.0 * (costhe * v_ijk + nontrad * sinthe * u_ijk);
             const double rhs_w = -dpdphi_invrs - tr_w + diffusion_w
                 + 1.0 * a.force_nd * coriolis_phi
-                + a.coeff_MC_vel * __ldg(a.MC_w + c)
+                + a.coeff_MC_vel * forcing(ATHAD_MC_W)
                 - surf_drag * w_ijk;
-            stage_update<STAGE>(a, 3, c, rhs_w);
+            stage_update<STAGE>(a, 3, c, rhs_w, once);
             if (STAGE == 4) a.aux_w[c] = rhs_w + dpdphi_invrs;
         }
         // ---- temperature (RHS_Atm_Turb.cpp:752, 829, 866-868, 963-992) ----
         {
             const Star T = star(0);
             const double t_ijk = T.c;
-            const double r_h = __ldg(a.r_humid + c);
+            const double r_h = forcing(ATHAD_R_HUMID);
             const double pressure_t = a.coeff_energy_p * (u_exp * dpdr + v_invrm * dpdthe + w_invrs * dpdphi);
             const double tr_t = u_exp * ar(T, a) + v_invrm * at(T, a) + w_invrs * ap(T, a);
             const double diffusion_t_re = (a.inv_re + nue_ijk) / a.pr_turb * a.diffusion_ramp;
             const double diffusion_t = (d2r(T, a) * exp_2_rm + d1r(T, a) * two_over_rm_exp
                 + d2t(T, a) * inv_rm2 + d1t(T, a) * cos_rm2sin + d2p(T, a) * inv_rm2sinthe2) * diffusion_t_re;
             double rhs_t = pressure_t - tr_t + diffusion_t
-                + a.coeff_MC_t * __ldg(a.MC_t + c)
-                + a.coeff_energy * (__ldg(a.S_c + c) + __ldg(a.S_r + c)) * a.lv * r_h
-                + a.coeff_energy * (__ldg(a.S_i + c) + __ldg(a.S_s + c) + __ldg(a.S_g + c)) * a.ls * r_h;
+                + a.coeff_MC_t * forcing(ATHAD_MC_T)
+                + a.coeff_energy * (forcing(ATHAD_S_C) + forcing(ATHAD_S_R)) * a.lv * r_h
+                + a.coeff_energy * (forcing(ATHAD_S_I) + forcing(ATHAD_S_S) + forcing(ATHAD_S_G)) * a.ls * r_h;
             const double k_a = 1.0 / (4.0 * 86400.0), k_s = 1.0 / (0.4 * 86400.0), sigma_b = 0.7;
             const double p_surf = __ldg(a.p_stat + idx3(d, 0, j, k));
-            const double sigma = (p_surf > 0.0) ? __ldg(a.p_stat + c) / p_surf : 0.0;
+            const double sigma = (p_surf > 0.0) ? forcing(ATHAD_P_STAT) / p_surf : 0.0;
             double bl = (sigma - sigma_b) / (1.0 - sigma_b);
             if (bl < 0.0) bl = 0.0;
             const double k_T = k_a + (k_s - k_a) * bl * G->cos4lat;
-            rhs_t -= (k_T * a.L_atm / a.u_0) * (t_ijk - __ldg(a.t_eq + c));
-            stage_update<STAGE>(a, 0, c, rhs_t);
+            rhs_t -= (k_T * a.L_atm / a.u_0) * (t_ijk - forcing(ATHAD_T_EQ));
+            stage_update<STAGE>(a, 0, c, rhs_t, once);
         }
     }
     // ---- moisture and tracers (RHS_Atm_Turb.cpp:830-834, 911-934, 1059-1072) ----
@@ -506,7 +459,7 @@ rk4_stage_kernel(const RK4Args a)
         const double exp_2_rm = G->exp_2_rm, inv_rm2 = G->inv_rm2, inv_rm2sinthe2 = G->inv_rm2sinthe2;
         const double cos_rm2sin = G->costhe_inv_rm2sinthe, two_over_rm_exp = G->two_over_rm_exp;
         const double dlnrho_dr_i = a.tracer_diff_flux ? __ldg(a.dlnrho + i) * exp_2_rm : 0.0;
-        const double r_h = __ldg(a.r_humid + c);
+        const double r_h = forcing(ATHAD_R_HUMID);
 #pragma unroll kTracerUnroll64
         for (int n = 4; n <= 8; n++) {
             const Star Q = star(n);
@@ -519,12 +472,12 @@ rk4_stage_kernel(const RK4Args a)
                 + d2p(Q, a) * inv_rm2sinthe2
                 + q1r * dlnrho_dr_i) * coef;
             double rhs;
-            if (n == 4)      rhs = -tr + dif + 1.0 * __ldg(a.S_v + c) * r_h + a.coeff_MC_q * __ldg(a.MC_q + c);
-            else if (n == 5) rhs = -tr + dif + 1.0 * __ldg(a.S_c + c) * r_h;
-            else if (n == 6) rhs = -tr + dif + 1.0 * __ldg(a.S_i + c) * r_h;
-            else if (n == 7) rhs = -tr + dif + 1.0 * __ldg(a.S_g + c) * r_h;
+            if (n == 4)      rhs = -tr + dif + 1.0 * forcing(ATHAD_S_V) * r_h + a.coeff_MC_q * forcing(ATHAD_MC_Q);
+            else if (n == 5) rhs = -tr + dif + 1.0 * forcing(ATHAD_S_C) * r_h;
+            else if (n == 6) rhs = -tr + dif + 1.0 * forcing(ATHAD_S_I) * r_h;
+            else if (n == 7) rhs = -tr + dif + 1.0 * forcing(ATHAD_S_G) * r_h;
             else             rhs = -tr + dif;
-            stage_update<STAGE>(a, n, c, rhs);
+            stage_update<STAGE>(a, n, c, rhs, once);
         }
     }
 }
