@@ -1293,7 +1293,7 @@ athad_status athad_checkpoint_wait(athad_ctx* ctx)
     return cuda_check(ctx, cudaEventSynchronize(ctx->ckpt_done), "checkpoint_wait");
 }
 
-static athad_status multilayer_radiation(athad_ctx* ctx)
+static RadArgs rad_args(athad_ctx* ctx)
 {
     const athad_params& p = ctx->p;
     RadArgs a;
@@ -1304,35 +1304,29 @@ static athad_status multilayer_radiation(athad_ctx* ctx)
     a.cloud = F[ATHAD_CLOUD]; a.ice = F[ATHAD_ICE];
     a.radiation = F[ATHAD_RADIATION]; a.epsilon = F[ATHAD_EPSILON];
     a.epsilon_2D = ctx->f2d[ATHAD_2D_EPSILON]; a.albedo = ctx->f2d[ATHAD_2D_ALBEDO];
-    a.T = ctx->stA[1]; a.dn = ctx->stA[2];   // RK4 stage buffers, free between RK4 steps
+    a.T = ctx->stA[1];   // RK4 stage buffer, free between RK4 steps
     a.step_f = ctx->step_f;
     a.t_0 = p.t_0; a.g = p.g; a.R_bg = p.R_bg; a.sigma = p.sigma;
     a.kappa_H2O = p.kappa_H2O; a.kappa_CO2 = p.kappa_CO2; a.kappa_bg = p.kappa_bg;
     a.geothermal_flux = p.geothermal_flux; a.albedo_surface = p.albedo_surface;
     a.albedo_cloud = p.albedo_cloud; a.rad_equator_short = p.rad_equator_short;
     a.rad_pole_short = p.rad_pole_short;
-    launch_multilayer_radiation(a, ctx->stream);
-    ATHAD_CHECK_LAUNCH(ctx, "multilayer_radiation");
-    return ATHAD_OK;
+    return a;
 }
 
 athad_status athad_multilayer_radiation(athad_ctx* ctx)
 {
     if (!ctx) return ATHAD_ERR_INVALID;
-    return multilayer_radiation(ctx);
+    launch_multilayer_radiation(rad_args(ctx), ctx->stream);
+    ATHAD_CHECK_LAUNCH(ctx, "multilayer_radiation");
+    return ATHAD_OK;
 }
 
 athad_status athad_radiative_heating(athad_ctx* ctx, double omega_rad)
 {
     if (!ctx) return ATHAD_ERR_INVALID;
-    double* t = ctx->field[ATHAD_T];
-    double* t_before = ctx->stA[0];
-    athad_status s = cuda_check(ctx, cudaMemcpyAsync(t_before, t, ctx->L.field_elems * sizeof(double),
-                                                     cudaMemcpyDeviceToDevice, ctx->stream), "radiative_heating");
-    if (s == ATHAD_OK) s = multilayer_radiation(ctx);
-    if (s != ATHAD_OK) return s;
-    launch_rad_blend(ctx->L.d, t_before, t, omega_rad, ctx->stream);
-    ATHAD_CHECK_LAUNCH(ctx, "radiative_heating blend");
+    launch_radiative_heating(rad_args(ctx), omega_rad, ctx->stream);
+    ATHAD_CHECK_LAUNCH(ctx, "radiative_heating");
     return ATHAD_OK;
 }
 

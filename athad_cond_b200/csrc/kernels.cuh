@@ -286,12 +286,13 @@ struct RadArgs {
     const double* c; const double* co2; const double* p_stat; const double* cloud; const double* ice;
     double* radiation; double* epsilon;
     double* epsilon_2D; double* albedo;   // 2-D, jm rows of pitch
-    double* T; double* dn;                // scratch fields: layer temperature [K], downward flux
+    double* T;                            // scratch field (columns too tall for shared memory)
     const double* step_f;                 // [im] float layer thickness
     double t_0, g, R_bg, sigma, kappa_H2O, kappa_CO2, kappa_bg, geothermal_flux;
     double albedo_surface, albedo_cloud, rad_equator_short, rad_pole_short;
 };
 void launch_multilayer_radiation(const RadArgs& a, cudaStream_t st);
+void launch_radiative_heating(const RadArgs& a, double omega, cudaStream_t st);   // blended into t
 
 // the moist iteration's caps and the vapour ceiling (k_caps.cu)
 struct CapsArgs {
@@ -368,6 +369,5 @@ void launch_water_vapour_evaporation(const SurfaceArgs& a, cudaStream_t st);
 void launch_latent_sensible_heat(const SurfaceArgs& a, cudaStream_t st);
 // planetaryShortWave's per-row albedo sums, summed over k in order (k_rad.cu)
 void launch_albedo_rows(const Dims& d, const double* albedo, double* out, cudaStream_t st);
-void launch_rad_blend(const Dims& d, const double* t_before, double* t, double omega, cudaStream_t st);
 
 }  // namespace athad

@@ -84,3 +84,18 @@ def test_skin_temperature_matches_oracle():
             want = update_skin_temperature(p, albedo, t, 0.25)
             t = g.update_skin_temperature(0.25)
             assert t == want and t != p.t_skin
+
+
+@pytest.mark.parametrize("grid", [(4, 5, 5), (13, 9, 33), (61, 7, 65), (300, 5, 37)])
+def test_column_heights_and_ragged_rows(grid):
+    """The fewest layers, rows that end inside a CTA's 32 columns, and columns that do not
+    fit shared memory (more than 288 layers)."""
+    st = state(grid, 85)
+    o = OracleState(st, config_params())
+    with GpuAtmosphere(*grid, config_params()) as g:
+        g.upload_state(st)
+        g.radiative_heating(0.05)
+        o.radiative_heating(0.05)
+        for n in ("t", "radiation", "epsilon"):
+            assert close(g.download(n), o.f[n]) <= 1e-12, n
+        assert close(g.download_2d("albedo"), o.f2["albedo"]) <= 1e-12
