@@ -726,7 +726,12 @@ athad_status athad_pressure_sweep(athad_ctx* ctx, int32_t n_sweeps, int32_t tota
     if (n_sweeps == 0) return ATHAD_OK;
     PoissonArgs a = poisson_args(ctx, total_iter_count);
     a.aux_lid = 1;
-    for (int i = 0; i < n_sweeps; i++) {
+    a.first_sweep = 1;
+    if (poisson_sweeps_split(ctx->L.d, n_sweeps)) {
+        // RK4 stage buffers: scratch between RK4 steps
+        launch_poisson_sweeps_split(a, n_sweeps, ctx->stA[0], ctx->stA[1], ctx->stream);
+        ATHAD_CHECK_LAUNCH(ctx, "poisson sweeps");
+    } else for (int i = 0; i < n_sweeps; i++) {
         a.first_sweep = (i == 0) ? 1 : 0;
         launch_poisson_sweep(a, ctx->stream);
         ATHAD_CHECK_LAUNCH(ctx, "poisson sweep");

@@ -293,6 +293,208 @@ void launch_poisson_sweep(const PoissonArgs& a, cudaStream_t st)
     launch_dependent(poisson_ceiling_kernel, dim3((unsigned)blocks), dim3(256), 0, st, a);
 }
 
+// ---------------------------------------------------------------------------------------
+// Many sweeps in a row (project_initial_velocity's 200).  The source is the same in every
+// sweep (aux is constant), so it is formed once; from the second sweep on, p and the source
+// stand in scratch fields whose rows are split by the parity of k, even longitudes first, so
+// that a colour's cells, and the neighbours it reads, are consecutive.  In the model's layout
+// each colour pass moves both colours' lines (12.4 us per pass at 41x181x361, with the
+// source, boundary and ceiling launches 49 us per sweep); split, half of them (18 us per sweep).
+//
+// The boundary cells are not stored between sweeps.  After a sweep's boundary passes each is
+// a copy of the interior cell next to it (radial, poles) or the average of the two cells next
+// to the seam, limited by the ceiling.  A cell's boundary neighbour is therefore its own
+// value before the update, and at the seam the average of its own and the opposite cell's;
+// with an odd km (every grid with an equator and a seam meridian) those two have the same
+// colour, and the thread of the first updates both after reading both.  Values are stored
+// unlimited; a pass that reads a value of the sweep before applies the ceiling to it, so the
+// results are those of the separate launches bit for bit.  The first sweep, which reads p
+// and its boundary cells as the caller left them, runs as separate launches, and the second
+// sweep's colours read its boundary cells in the model's layout; from there on every value is
+// finite (the clamped source moves a limited value by at most 2).
+__device__ __forceinline__ long long split_at(long long row, int pitch, int k) { return row + (k & 1) * (pitch >> 1) + (k >> 1); }
+
+// p and the source of the interior cells into the split rows
+__global__ void __launch_bounds__(256) poisson_split_kernel(PoissonArgs a, double* __restrict__ ps, double* __restrict__ ss)
+{
+    pdl_trigger();
+    pdl_wait();
+    const Dims& d = a.d;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z;
+    if (k >= d.km || j >= d.jm) return;
+    const long long row = idx3(d, i, j, 0), q = split_at(row, d.pitch, k);
+    ps[q] = a.p[row + k];
+    ss[q] = a.src[row + k];
+}
+
+__device__ __forceinline__ double ceiling_finite(double v, double cap) { return (v > cap) ? cap : (v < -cap) ? -cap : v; }
+
+// The coefficients of one row's cells
+struct RowCoef { double num1, num2, num3, num_a, inv_denom; };
+
+__device__ __forceinline__ double split_update(const RowCoef& R, double pip, double pim, double pjp, double pjm,
+                                               double pkp, double pkm, double src)
+{
+    return ((pip + pim) * R.num1 + (pjp + pjm) * R.num2 + (pkp + pkm) * R.num3 + (pip - pim) * R.num_a - src)
+         * R.inv_denom;
+}
+
+__device__ __forceinline__ RowCoef row_coef(const PoissonArgs& a, int i, int j)
+{
+    const PoiIJ& Q = a.poi[i * a.d.jm + j];
+    RowCoef R{Q.num1, Q.num2, Q.num3, 0.0, Q.inv_denom};
+    if (a.anelastic) R.num_a = Q.exp_2_rm * __ldg(a.dlnrho + i) * a.inv_2dr;
+    return R;
+}
+
+// The two cells next to the seam, k = 1 and km - 2, of row (i, j): both read before either is
+// written.  LIMIT0: the values of the other colour are the sweep before's.
+template <bool LIMIT0>
+__device__ __forceinline__ bool split_seam(const PoissonArgs& a, double* ps, const double* ss, int i, int j)
+{
+    const Dims& d = a.d;
+    const double cap = a.ceiling;
+    const int half = d.pitch >> 1, last = (d.km - 3) / 2;            // slot of km - 2 in the odd half
+    const long long row = idx3(d, i, j, 0);
+    const RowCoef R = row_coef(a, i, j);
+    const double own[2] = {ps[row + half], ps[row + half + last]};
+    const double seam = ceiling_finite((own[0] + own[1]) / 2.0, cap);
+    auto other = [&](long long at) { const double v = ps[at]; return LIMIT0 ? ceiling_finite(v, cap) : v; };
+    double v[2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const long long c = row + half + (e ? last : 0);
+        const double bnd = ceiling_finite(own[e], cap);
+        // even slots 1 (k = 2) and last (k = km - 3)
+        const double inner = other(row + (e ? last : 1));
+        v[e] = split_update(R, i + 1 == d.im - 1 ? bnd : other(c + d.plane), i - 1 == 0 ? bnd : other(c - d.plane),
+                            j + 1 == d.jm - 1 ? bnd : other(c + d.pitch), j - 1 == 0 ? bnd : other(c - d.pitch),
+                            e ? seam : inner, e ? inner : seam, ss[c]);
+    }
+    ps[row + half] = v[0];
+    ps[row + half + last] = v[1];
+    return !(fabs(v[0]) <= cap) || !(fabs(v[1]) <= cap);
+}
+
+// One colour of one sweep: a thread takes two consecutive cells of a row's half (16-byte
+// loads of its neighbours, which have the same slots in the rows around); the CTAs of the
+// last blockIdx.x take the cells next to the seam, a row per thread.  counters[5] is set once
+// a value beyond the ceiling was formed; from then on the values of the sweep before are
+// limited as they are read.
+// 200 sweeps of 41x181x361: 3584 us with 32 x 8 threads and 64 registers, 3794 with 32 x 4,
+// 3868 with 32 x 16 (each row's halves are read again by the CTAs above and below, and the
+// pass runs at the L2's bandwidth), 4050 with 48 registers, 5085 with 40 (spills).
+constexpr int kSplitX = 32, kSplitY = 8;
+template <int COLOUR>
+__global__ void __launch_bounds__(kSplitX * kSplitY, 4)
+poisson_split_colour_kernel(PoissonArgs a, double* ps, const double* ss)
+{
+    pdl_trigger();
+    const Dims& d = a.d;
+    bool beyond = false;
+    if (blockIdx.x == gridDim.x - 1) {
+        pdl_wait();
+        const int i = 1 + blockIdx.z;
+        const int j = 1 + blockIdx.y * (kSplitX * kSplitY) + threadIdx.y * kSplitX + threadIdx.x;
+        if (j < d.jm - 1 && ((i + j + COLOUR) & 1)) beyond = split_seam<COLOUR == 0>(a, ps, ss, i, j);
+    } else {
+        const int j = 1 + blockIdx.y * kSplitY + threadIdx.y;
+        const int i = 1 + blockIdx.z;
+        const int s0 = 2 * (blockIdx.x * kSplitX + threadIdx.x);         // first slot of the half
+        const int par = (i + j + COLOUR) & 1;                            // parity of the colour's k
+        // the slots of cells that are not next to the seam: even k 2 .. km - 3, odd k 3 .. km - 4
+        const int hi = par ? (d.km - 5) / 2 : (d.km - 3) / 2;
+        const bool mine = j < d.jm - 1 && s0 <= hi;
+        RowCoef R;
+        if (mine) R = row_coef(a, i, j);
+        pdl_wait();
+        if (mine) {
+            const double cap = a.ceiling;
+            const int half = d.pitch >> 1;
+            const int sI = (int)d.plane, sJ = d.pitch;
+            const long long row = idx3(d, i, j, 0) + s0;
+            double* P0 = ps + row + par * half;                          // own cells
+            const double* O = ps + row + (1 - par) * half;               // the other parity's slots
+            auto two = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
+            // even k: the neighbours k - 1, k + 1 are the odd slots s0 - 1 .. s0 + 1; odd k:
+            // the even slots s0 .. s0 + 2
+            double2 ip = two(P0 + sI), im = two(P0 - sI), jp = two(P0 + sJ), jm = two(P0 - sJ), o = two(O);
+            double out = par ? O[2] : (s0 > 0 ? O[-1] : 0.0);
+            const double2 src = two(ss + row + par * half);
+            const bool limit = a.counters[5] != 0ull;
+            if (COLOUR == 0 && limit) {
+                auto lim2 = [&](double2& v) { v.x = ceiling_finite(v.x, cap); v.y = ceiling_finite(v.y, cap); };
+                lim2(ip); lim2(im); lim2(jp); lim2(jm); lim2(o);
+                out = ceiling_finite(out, cap);
+            }
+            if (i == 1 || i == d.im - 2 || j == 1 || j == d.jm - 2) {
+                double2 own = two(P0);
+                if (limit) own = make_double2(ceiling_finite(own.x, cap), ceiling_finite(own.y, cap));
+                if (i == d.im - 2) ip = own;
+                if (i == 1) im = own;
+                if (j == d.jm - 2) jp = own;
+                if (j == 1) jm = own;
+            }
+            const double vx = split_update(R, ip.x, im.x, jp.x, jm.x, par ? o.y : o.x, par ? o.x : out, src.x);
+            const double vy = split_update(R, ip.y, im.y, jp.y, jm.y, par ? out : o.y, par ? o.y : o.x, src.y);
+            const bool mx = s0 > 0, my = s0 + 1 <= hi;
+            if (mx && my) *reinterpret_cast<double2*>(P0) = make_double2(vx, vy);
+            else if (mx) P0[0] = vx;
+            else if (my) P0[1] = vy;
+            beyond = (mx && !(fabs(vx) <= cap)) || (my && !(fabs(vy) <= cap));
+        }
+    }
+    if (__any_sync(0xffffffffu, beyond) && (threadIdx.x & 31) == 0) atomicOr(a.counters + 5, 1ull);
+}
+
+// the split rows back into p: the boundary values formed from the interior, everything
+// limited; the call's clamp count is the one source's times the sweeps
+__global__ void __launch_bounds__(256) poisson_merge_kernel(PoissonArgs a, const double* __restrict__ ps, int n_sweeps)
+{
+    pdl_wait();
+    const Dims& d = a.d;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z;
+    if (a.counters && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0) {
+        a.counters[0] *= (unsigned long long)n_sweeps;   // the first sweep's count
+    }
+    if (k >= d.km || j >= d.jm) return;
+    const int ii = min(max(i, 1), d.im - 2), jj = min(max(j, 1), d.jm - 2);
+    const long long row = idx3(d, ii, jj, 0);
+    double v;
+    if (k == 0 || k == d.km - 1) v = (ps[split_at(row, d.pitch, 1)] + ps[split_at(row, d.pitch, d.km - 2)]) / 2.0;
+    else v = ps[split_at(row, d.pitch, k)];
+    a.p[idx3(d, i, j, k)] = ceiling_finite(v, a.ceiling);
+}
+
+// At least kSplitFrom sweeps, of which two run in the model's layout.  Projections of 5, 8
+// and 200 sweeps: 346 -> 255 us, 494 -> 309, 9744 -> 3584 at 41x181x361; 130 -> 93 us (5)
+// and 3322 -> 1141 (200) at 21x91x181; with 4 sweeps only two would be split.
+constexpr int kSplitFrom = 5;
+bool poisson_sweeps_split(const Dims& d, int n_sweeps) { return n_sweeps >= kSplitFrom && (d.km & 1); }
+
+void launch_poisson_sweeps_split(const PoissonArgs& a, int n_sweeps, double* ps, double* ss, cudaStream_t st)
+{
+    const Dims& d = a.d;
+    const dim3 block(32, 8), grid((d.km + 31) / 32, (d.jm + 7) / 8, d.im);
+    const dim3 half_grid(((d.km + 1) / 2 + 31) / 32, (d.jm + 7) / 8, d.im);
+    launch_poisson_sweep(a, st);
+    launch_dependent(poisson_colour_kernel<0>, half_grid, block, 0, st, a);
+    launch_dependent(poisson_colour_kernel<1>, half_grid, block, 0, st, a);
+    launch_dependent(poisson_split_kernel, grid, block, 0, st, a, ps, ss);
+    // pairs of the slots 0 .. (km - 3) / 2, and one more column of CTAs for the seam
+    const dim3 sblock(kSplitX, kSplitY);
+    const dim3 sgrid((((d.km - 1) / 2 + 1) / 2 + kSplitX - 1) / kSplitX + 1, (d.jm - 2 + kSplitY - 1) / kSplitY, d.im - 2);
+    for (int s = 2; s < n_sweeps; s++) {
+        launch_dependent(poisson_split_colour_kernel<0>, sgrid, sblock, 0, st, a, ps, (const double*)ss);
+        launch_dependent(poisson_split_colour_kernel<1>, sgrid, sblock, 0, st, a, ps, (const double*)ss);
+    }
+    launch_dependent(poisson_merge_kernel, grid, block, 0, st, a, (const double*)ps, n_sweeps);
+}
+
 // the boundary conditions of a sweep alone (radial, pole, seam), PressureSolverAtm.h:504-552
 void launch_poisson_bcs(const PoissonArgs& a, cudaStream_t st)
 {

@@ -341,3 +341,33 @@ def test_report_counts_nonfinite_temperature_and_times_the_step(precision):
         g.upload("t", t)
         g.solveRungeKutta_Atmosphere_Turb(4e-5, 1.0, 0.5)
         assert g.report()["nonfinite_inputs"] == 3
+
+
+@pytest.mark.parametrize("grid", [(4, 5, 5), (5, 6, 7), (11, 21, 41), (9, 14, 66), (13, 18, 131)])
+@pytest.mark.parametrize("n_sweeps, anelastic", [(4, 0), (5, 0), (6, 1), (23, 0)])
+def test_many_sweeps_bit_exact(grid, n_sweeps, anelastic):
+    """Enough sweeps in a row for the split rows (odd km): from a pressure with non-finite
+    values and boundary cells of its own, and sources that drive it beyond the ceiling."""
+    p = config_params()
+    p.anelastic = anelastic
+    p.metric_divergence = anelastic
+    st = make_state(*grid, seed=29)
+    rng = np.random.default_rng(31)
+    for n in ("aux_u", "aux_v", "aux_w"):
+        st[n] = 0.2 * rng.standard_normal(grid)
+    st["aux_v"][1, 2, 1:4] = 1e6
+    st["p_dyn"] = 4.0 * rng.standard_normal(grid)
+    st["p_dyn"][1, 2, 1] = np.nan
+    st["p_dyn"][2, 1, grid[2] - 2] = np.inf
+    st["p_dyn"][0, 2, 2] = -np.inf
+    if anelastic:
+        st["dlnrho_dr"] = np.linspace(-1.0, -3.0, grid[0])
+    o = OracleState(st, p)
+    cells, clamped = o.pressure_sweep(n_sweeps=n_sweeps, total_iter_count=400)
+    assert np.max(np.abs(o.f["p_dyn"])) == 3.0          # the ceiling was reached
+    with gpu_with(st, p) as g:
+        g.PressureSolverAtm_run(total_iter_count=400, n_sweeps=n_sweeps)
+        for n in ("p_dyn", "aux_u", "aux_v", "aux_w"):
+            assert np.array_equal(g.download(n), o.f[n]), n
+        r = g.report()
+        assert r["poisson_src_cells"] == cells and r["poisson_src_clamped"] == clamped
