@@ -2,12 +2,12 @@
 // the configuration's CategoryIceScheme = 2) of the ATHAD_COND atmosphere on sm_100a, flat
 // terrain:
 //
-//   ice_init_kernel      initArrays (:126-158): non-negative water species, the falling
-//                        fluxes restarted from the time level n;
-//   ice_columns_kernel   computeColumns (:162-484): one thread per (j, k) column walks the
-//                        column top-down, up to three passes until the rain flux at i = 1
-//                        settles; per cell the COSMO sources and sinks, the cloud-water and
-//                        cloud-ice limiters and the capped flux integration;
+//   ice_columns_kernel   initArrays (:126-158): non-negative water species, the falling
+//                        fluxes restarted from the time level n; then computeColumns
+//                        (:162-484): one thread per (j, k) column walks the column top-down,
+//                        up to three passes until the rain flux at i = 1 settles; per cell
+//                        the COSMO sources and sinks, the cloud-water and cloud-ice limiters
+//                        and the capped flux integration;
 //   ice_bc_*_kernel      applyBoundaryConditions (:489-492): IceSchemeCommon::extrapolateBC
 //                        (IceSchemeCommon.h:27-52) of P_rain and P_snow, radial lid, poles,
 //                        then the seam with its average (launch_precip_bc, shared with the
@@ -19,6 +19,14 @@
 // exp, log and the saturation curves are CUDA's.  The reference's pow calls become powers of
 // one root per cell (Rain^(1/18), Snow^(1/26)), cbrt and x * sqrt(x): the same exponents
 // within a few ulp.
+//
+// The columns are one wave of warps and bound by the latency of a level: 147 registers
+// left room for three of the 3.7 CTAs per SM (two waves, 536 us at 41x181x361; 128
+// registers, 312), a level read its operands where it used them (loads ahead of everything
+// and the fluxes above in registers, with the initial clamps, 45 us as a launch of their
+// own, folded into the first pass: 254 of 591 us for the scheme).  Keeping the saturation
+// values for the later passes in scratch fields, 260: most columns settle in one pass.
+// Prefetching the next levels into L2: 247-254.
 #include "ice_common.cuh"
 
 namespace athad {
@@ -39,53 +47,72 @@ constexpr int kIterPrecEnd = 3, kIcheck = 1;
 
 using ice::dmax;
 using ice::dmin;
-using ice::q_sat_at;
 using ice::evaporate_cell;
 
-__global__ void __launch_bounds__(256) ice_init_kernel(IceArgs a)
+// initArrays (:126-158) of one cell: the water species and level n's fluxes non-negative
+// (stored only where that changes them); returns level n's fluxes
+__device__ __forceinline__ double floor0(double* p, double v)
 {
-    const long long n = a.d.fstride;
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n;
-         c += (long long)gridDim.x * blockDim.x) {
-        a.c[c] = dmax(0.0, a.c[c]);
-        a.cloud[c] = dmax(0.0, a.cloud[c]);
-        a.ice[c] = dmax(0.0, a.ice[c]);
-        const double pr = dmax(0.0, a.P_rainn[c]);
-        const double ps = dmax(0.0, a.P_snown[c]);
-        a.P_rainn[c] = pr; a.P_snown[c] = ps;
-        a.P_rain[c] = pr; a.P_snow[c] = ps;
-    }
+    const double w = dmax(0.0, v);
+    if (__double_as_longlong(v) != __double_as_longlong(w)) *p = w;
+    return w;
+}
+__device__ __forceinline__ double2 init_cell(const IceArgs& a, long long c)
+{
+    const double cv = a.c[c], cl = a.cloud[c], ic = a.ice[c], pr = a.P_rainn[c], ps = a.P_snown[c];
+    floor0(a.c + c, cv);
+    floor0(a.cloud + c, cl);
+    floor0(a.ice + c, ic);
+    return make_double2(floor0(a.P_rainn + c, pr), floor0(a.P_snown + c, ps));
 }
 
-__global__ void __launch_bounds__(128) ice_columns_kernel(IceArgs a)
+__global__ void __launch_bounds__(128, 4) ice_columns_kernel(IceArgs a)
 {
     const Dims& d = a.d;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
-    if (k < 1 || k >= d.km - 1 || j < 1 || j >= d.jm - 1) return;
-    const long long sI = d.plane;
+    if (k >= d.km) return;
+    if (k < 1 || k >= d.km - 1 || j < 1 || j >= d.jm - 1) {
+        for (int i = 0; i < d.im; i++) {
+            const long long c = idx3(d, i, j, k);
+            const double2 f = init_cell(a, c);
+            a.P_rain[c] = f.x; a.P_snow[c] = f.y;
+        }
+        return;
+    }
     const double t_0 = a.t_0;
     const double P_max = 50.0 / 86400.0;
-    const double Rain_check = a.P_rain[idx3(d, kIcheck, j, k)];
+    init_cell(a, idx3(d, d.im - 1, j, k));
+    const double Rain_check = dmax(0.0, a.P_rainn[idx3(d, kIcheck, j, k)]);
     double m_i = kMiMax, N_i = 0.0, S_nuc = 0.0, S_i_dep = 0.0;
     for (int iter_prec = 1; iter_prec <= kIterPrecEnd; iter_prec++) {
         a.P_rain[idx3(d, d.im - 1, j, k)] = 0.0;
         a.P_snow[idx3(d, d.im - 1, j, k)] = 0.0;
+        double* P_r = (iter_prec == 1) ? a.P_rainn : a.P_rain;
+        double* P_s = (iter_prec == 1) ? a.P_snown : a.P_snow;
+        double rain_above = 0.0, snow_above = 0.0, P_rain_check = 0.0;   // the new fluxes of level i + 1; at kIcheck
         for (int i = d.im - 2; i >= 0; i--) {
             const long long c = idx3(d, i, j, k);
+            // everything the cell reads, before anything is computed from it
             const double t_u = a.t[c] * t_0;
+            const double co2 = a.co2[c], p_local = a.p_stat[c], rh = a.r_humid[c], S_c_c = a.S_c_c[c];
+            double cv = a.c[c], cl = a.cloud[c], ic = a.ice[c], Rain = P_r[c], Snow = P_s[c];
+            if (iter_prec == 1) {
+                cv = floor0(a.c + c, cv); cl = floor0(a.cloud + c, cl); ic = floor0(a.ice + c, ic);
+                Rain = floor0(P_r + c, Rain); Snow = floor0(P_s + c, Snow);
+            }
             // IceSchemeCommon::canCondense (IceSchemeCommon.h:108-111); its q_sat is the
             // scheme's own
-            if (t_u >= T_CRIT) {
-                evaporate_cell(a, c, t_u);
-                continue;
-            }
-            const double q_sat = q_sat_at(a, c, saturation_pressure(t_u));
+            const double M_other = M_nonwater(cv, co2, a.M_bg);
+            double q_sat = 1.0;
+            if (t_u < T_CRIT) q_sat = saturation_mass_fraction(saturation_pressure(t_u), p_local, M_other);
             if (!(q_sat < 1.0)) {
+                if (iter_prec == 1) { a.P_rain[c] = Rain; a.P_snow[c] = Snow; }
                 evaporate_cell(a, c, t_u);
+                rain_above = 0.0; snow_above = 0.0;
                 continue;
             }
-            const double Rain = a.P_rain[c], Snow = a.P_snow[c];
+            const double q_Ice = saturation_mass_fraction(sublimation_pressure(t_u), p_local, M_other);
             // the rain powers 4/9, 7/9, 13/9 and 1/6 from one logarithm: r18 = Rain^(1/18)
             double R49 = 0.0, R79 = 0.0, R139 = 0.0, R16 = 0.0;
             if (Rain > 1e-12) {
@@ -104,12 +131,9 @@ __global__ void __launch_bounds__(128) ice_columns_kernel(IceArgs a)
                 const double s8 = s4 * s4;
                 S526 = s4 * s26; S813 = s8 * s8;
             }
-            const double q_Ice = q_sat_at(a, c, sublimation_pressure(t_u));
             const double step = a.step_f[i];
-            const double rh = a.r_humid[c];
             const double mass_layer = rh * step;
             const double dt_snow_dim = step / 0.96;
-            const double cv = a.c[c], cl = a.cloud[c], ic = a.ice[c];
             if (!(t_u > t_0) && !(t_u <= kThn)) {
                 N_i = kNi0 * exp(0.2 * (t_0 - t_u));
                 m_i = dmin((rh * ic) / N_i, kMiMax);
@@ -178,7 +202,6 @@ __global__ void __launch_bounds__(128) ice_columns_kernel(IceArgs a)
                 const double fac = max_ice_loss / S_ice_total;
                 S_i_au *= fac; S_d_au *= fac; S_agg *= fac; S_i_cri *= fac; S_i_melt *= fac;
             }
-            const double S_c_c = a.S_c_c[c];
             a.S_v[c] = -S_c_c + S_ev - S_i_dep - S_s_dep - S_nuc;
             a.S_c[c] = S_c_c - S_c_au - S_ac - S_c_frz + S_i_melt - S_rim - S_shed;
             a.S_i[c] = S_nuc + S_c_frz + S_i_dep - S_i_melt - S_i_au - S_d_au - S_agg - S_i_cri;
@@ -186,14 +209,16 @@ __global__ void __launch_bounds__(128) ice_columns_kernel(IceArgs a)
             a.S_s[c] = S_i_au + S_d_au + S_agg + S_rim + S_s_dep + S_i_cri + S_r_cri + S_r_frz - S_s_melt;
             // the fluxes, integrated top-down and capped at 50 mm/d (:478-509)
             const double dP_rain = (S_c_au + S_ac + S_shed + S_s_melt - S_ev - S_r_frz) * mass_layer;
-            const double pr = dmin(P_max, dmax(0.0, a.P_rain[c + sI] + dP_rain));
+            const double pr = dmin(P_max, dmax(0.0, rain_above + dP_rain));
             a.P_rain[c] = pr;
             const double dP_snow = (S_i_au + S_d_au + S_rim + S_agg + S_r_frz - S_s_melt) * mass_layer;
-            const double ps = (t_u < t_0 && t_u >= a.t_000) ? dmin(P_max, dmax(0.0, a.P_snow[c + sI] + dP_snow)) : 0.0;
+            const double ps = (t_u < t_0 && t_u >= a.t_000) ? dmin(P_max, dmax(0.0, snow_above + dP_snow)) : 0.0;
             a.P_snow[c] = ps;
             a.Precipitation[c] = dmin(P_max, pr + ps);
+            rain_above = pr; snow_above = ps;
+            if (i == kIcheck) P_rain_check = pr;
         }
-        const double P_rain_diff = fabs(a.P_rain[idx3(d, kIcheck, j, k)] - Rain_check) * 8.64e4;
+        const double P_rain_diff = fabs(P_rain_check - Rain_check) * 8.64e4;
         if (P_rain_diff <= 1.0e-3) break;
     }
 }
@@ -243,7 +268,6 @@ __global__ void ice_bc_seam_kernel(Dims d, PrecipBc b)
 void launch_two_cat_ice(const IceArgs& a, cudaStream_t st)
 {
     const Dims& d = a.d;
-    ice_init_kernel<<<148 * 8, 256, 0, st>>>(a);
     ice_columns_kernel<<<dim3((d.km + 127) / 128, d.jm), 128, 0, st>>>(a);
     double* P[3] = {a.P_rain, a.P_snow, nullptr};
     const int avg[3] = {1, 1, 0};

@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kScanThreads) one_cat_scan_kernel(IceArgs a, l
     }
 }
 
-__global__ void __launch_bounds__(128) one_cat_columns_kernel(IceArgs a)
+__global__ void __launch_bounds__(128, 4) one_cat_columns_kernel(IceArgs a)
 {
     const Dims& d = a.d;
     int j, k;
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(128) one_cat_columns_kernel(IceArgs a)
 // ---------------------------------------------------------------------------------------
 // ThreeCatIceScheme::computeColumns (ThreeCatIceScheme.h:147-420)
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) three_cat_columns_kernel(IceArgs a)
+__global__ void __launch_bounds__(128, 4) three_cat_columns_kernel(IceArgs a)
 {
     const Dims& d = a.d;
     int j, k;
