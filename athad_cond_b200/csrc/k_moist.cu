@@ -389,6 +389,7 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
     }
     if (interior) cloud_base_update(X, j, k, i_deep_beg, i_lfs, &i_base);
 
+    int i_eu = im;
     for (int ip = 1; ip <= p->iter_prec; ip++) {
         /* updraftEntrainment, :780-908 (interior columns) */
         if (interior && !(i_base < 0 || i_lfs <= i_base)) {
@@ -407,20 +408,39 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
             }
             M_d_LFS = clamp_M(MC_GAM_D * p->F[ATHAD_M_U][IDX(ib, j, k)]);
             double Mu_m = p->F[ATHAD_M_U][IDX(ib, j, k)];   // level i-1 as this loop left it
+            // The advective part of the entrainment reads only fields that this routine does
+            // not write, so a level forms it in its first pass and leaves it in MC_t (which
+            // rhsForcing writes for every level below im - 1 at the end) for the later ones.
+            // The next level's values are loaded while this level computes.
+            const bool deep = (pb - pl) >= MC_F_DIFF * p0;
+            struct In { double T, Rh, Mu, qcu, eu; } nxt{};
+            auto load = [&](int i) {
+                const long long c = IDX(i, j, k);
+                In v;
+                v.T = p->F[ATHAD_T][c]; v.Rh = p->F[ATHAD_R_HUMID][c];
+                v.Mu = p->F[ATHAD_M_U][c];           // the previous pass's mass flux here
+                v.qcu = p->F[ATHAD_Q_C_U][c];        // not written by this loop
+                v.eu = 0.0;
+                if (deep) {
+                    if (ip > 1 && i >= i_eu) {
+                        v.eu = p->F[ATHAD_MC_T][c];
+                    } else {
+                        const double Uc = p->F[ATHAD_U][c], Vc = p->F[ATHAD_V][c], Wc = p->F[ATHAD_W][c];
+                        double dcdr, dcdthe, dcdphi, c_ijk;
+                        entrainment_gradients(X, i, j, k, &dcdr, &dcdthe, &dcdphi, &c_ijk);
+                        v.eu = -v.Rh / c_ijk * (Uc * dcdr + Vc * dcdthe + Wc * dcdphi);
+                    }
+                }
+                return v;
+            };
+            if (ib + 1 <= il) nxt = load(ib + 1);
             for (int i = ib + 1; i <= il; i++) {
                 const long long c = IDX(i, j, k);
+                const In v = nxt;
+                if (i + 1 <= il) nxt = load(i + 1);
                 const double height_i = p->height[i];
-                const double t_u = p->F[ATHAD_T][c] * t_0, r_h_i = p->F[ATHAD_R_HUMID][c];
-                double dcdr, dcdthe, dcdphi, c_ijk;
-                entrainment_gradients(X, i, j, k, &dcdr, &dcdthe, &dcdphi, &c_ijk);
-                const double Mu_c = p->F[ATHAD_M_U][c];   // the previous pass's mass flux here
-                const double qcu_c = p->F[ATHAD_Q_C_U][c];  // not written by this loop
-                double eu;
-                if ((pb - pl) >= MC_F_DIFF * p0)
-                    eu = -r_h_i / c_ijk * (p->F[ATHAD_U][c] * dcdr + p->F[ATHAD_V][c] * dcdthe + p->F[ATHAD_W][c] * dcdphi)
-                         + MC_EPS_U * Mu_c;
-                else
-                    eu = 0.0;
+                const double t_u = v.T * t_0, r_h_i = v.Rh, Mu_c = v.Mu, qcu_c = v.qcu;
+                double eu = deep ? v.eu + MC_EPS_U * Mu_c : 0.0;
                 if (t_u <= MC_T00M2) eu = 0.0;
                 double du = (i <= il) ? MC_EPS_U * Mu_c : 0.0;
                 if (ip > 1 && i == il)
@@ -430,6 +450,7 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 if (t_u <= MC_T00M2) du = 0.0;
                 const double d_Mu = eu - du;
                 const double Mu = clamp_M(Mu_m + d_Mu * p->step[i]);
+                p->F[ATHAD_MC_T][c] = v.eu;
                 p->F[ATHAD_E_U][c] = eu;
                 p->F[ATHAD_D_U][c] = du;
                 p->F[ATHAD_M_U][c] = Mu;
@@ -447,6 +468,7 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 if (t_u >= t_0) p->F[ATHAD_G_P][c] = (ip == 1) ? 0.0 : K_p * qcu_c;
                 else p->F[ATHAD_G_P][c] = 0.0;
             }
+            i_eu = ib + 1;   // levels from here on hold theirs (the base only moves down)
             p->F[ATHAD_M_U][IDX(il, j, k)] = 0.0;
         }
         if (interior) cloud_base_update(X, j, k, i_deep_beg, i_lfs, &i_base);
@@ -463,24 +485,41 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
             double eu_m = p->F[ATHAD_E_U][cb], du_m = p->F[ATHAD_D_U][cb], gp_m = p->F[ATHAD_G_P][cb];
             const double inv_a_u = 1.0 / (MC_A_U * p->u_0);
             const double cap = MC_W_CONV_MAX / p->u_0;
+            // the environment of a level and the entrainment's values there, loaded while the
+            // level below computes; a level stores its own cells only
+            struct Env { double T, Rh, C, CL, V, W, U, S, P, CO2, E, D, G; } prev, cur, nxt{};
+            auto load = [&](int i) {
+                const long long c = IDX(i, j, k);
+                Env v;
+                v.T = p->F[ATHAD_T][c]; v.Rh = p->F[ATHAD_R_HUMID][c]; v.C = p->F[ATHAD_C][c];
+                v.CL = p->F[ATHAD_CLOUD][c]; v.V = p->F[ATHAD_V][c]; v.W = p->F[ATHAD_W][c];
+                v.U = p->F[ATHAD_U][c]; v.S = p->F[ATHAD_MC_S][c]; v.P = p->F[ATHAD_P_STAT][c];
+                v.CO2 = p->F[ATHAD_CO2][c];
+                v.E = p->F[ATHAD_E_U][c]; v.D = p->F[ATHAD_D_U][c]; v.G = p->F[ATHAD_G_P][c];
+                return v;
+            };
+            prev = load(i_base);
+            if (i_base + 1 <= i_lfs - 1) nxt = load(i_base + 1);
             for (int i = i_base + 1; i <= i_lfs - 1; i++) {
-                const long long c = IDX(i, j, k), cm = IDX(i - 1, j, k);
-                const double t_u = p->F[ATHAD_T][cm] * t_0;
-                const double r_h_prev = p->F[ATHAD_R_HUMID][cm];
+                const long long c = IDX(i, j, k);
+                cur = nxt;
+                if (i + 1 <= i_lfs - 1) nxt = load(i + 1);
+                const double t_u = prev.T * t_0;
+                const double r_h_prev = prev.Rh;
                 const double step_prev = p->step[i - 1];
-                const double r_h_i = p->F[ATHAD_R_HUMID][c];
+                const double r_h_i = cur.Rh;
                 const double d_Mu = eu_m - du_m;
                 double Mu = clamp_M(Mu_m + d_Mu * step_prev);
                 if (t_u <= MC_T00M2) Mu = 0.0;
                 const double M_u_prev = Mu_m;
                 const double dq_v = M_u_prev * qvu_m
-                    + step_prev * (eu_m * p->F[ATHAD_C][cm] - du_m * qvu_m);
+                    + step_prev * (eu_m * prev.C - du_m * qvu_m);
                 const double dq_c = M_u_prev * qcu_m
-                    + step_prev * (-du_m * p->F[ATHAD_CLOUD][cm] - r_h_prev * gp_m);
-                const double dv = M_u_prev * vu_m + step_prev * eu_m * p->F[ATHAD_V][cm];
-                const double dw = M_u_prev * wu_m + step_prev * eu_m * p->F[ATHAD_W][cm];
+                    + step_prev * (-du_m * prev.CL - r_h_prev * gp_m);
+                const double dv = M_u_prev * vu_m + step_prev * eu_m * prev.V;
+                const double dw = M_u_prev * wu_m + step_prev * eu_m * prev.W;
                 const double ds = (M_u_prev * su_m
-                    + step_prev * (eu_m * p->F[ATHAD_MC_S][cm] - du_m * su_m)) / p->s_0;
+                    + step_prev * (eu_m * prev.S - du_m * su_m)) / p->s_0;
                 double qvu, qcu, vu, wu, su;
                 if (fabs(Mu) > MC_COEFF_RECURR) {
                     const double inv = 1.0 / Mu;
@@ -490,24 +529,24 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                     wu = dw * inv;
                     su = ds * inv;
                 } else {
-                    su = p->F[ATHAD_MC_S][c];
-                    qvu = p->F[ATHAD_C][c];
+                    su = cur.S;
+                    qvu = cur.C;
                     qcu = 0.0;
-                    vu = p->F[ATHAD_V][c];
-                    wu = p->F[ATHAD_W][c];
+                    vu = cur.V;
+                    wu = cur.W;
                 }
                 double cu = 0.0;
                 if (fabs(Mu) > MC_COEFF_RECURR) {
                     double T_u = su * p->s_0 / p->cp_l;
-                    const double p_u = p->F[ATHAD_P_STAT][c];
+                    const double p_u = cur.P;
                     double dcond_tot = 0.0;
                     for (int it = 0; it < 2; ++it) {
                         const double E_s = saturation_pressure_auto(T_u);
-                        const double q_sat_u = safe_q_sat(X, E_s, p_u, p->F[ATHAD_C][c]);
+                        const double q_sat_u = safe_q_sat(X, E_s, p_u, cur.C);
                         const double dq = qvu - q_sat_u;
                         if (dq <= 0.0) break;
                         const double L_u = (T_u >= t_0) ? p->lv : p->ls;
-                        const double M_o_u = M_nonwater(p->F[ATHAD_C][c], p->F[ATHAD_CO2][c], p->M_bg);
+                        const double M_o_u = M_nonwater(cur.C, cur.CO2, p->M_bg);
                         const double dqsdT = dqsat_dT_from(E_s, latent_heat_auto(T_u), T_u, p_u, M_o_u);
                         const double G = (L_u / p->cp_l) * dqsdT;
                         const double dcond = dq / (1.0 + G);
@@ -519,13 +558,13 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                     su = p->cp_l * T_u / p->s_0;
                     cu = dcond_tot * Mu / (smax(r_h_i, 0.01) * p->step[i]);
                 }
-                double uu = p->F[ATHAD_U][c] + Mu * inv_a_u / safe_r_humid(r_h_i);
+                double uu = cur.U + Mu * inv_a_u / safe_r_humid(r_h_i);
                 uu = smax(-cap, smin(uu, cap));
                 if (qvu <= 0.0) qvu = 0.0;
                 if (qcu <= 0.0) qcu = 0.0;
                 if (qcu > MC_Q_C_U_MAX) qcu = MC_Q_C_U_MAX;
                 if (su <= 0.0) su = 0.0;
-                double eu = p->F[ATHAD_E_U][c], du = p->F[ATHAD_D_U][c], gp = p->F[ATHAD_G_P][c];
+                double eu = cur.E, du = cur.D, gp = cur.G;
                 if (t_u <= MC_T00) {
                     eu = 0.0; du = 0.0; Mu = 0.0;
                     qvu = 0.0; qcu = 0.0;
@@ -541,6 +580,7 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 p->F[ATHAD_MC_S_U][c] = su; p->F[ATHAD_C_U][c] = cu; p->F[ATHAD_U_U][c] = uu;
                 Mu_m = Mu; qvu_m = qvu; qcu_m = qcu; vu_m = vu; wu_m = wu; su_m = su;
                 eu_m = eu; du_m = du; gp_m = gp;
+                prev = cur;
             }
         }
 
@@ -576,18 +616,37 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
             // in a register.  The differences that the serial order forms from stored and
             // reloaded products are formed without contraction into a fused multiply-add.
             double Md_up = p->F[ATHAD_M_D][cl];
+            // The next level's values are loaded while this level computes.  The saturation
+            // value depends on nothing that this routine writes: a level forms it in the first
+            // pass and leaves it in MC_q (rhsForcing writes that at the end) for the others.
+            struct In { double P, T, Rh, C, CL, Md, U, V, W, Pc, ep, qs; } nxt{};
+            auto load = [&](int i) {
+                const long long c = IDX(i, j, k);
+                In v;
+                v.P = (ip == 1) ? p->F[ATHAD_P_STAT][c] : 0.0;
+                v.T = p->F[ATHAD_T][c]; v.Rh = p->F[ATHAD_R_HUMID][c];
+                v.C = (ip == 1) ? p->F[ATHAD_C][c] : 0.0;
+                v.CL = p->F[ATHAD_CLOUD][c]; v.Md = p->F[ATHAD_M_D][c];
+                v.U = p->F[ATHAD_U][c]; v.V = p->F[ATHAD_V][c]; v.W = p->F[ATHAD_W][c];
+                v.Pc = p->F[ATHAD_P_CONV][c]; v.ep = p->F[ATHAD_E_P][c];
+                v.qs = (ip == 1) ? 0.0 : p->F[ATHAD_MC_Q][c];
+                return v;
+            };
+            if (il - 1 >= 0) nxt = load(il - 1);
             for (int i = il - 1; i >= 0; i--) {
                 const long long c = IDX(i, j, k);
-                p_u = p->F[ATHAD_P_STAT][c];
-                t_u = p->F[ATHAD_T][c] * t_0;
-                const double r_h_i = p->F[ATHAD_R_HUMID][c];
-                const double Cc = p->F[ATHAD_C][c], CLc = p->F[ATHAD_CLOUD][c];
-                const double Md_old = p->F[ATHAD_M_D][c];
-                const double Uc = p->F[ATHAD_U][c], Vc = p->F[ATHAD_V][c], Wc = p->F[ATHAD_W][c];
-                const double precip_i = p->F[ATHAD_P_CONV][c];
-                const double ep_old = p->F[ATHAD_E_P][c];
+                const In v = nxt;
+                if (i - 1 >= 0) nxt = load(i - 1);
+                p_u = v.P;
+                t_u = v.T * t_0;
+                const double r_h_i = v.Rh, Cc = v.C, CLc = v.CL, Md_old = v.Md;
+                const double Uc = v.U, Vc = v.V, Wc = v.W, precip_i = v.Pc, ep_old = v.ep;
                 p->F[ATHAD_MC_S_D][c] = p->cp_l * t_u / p->s_0;
-                const double q_sat = safe_q_sat(X, saturation_pressure_auto(t_u), p_u, Cc);
+                double q_sat = v.qs;
+                if (ip == 1) {
+                    q_sat = safe_q_sat(X, saturation_pressure_auto(t_u), p_u, Cc);
+                    p->F[ATHAD_MC_Q][c] = q_sat;
+                }
                 const double qvd = 0.5 * (CLc + MC_SCALE * q_sat);
                 p->F[ATHAD_Q_V_D][c] = qvd;
                 const double ed = MC_EPS_D * fabs(Md_old);
@@ -640,24 +699,40 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
             double ed_p = p->F[ATHAD_E_D][c0], dd_p = p->F[ATHAD_D_D][c0], edd_p = p->F[ATHAD_E_DD][c0];
             double pconv_p = p->F[ATHAD_P_CONV][c0], rh_p = p->F[ATHAD_R_HUMID][c0];
             const double inv_a_d = 1.0 / (MC_A_D * p->u_0);
+            // a level's environment, loaded while the level above computes
+            struct Env { double T, Rh, C, V, W, U, S, G, E, D, edd, ep; } up, cur, nxt{};
+            auto load = [&](int i) {
+                const long long c = IDX(i, j, k);
+                Env v;
+                v.T = p->F[ATHAD_T][c]; v.Rh = p->F[ATHAD_R_HUMID][c]; v.C = p->F[ATHAD_C][c];
+                v.V = p->F[ATHAD_V][c]; v.W = p->F[ATHAD_W][c]; v.U = p->F[ATHAD_U][c];
+                v.S = p->F[ATHAD_MC_S][c]; v.G = p->F[ATHAD_G_P][c];   // not written by this loop
+                v.E = p->F[ATHAD_E_D][c]; v.D = p->F[ATHAD_D_D][c];
+                v.edd = p->F[ATHAD_E_DD][c]; v.ep = p->F[ATHAD_E_P][c];
+                return v;
+            };
+            up = load(i_lfs);
+            if (i_lfs - 1 >= 0) nxt = load(i_lfs - 1);
             for (int i = i_lfs - 1; i >= 0; i--) {
-                const long long c = IDX(i, j, k), cp = IDX(i + 1, j, k);
-                const double t_u = p->F[ATHAD_T][c] * t_0;
-                const double gp_c = p->F[ATHAD_G_P][c];   // not written by this loop
+                const long long c = IDX(i, j, k);
+                cur = nxt;
+                if (i - 1 >= 0) nxt = load(i - 1);
+                const double t_u = cur.T * t_0;
+                const double gp_c = cur.G;
                 const double step_ip1 = p->step[i + 1];
-                const double r_h_ip1 = rh_p, r_h_i = p->F[ATHAD_R_HUMID][c];
-                double ed = p->F[ATHAD_E_D][c], dd = p->F[ATHAD_D_D][c];
+                const double r_h_ip1 = rh_p, r_h_i = cur.Rh;
+                double ed = cur.E, dd = cur.D;
                 const double d_Md = ed - dd;
                 double Md = clamp_M(Md_p - d_Md * step_ip1);
                 if (t_u <= MC_T00M2) Md = 0.0;
                 const double L_latent = (t_u >= t_0) ? p->lv : p->ls;
                 const double M_d_ip1 = Md_p;
                 const double dq_v = M_d_ip1 * qvd_p
-                    - step_ip1 * (ed_p * p->F[ATHAD_C][cp] - dd_p * qvd_p + r_h_ip1 * edd_p);
-                const double dv = M_d_ip1 * vd_p - step_ip1 * (ed_p * p->F[ATHAD_V][cp] - dd_p * vd_p);
-                const double dw = M_d_ip1 * wd_p - step_ip1 * (ed_p * p->F[ATHAD_W][cp] - dd_p * wd_p);
+                    - step_ip1 * (ed_p * up.C - dd_p * qvd_p + r_h_ip1 * edd_p);
+                const double dv = M_d_ip1 * vd_p - step_ip1 * (ed_p * up.V - dd_p * vd_p);
+                const double dw = M_d_ip1 * wd_p - step_ip1 * (ed_p * up.W - dd_p * wd_p);
                 const double ds = (M_d_ip1 * sd_p
-                    - step_ip1 * (ed_p * p->F[ATHAD_MC_S][cp] - dd_p * sd_p - L_latent * r_h_ip1 * edd_p)) / p->s_0;
+                    - step_ip1 * (ed_p * up.S - dd_p * sd_p - L_latent * r_h_ip1 * edd_p)) / p->s_0;
                 double qvd, vd, wd, sd;
                 if (fabs(Md) > MC_COEFF_RECURR) {
                     const double inv = 1.0 / Md;
@@ -666,15 +741,15 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                     wd = dw * inv;
                     sd = ds * inv;
                 } else {
-                    qvd = p->F[ATHAD_C][c];
-                    vd = p->F[ATHAD_V][c];
-                    wd = p->F[ATHAD_W][c];
-                    sd = p->F[ATHAD_MC_S][c];
+                    qvd = cur.C;
+                    vd = cur.V;
+                    wd = cur.W;
+                    sd = cur.S;
                 }
-                double ud = p->F[ATHAD_U][c] + Md * inv_a_d / safe_r_humid(r_h_i);
+                double ud = cur.U + Md * inv_a_d / safe_r_humid(r_h_i);
                 if (qvd <= 0.0) qvd = 0.0;
                 if (sd <= 0.0) sd = 0.0;
-                double edd = p->F[ATHAD_E_DD][c], ep = p->F[ATHAD_E_P][c];
+                double edd = cur.edd, ep = cur.ep;
                 if (t_u <= MC_T00) {
                     ed = 0.0; dd = 0.0; Md = 0.0;
                     qvd = 0.0;
@@ -693,6 +768,7 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 }
                 Md_p = Md; qvd_p = qvd; vd_p = vd; wd_p = wd; sd_p = sd;
                 ed_p = ed; dd_p = dd; edd_p = edd; pconv_p = pconv; rh_p = r_h_i;
+                up = cur;
             }
         }
         p->F[ATHAD_P_CONV][IDX(0, j, k)] = p->F[ATHAD_P_CONV][IDX(1, j, k)];
@@ -704,30 +780,53 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
     auto clamp3 = [](double v) { return !is_finite_bits(v) ? 0.0 : (v < -3.0) ? -3.0 : (v > 3.0) ? 3.0 : v; };
     // the four mass fluxes at a level; level i+1's are level i's upper fluxes and the next
     // level's lower ones, so each is formed once and carried (same operands, same values)
-    auto flux_at = [&](long long c, double& fs, double& fq, double& fv, double& fw) {
-        const double Mu = clamp3(p->F[ATHAD_M_U][c]), Md = clamp3(p->F[ATHAD_M_D][c]);
-        const double su = p->F[ATHAD_MC_S_U][c], sm = p->F[ATHAD_MC_S][c], sd = p->F[ATHAD_MC_S_D][c];
-        const double qu = p->F[ATHAD_Q_V_U][c], qm = p->F[ATHAD_C][c], qd = p->F[ATHAD_Q_V_D][c];
-        const double vu = p->F[ATHAD_V_U][c], vm = p->F[ATHAD_V][c], vd = p->F[ATHAD_V_D][c];
-        const double wu = p->F[ATHAD_W_U][c], wm = p->F[ATHAD_W][c], wd = p->F[ATHAD_W_D][c];
+    struct Flux { double Mu, Md, su, sm, sd, qu, qm, qd, vu, vm, vd, wu, wm, wd; } fl;
+    auto load_flux = [&](int i) {
+        const long long c = IDX(i, j, k);
+        Flux v;
+        v.Mu = p->F[ATHAD_M_U][c]; v.Md = p->F[ATHAD_M_D][c];
+        v.su = p->F[ATHAD_MC_S_U][c]; v.sm = p->F[ATHAD_MC_S][c]; v.sd = p->F[ATHAD_MC_S_D][c];
+        v.qu = p->F[ATHAD_Q_V_U][c]; v.qm = p->F[ATHAD_C][c]; v.qd = p->F[ATHAD_Q_V_D][c];
+        v.vu = p->F[ATHAD_V_U][c]; v.vm = p->F[ATHAD_V][c]; v.vd = p->F[ATHAD_V_D][c];
+        v.wu = p->F[ATHAD_W_U][c]; v.wm = p->F[ATHAD_W][c]; v.wd = p->F[ATHAD_W_D][c];
+        return v;
+    };
+    auto flux_at = [&](long long c, const Flux& v, double& fs, double& fq, double& fv, double& fw) {
+        const double Mu = clamp3(v.Mu), Md = clamp3(v.Md);
         p->F[ATHAD_M_U][c] = Mu;
         p->F[ATHAD_M_D][c] = Md;
-        fs = Mu * (su - sm) + Md * (sd - sm);
-        fq = Mu * (qu - qm) + Md * (qd - qm);
-        fv = Mu * (vu - vm) + Md * (vd - vm);
-        fw = Mu * (wu - wm) + Md * (wd - wm);
+        fs = Mu * (v.su - v.sm) + Md * (v.sd - v.sm);
+        fq = Mu * (v.qu - v.qm) + Md * (v.qd - v.qm);
+        fv = Mu * (v.vu - v.vm) + Md * (v.vd - v.vm);
+        fw = Mu * (v.wu - v.wm) + Md * (v.wd - v.wm);
+    };
+    // the level's forcing values and the fluxes of the level after next, loaded while this
+    // level computes
+    struct Src { double T, Rh, cu, edd, el, ep; } sc;
+    auto load_src = [&](int i) {
+        const long long c = IDX(i, j, k);
+        return Src{p->F[ATHAD_T][c], p->F[ATHAD_R_HUMID][c], p->F[ATHAD_C_U][c], p->F[ATHAD_E_DD][c],
+                   p->F[ATHAD_E_L][c], p->F[ATHAD_E_P][c]};
     };
     double fs0, fq0, fv0, fw0;
-    flux_at(IDX(0, j, k), fs0, fq0, fv0, fw0);
+    fl = load_flux(0);
+    sc = load_src(0);
+    {
+        const Flux f0 = fl;
+        fl = load_flux(1);
+        flux_at(IDX(0, j, k), f0, fs0, fq0, fv0, fw0);
+    }
     for (int i = 0; i < im - 1; i++) {
         const long long c = IDX(i, j, k), cp = IDX(i + 1, j, k);
-        const double Tc = p->F[ATHAD_T][c], Rc = p->F[ATHAD_R_HUMID][c];
-        const double cu = p->F[ATHAD_C_U][c], edd = p->F[ATHAD_E_DD][c];
-        const double el = p->F[ATHAD_E_L][c], ep = p->F[ATHAD_E_P][c];
+        const Flux f1 = fl;
+        const Src s0 = sc;
+        if (i + 2 < im) fl = load_flux(i + 2);
+        if (i + 1 < im - 1) sc = load_src(i + 1);
+        const double Tc = s0.T, Rc = s0.Rh, cu = s0.cu, edd = s0.edd, el = s0.el, ep = s0.ep;
         const double L_latent = (Tc * t_0 >= t_0) ? p->lv : p->ls;
         const double inv_step_rh = 1.0 / (p->step[i] * smax(Rc, 0.01));
         double fs1, fq1, fv1, fw1;
-        flux_at(cp, fs1, fq1, fv1, fw1);
+        flux_at(cp, f1, fs1, fq1, fv1, fw1);
         const double conv_src = cu - edd - el - ep;
         double v = -(fs1 - fs0) * inv_step_rh * t_0 + (L_latent / p->cp_l) * conv_src * t_0;
         p->F[ATHAD_MC_T][c] = !is_finite_bits(v) ? 0.0 : (v < -0.01) ? -0.01 : (v > 0.01) ? 0.01 : v;
@@ -746,7 +845,12 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
 #define ATHAD_MC_BLOCK 128   // columns per CTA
 #endif
 
-__global__ void __launch_bounds__(ATHAD_MC_BLOCK) moist_convection_kernel(const MoistArgs X)
+// 128 registers: the columns of 41x181x361 (3.7 CTAs per SM) in one wave.  A warp spends
+// its time on one level after another, so each level's operands are loaded while the level
+// before it computes, and what does not change between the iter_prec passes (the advective
+// entrainment, the downdraft's saturation value) is formed once: 1310 -> 1020 us on a
+// convecting state; without the register limit (160: two waves) 1570.
+__global__ void __launch_bounds__(ATHAD_MC_BLOCK, 512 / ATHAD_MC_BLOCK) moist_convection_kernel(const MoistArgs X)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
