@@ -73,30 +73,33 @@ __host__ __device__ __forceinline__ double p_subl_r(double T, double invT)
 {
     if (T <= 0.0) return 0.0;
     const double lt = log(T * (1.0 / T_TRIPLE));
-    const double sum = -0.212144006e2 * exp(0.333333333e-2 * lt)
-                     + 0.273203819e2 * exp(0.120666667e1 * lt)
+    // theta^(1/300): the exponent is within 0.004 for T of 82 to 907 K, where the series to
+    // the fifth power is exact to less than an ulp (x^6 / 720 < 6e-18)
+    const double x = 0.333333333e-2 * lt;
+    const double r = (fabs(x) < 0.004)
+        ? 1.0 + x * (1.0 + x * (0.5 + x * (1.0 / 6.0 + x * (1.0 / 24.0 + x * (1.0 / 120.0))))) : exp(x);
+    const double sum = -0.212144006e2 * r + 0.273203819e2 * exp(0.120666667e1 * lt)
                      + -0.610598130e1 * exp(0.170333333e1 * lt);
     return 6.11657 * exp(sum * (T_TRIPLE * invT));
 }
-__host__ __device__ __forceinline__ double q_sat_r(double E, double p, double inv_p, double M_other)
+// saturation mass fraction and its derivative factor (dq_sat/dT = A L / (R_H2O T^2)) from one
+// division.  The Newton step issues its instructions at 70 % of the rate (no loads to wait
+// for), so its count is its time: this, the shared cp and the 1/T of the heat capacities take
+// it from 12 divisions to 6 (704 -> 610 us for the kernel, 527 -> 479 M warp instructions;
+// most cells, four of five, take 3 to 5 steps, and the ice curve is needed in nearly all of
+// them because transport leaves traces of ice everywhere)
+struct SatValue { double q, A; };
+__host__ __device__ __forceinline__ SatValue sat_value(double E, double p, double inv_p, double M_other)
 {
-    if (E == NO_SATURATION) return 1.0;
-    if (!(p > 0.0)) return 0.0;
-    if (E >= p) return 1.0;
+    if (E == NO_SATURATION) return {1.0, 0.0};
+    if (!(p > 0.0)) return {0.0, 0.0};
+    if (E >= p) return {1.0, 0.0};
     const double x = E * inv_p;
     const double num = x * M_H2O;
     const double den = num + (1.0 - x) * M_other;
-    return (den > 0.0) ? num / den : 1.0;
-}
-__host__ __device__ __forceinline__ double dqsat_r(double E, double L, double T, double invT, double p,
-                                                   double inv_p, double M_other)
-{
-    if (!(T > 0.0)) return 0.0;
-    if (E == NO_SATURATION || !(p > 0.0) || E >= p) return 0.0;
-    const double x = E * inv_p;
-    const double den = x * M_H2O + (1.0 - x) * M_other;
-    if (!(den > 0.0)) return 0.0;
-    return x * M_H2O * M_other / (den * den) * L * (invT * invT) * (1.0 / R_H2O);
+    if (!(den > 0.0)) return {1.0, 0.0};
+    const double r = 1.0 / den;
+    return {num * r, num * M_other * (r * r)};
 }
 // The mixture heat capacity of the Newton step (MixtureAtm.h:123-178) with the three
 // Shomate polynomials sharing t, t^2, t^3 and 1/t^2, and products by the reciprocal molar
@@ -104,10 +107,11 @@ __host__ __device__ __forceinline__ double dqsat_r(double E, double L, double T,
 // components at T (shomate_r), and their mixture (cp_mix), so a Newton step that moves the
 // composition but not T reuses the first.
 struct SpecificHeats { double h2o, co2, bg; };
-__host__ __device__ __forceinline__ SpecificHeats shomate_r(double T, double inv_M_b)
+__host__ __device__ __forceinline__ SpecificHeats shomate_r(double T, double invT, double inv_M_b)
 {
     const double t = smin(smax(T, 298.0), 2000.0) * 1.0e-3;
-    const double t2 = t * t, t3 = t2 * t, it2 = 1.0 / t2;
+    const double t2 = t * t, t3 = t2 * t;
+    const double it2 = (T < 298.0) ? 1.0 / (0.298 * 0.298) : (T > 2000.0) ? 0.25 : 1.0e6 * (invT * invT);
     const double h2o = 30.09200 + 6.832514 * t + 6.793435 * t2 + -2.534480 * t3 + 0.082139 * it2;
     const double co2s = 24.99735 + 55.18696 * t + -33.69137 * t2 + 7.948387 * t3 + -0.136638 * it2;
     const double bg = 28.98641 + 1.853978 * t + -9.647459 * t2 + 16.63537 * t3 + 0.000117 * it2;
@@ -128,7 +132,9 @@ __host__ __device__ __forceinline__ double cp_mix(double c, double co2, const Sp
 // the densities) in a few cells within 300 iterations; in FP64 the mixed form stays within
 // 1e-9 of the FP64 form in c and cloud over the same iterations.
 #ifndef ATHAD_SATADJ_MIN_BLOCKS
-#define ATHAD_SATADJ_MIN_BLOCKS 7         // 72 registers, 7 CTAs of 128 threads per SM
+#define ATHAD_SATADJ_MIN_BLOCKS 8         // 64 registers, 8 CTAs of 128 threads per SM: 653 us
+                                          // per call (with the four uploads) at 41x181x361
+                                          // before a moist iteration, 660 at 7, 664 at 6
 #endif
 // One cell (i, j, k < km) of the fused pass; returns whether the vapour hit its 1 - co2 cap.
 // __host__ __device__: tests/host_columns.cu runs the same source on the host.
@@ -169,7 +175,7 @@ __host__ __device__ __forceinline__ bool satadj_cell(const ColumnArgs& a, int i,
                     double L_T = latent_heat(T);
                     const double inv_p = 1.0 / p_local;
                     const double inv_M_b = 1.0 / a.M_bg;
-                    SpecificHeats sh = shomate_r(T, inv_M_b);   // at the T of the step's start
+                    SpecificHeats sh = shomate_r(T, 1.0 / T, inv_M_b);   // at the T of the step's start
                     for (int iter = 1; iter <= 20; iter++) {
                         const double CND = smax(0.0, smin(1.0, (T - a.t_00) * t_range_inv));
                         const double DEP = 1.0 - CND;
@@ -185,24 +191,24 @@ __host__ __device__ __forceinline__ bool satadj_cell(const ColumnArgs& a, int i,
                         const double cp_loc = cp_mix(q_v_b, co2, sh);
                         T -= (L_T * d_cnd + (L_T + 3.337e5) * d_dep) / cp_loc;
                         const double invT = 1.0 / T;
-                        const double E_sat = p_sat_r(T, invT);
-                        const double q_sat = q_sat_r(E_sat, p_local, inv_p, M_other);
+                        const SatValue liq = sat_value(p_sat_r(T, invT), p_local, inv_p, M_other);
                         const double q_sum = q_c_b + q_i_b;
                         const bool need_ice = (DEP != 0.0) || (q_i_b > 0.0) || (!(q_sum > 1e-12) && !(T >= a.t_0));
-                        const double E_Ice = need_ice ? p_subl_r(T, invT) : 0.0;
-                        const double q_Ice = need_ice ? q_sat_r(E_Ice, p_local, inv_p, M_other) : 0.0;
-                        const double q_v_target = (q_sum > 1e-12) ? (q_c_b * q_sat + q_i_b * q_Ice) / q_sum
-                                                                  : ((T >= a.t_0) ? q_sat : q_Ice);
-                        sh = shomate_r(T, inv_M_b);   // the updated T: the next step starts from it
+                        SatValue sol{0.0, 0.0};
+                        if (need_ice) sol = sat_value(p_subl_r(T, invT), p_local, inv_p, M_other);
+                        const double q_v_target = (q_sum > 1e-12) ? (q_c_b * liq.q + q_i_b * sol.q) / q_sum
+                                                                  : ((T >= a.t_0) ? liq.q : sol.q);
+                        sh = shomate_r(T, invT, inv_M_b);   // the updated T: the next step starts from it
                         const double cp_g = cp_mix(q_v_b, co2, sh);
                         const double L_cnd = latent_heat(T);
                         const double L_dep = L_cnd + 3.337e5;
-                        double Gain = CND * (L_cnd / cp_g) * dqsat_r(E_sat, L_cnd, T, invT, p_local, inv_p, M_other);
-                        if (need_ice) Gain += DEP * (L_dep / cp_g) * dqsat_r(E_Ice, L_dep, T, invT, p_local, inv_p, M_other);
                         L_T = L_cnd;
-                        const double omega = 1.0 / (1.0 + Gain);
-                        q_v_hyp = q_v_b + omega * (q_v_target - q_v_b);
-                        if (fabs(q_v_b / q_v_hyp - 1.0) <= 1.0e-6) break;
+                        // 1 / (1 + Gain) with Gain = sum of weight L / cp_g dq_sat/dT: one division
+                        const double S = (CND * (L_cnd * L_cnd) * liq.A + DEP * (L_dep * L_dep) * sol.A)
+                                       * ((invT * invT) * (1.0 / R_H2O));
+                        q_v_hyp = q_v_b + (q_v_target - q_v_b) * cp_g / (cp_g + S);
+                        // |q_v_b / q_v_hyp - 1| <= 1e-6
+                        if (fabs(q_v_b - q_v_hyp) <= 1.0e-6 * fabs(q_v_hyp) && q_v_hyp != 0.0) break;
                     }
                     q_c_b = smax(0.0, q_c_b);
                     q_i_b = smax(0.0, q_i_b);
