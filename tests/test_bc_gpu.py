@@ -63,3 +63,24 @@ def test_boundary_conditions_keep_mirror_symmetry():
         for n in FIELD_NAMES:
             a = g.download(n)
             assert np.array_equal(a, mirror(a, n in ANTI)), n
+
+
+@pytest.mark.parametrize("grid", [(4, 5, 5), (5, 6, 33), (9, 40, 130)])
+def test_boundary_conditions_small_and_ragged(grid):
+    """The fewest levels (the lid's extrapolation reads the surface), rows that end inside a
+    CTA, velocities and turbulence beyond their limits, non-finite values."""
+    p = config_params()
+    st = state(grid, 29)
+    rng = np.random.default_rng(31)
+    for n in ("u", "vn", "tke", "dis", "prod", "tke_source", "c"):
+        a = st[n]
+        a[rng.random(grid) < 0.02] = -1e9
+        a[rng.random(grid) < 0.02] = np.nan
+    st["q_v_u"] = -np.abs(st["q_v_u"])
+    o = OracleState(st, p)
+    o.boundary_conditions()
+    with GpuAtmosphere(*grid, p) as g:
+        g.upload_state(st)
+        g.boundary_conditions()
+        for n in FIELD_NAMES:
+            assert np.array_equal(g.download(n), o.f[n], equal_nan=True), n
