@@ -79,10 +79,12 @@ __global__ void __launch_bounds__(128) rhs_diag_kernel(const RhsDiagArgs a)
         a.out[2][c] = -a.coeff_u_p * sqrt((dpdr * dpdr + pt * pt + pp * pp) / 3.0);
         // latent heat of the advected condensate (:458-488): the thresholds are saturation
         // mass fractions at p_hydro = 0 (never written), i.e. 0 below the critical point
-        // and 1 above it (no saturation) for rain, always 0 for ice
+        // and 1 above it (no saturation) for rain, always 0 for ice.  Stated, not formed from
+        // the curves, whose exponentials were most of this kernel's instructions
+        // (138 -> 85 us at 41x181x361, mixed)
         const double t_u = t_ijk * a.t_0;
-        const double q_rain = thermo::saturation_mass_fraction(thermo::saturation_pressure(t_u), 0.0, 0.0);
-        const double q_ice = thermo::saturation_mass_fraction(thermo::sublimation_pressure(t_u), 0.0, 0.0);
+        const double q_rain = (t_u >= thermo::T_CRIT) ? 1.0 : 0.0;
+        const double q_ice = 0.0;
         const StarD<TY> CL = star(ycol<TY>(a, 5), c, sI, sJ);
         const StarD<TY> IC = star(ycol<TY>(a, 6), c, sI, sJ);
         const double q_lat = (c_ijk >= 0.85 * q_rain)
