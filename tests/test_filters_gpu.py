@@ -64,3 +64,19 @@ def test_filters_keep_mirror_symmetry():
         for n, anti in (("u", False), ("v", True), ("w", False), ("t", False)):
             a = g.download(n)
             assert np.array_equal(a, mirror(a, anti)), n
+
+
+@pytest.mark.parametrize("grid", [(4, 5, 5), (7, 6, 33), (8, 9, 64), (17, 24, 257), (9, 33, 258)])
+def test_damp_wiggles_edges(grid):
+    """Rows and columns that end inside the cells a thread walks, odd and even km."""
+    st = rough(grid, 53)
+    st["t"][1, 2, grid[2] - 1] = np.inf
+    o = OracleState(st, config_params())
+    o.damp_wiggles("t")
+    o.damp_wiggles("c")
+    with GpuAtmosphere(*grid, config_params()) as g:
+        g.upload_state(st)
+        g.damp_wiggles("t")
+        g.damp_wiggles("c")
+        for n in ("t", "c"):
+            assert np.array_equal(g.download(n), o.f[n], equal_nan=True), n
