@@ -548,11 +548,10 @@ athad_status athad_rk4_step(athad_ctx* ctx, const athad_step_scalars* s)
         g.coeff_MC_vel = p.L_atm / (p.u_0 * p.u_0);
         g.nontrad = p.coriolis_nontrad;
         g.flags = s->write_diagnostics & 3;
-        for (int n = 0; n < kNY; n++) {
-            const int G = rk4m_field_group(n), q = rk4m_field_place(n);
-            if (ctx->p.precision == ATHAD_PRECISION_MIXED) g.Y32[n] = (const float*)ctx->mA[G] + q;
-            else g.Y64[n] = ctx->stA[n];
-        }
+        if (ctx->p.precision == ATHAD_PRECISION_MIXED)
+            for (int G = 0; G < kMixedGroups; G++) g.Y32[G] = ctx->mA[G];
+        else
+            for (int n = 0; n < kNY; n++) g.Y64[n] = ctx->stA[n];
         launch_rhs_diagnostics(g, ctx->stream);
         ATHAD_CHECK_LAUNCH(ctx, "rhs diagnostics");
     }

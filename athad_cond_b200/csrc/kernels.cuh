@@ -49,6 +49,16 @@ struct RK4Args {
     int store_n;               // fuse storeIntermediateData3D into stage 4
 };
 
+constexpr int kMixedGroups = 3;    // groups of four values per cell (k_rk4m.cu)
+constexpr int kMixedForcing = 2;   // groups of packed forcing
+// group and place of field n (0 t, 1 u, 2 v, 3 w, 4 c, 5 cloud, 6 ice, 7 gr, 8 co2, 9 tke,
+// 10 dis): (u, v, w, p_dyn), (tke, dis, t, c), (cloud, ice, gr, co2)
+ATHAD_HD constexpr int rk4m_field_group(int n) { return (n >= 1 && n <= 3) ? 0 : (n >= 5 && n <= 8) ? 2 : 1; }
+ATHAD_HD constexpr int rk4m_field_place(int n)
+{
+    return (n >= 1 && n <= 3) ? n - 1 : (n >= 5 && n <= 8) ? n - 5 : n == 0 ? 2 : n == 4 ? 3 : n - 9;
+}
+
 // The right-hand side's diagnostic outputs (k_rhsdiag.cu): out[0..2] CoriolisForce,
 // BuoyancyForce, PressureGradientForce, [3..4] Q_Latent, Q_Sensible (flags bit 0),
 // [5..10] vbud_*, [11..16] wbud_* (flags bit 1); the last stage's input state in FP64 or FP32.
@@ -58,7 +68,7 @@ struct RhsDiagArgs {
     const double* t_ref;
     const double* p_dyn; const double* nue; const double* MC_v; const double* MC_w;
     const double* Y64[11];      // the state read: FP64 (Y32[0] null) or the FP32 stage buffers,
-    const float* Y32[11];       // four values per cell: consecutive cells four floats apart
+    const float4* Y32[3];       // four fields per cell (rk4m_field_group)
     double* out[17];
     double inv_2dr, inv_2dthe, inv_2dphi, inv_dr2, inv_dthe2, inv_dphi2;
     double coeff_Coriolis, coeff_buoy, coeff_u_p, coeff_L, coeff_S, t_0;
@@ -77,15 +87,6 @@ struct GeoF {
     float exp_rm, exp_2_rm, sinthe, costhe, inv_rm, inv_rm2, inv_rmsinthe, inv_rm2sinthe,
           inv_rm2sinthe2, costhe_inv_rm2sinthe, two_over_rm_exp, v_metric, cos4lat, pad;
 };
-constexpr int kMixedGroups = 3;    // groups of four values per cell (k_rk4m.cu)
-constexpr int kMixedForcing = 2;   // groups of packed forcing
-// group and place of field n (0 t, 1 u, 2 v, 3 w, 4 c, 5 cloud, 6 ice, 7 gr, 8 co2, 9 tke,
-// 10 dis): (u, v, w, p_dyn), (tke, dis, t, c), (cloud, ice, gr, co2)
-ATHAD_HD constexpr int rk4m_field_group(int n) { return (n >= 1 && n <= 3) ? 0 : (n >= 5 && n <= 8) ? 2 : 1; }
-ATHAD_HD constexpr int rk4m_field_place(int n)
-{
-    return (n >= 1 && n <= 3) ? n - 1 : (n >= 5 && n <= 8) ? n - 5 : n == 0 ? 2 : n == 4 ? 3 : n - 9;
-}
 struct RK4MArgs {
     Dims d;
     const GeoF* geo;
