@@ -72,6 +72,16 @@ ATHAD_HD long long idx3(const Dims& d, int i, int j, int k)
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The same, and the wait ordered before everything that depends on `index`.  Loads the
+// compiler takes for read-only (__ldg, const __restrict__) are not held back by the wait's
+// memory clobber and were moved above it (in a kernel of k_mg.cu); with their addresses
+// formed from `index` they cannot be.
+__device__ __forceinline__ void pdl_wait(int& index)
+{
+    pdl_wait();
+    asm volatile("" : "+r"(index));
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                     cudaStream_t st, Args... args)

@@ -101,8 +101,8 @@ __device__ __forceinline__ double2 zonal_two(const double* __restrict__ row, int
 __global__ void __launch_bounds__(128) wiggle_kj_kernel(Dims d, const double* __restrict__ src, double* __restrict__ dst)
 {
     pdl_trigger();
-    pdl_wait();
-    const int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    pdl_wait(k);
     const int j0 = blockIdx.y * kWalk, i = blockIdx.z;
     if (k >= d.km) return;
     const int jn = min(j0 + kWalk, d.jm);
@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(128) wiggle_kj_kernel(Dims d, const double* __
 __global__ void __launch_bounds__(128) wiggle_i_kernel(Dims d, const double* __restrict__ src, double* __restrict__ dst)
 {
     pdl_trigger();
-    pdl_wait();
-    const int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    pdl_wait(k);
     const int j = blockIdx.y, i0 = blockIdx.z * kWalk;
     if (k >= d.km) return;
     const int in = min(i0 + kWalk, d.im);

@@ -111,9 +111,9 @@ template <int COLOUR>
 __global__ void __launch_bounds__(256, ATHAD_POISSON_MIN_BLOCKS) poisson_colour_kernel(PoissonArgs a)
 {
     pdl_trigger();
-    pdl_wait();
     const Dims& d = a.d;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    int j = blockIdx.y * blockDim.y + threadIdx.y;
+    pdl_wait(j);
     const int i = blockIdx.z;
     const int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((i + j + COLOUR) & 1);
     const bool fluid = !(k < 1 || k >= d.km - 1 || j < 1 || j >= d.jm - 1 || i < 1 || i >= d.im - 1);
@@ -315,7 +315,7 @@ void launch_poisson_sweep(const PoissonArgs& a, cudaStream_t st)
 __device__ __forceinline__ long long split_at(long long row, int pitch, int k) { return row + (k & 1) * (pitch >> 1) + (k >> 1); }
 
 // p and the source of the interior cells into the split rows
-__global__ void __launch_bounds__(256) poisson_split_kernel(PoissonArgs a, double* __restrict__ ps, double* __restrict__ ss)
+__global__ void __launch_bounds__(256) poisson_split_kernel(PoissonArgs a, double* ps, double* ss)
 {
     pdl_trigger();
     pdl_wait();
@@ -451,7 +451,7 @@ poisson_split_colour_kernel(PoissonArgs a, double* ps, const double* ss)
 
 // the split rows back into p: the boundary values formed from the interior, everything
 // limited; the call's clamp count is the one source's times the sweeps
-__global__ void __launch_bounds__(256) poisson_merge_kernel(PoissonArgs a, const double* __restrict__ ps, int n_sweeps)
+__global__ void __launch_bounds__(256) poisson_merge_kernel(PoissonArgs a, const double* ps, int n_sweeps)
 {
     pdl_wait();
     const Dims& d = a.d;

@@ -52,9 +52,9 @@ __global__ void __launch_bounds__(128) level_combine_kernel(Dims d, const double
                                                             double* __restrict__ out)
 {
     pdl_trigger();
-    pdl_wait();
+    int i = blockIdx.x;
+    pdl_wait(i);
     extern __shared__ double r[];   // [jm] row sums of level i
-    const int i = blockIdx.x;
     for (int j = threadIdx.x; j < d.jm; j += blockDim.x) r[j] = rows[(long long)i * d.jm + j];
     __syncthreads();
     if (threadIdx.x != 0) return;
@@ -195,9 +195,9 @@ __global__ void __launch_bounds__(kThreads, ATHAD_RK4_MIN_BLOCKS * 128 / kThread
 rk4_stage_kernel(const RK4Args a)
 {
     pdl_trigger();
-    pdl_wait();
     const Dims& d = a.d;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(k);
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     // the even stages walk the radial planes from the top down (ATHAD_RK4_SERPENTINE, kernels.cuh)
 #if ATHAD_RK4_SERPENTINE

@@ -537,8 +537,8 @@ __global__ void __launch_bounds__(ATHAD_RK4M_BX * ATHAD_RK4M_BY,
 rk4m_stage_kernel(const RK4MArgs a)
 {
     pdl_trigger();
-    pdl_wait();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(k);
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     // the even stages walk the radial planes from the top down, so that each stage starts
     // on the planes its predecessor wrote last (1.036 -> 1.030 ms per step at 41x181x361;
