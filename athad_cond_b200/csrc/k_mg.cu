@@ -75,95 +75,130 @@ __device__ __forceinline__ T offdiag(const OpView<T>& o, const T* __restrict__ x
     return s;
 }
 
-// r = f - S e (FP32, one level)
-__global__ void __launch_bounds__(128) mg_residual_kernel(OpView<float> o, const float* __restrict__ e,
-                                                          const float* __restrict__ f, float* __restrict__ r)
+// rows of one block's partial sum: the vector kernels take 128 longitudes of kRows rows, so
+// the one block that adds the partials has a quarter of them
+constexpr int kRows = 4;
+
+// the sum of v over the block's 128 threads, in a fixed order, into partial[block]
+__device__ __forceinline__ void block_partial(double v, double* __restrict__ partial)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
-    if (k >= o.nk) return;
-    const long long c = i * o.plane + (long long)j * o.pitch + k;
-    const float d = o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)];
-    r[c] = f[c] - (d * e[c] + offdiag(o, e, i, j, k, c));
+    __shared__ double red[4];
+    for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        partial[((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
 }
 
 // q = S x in FP64, with per-block partial sums of x.q
 __global__ void __launch_bounds__(128) mg_apply64_kernel(OpView<double> o, const double* __restrict__ x,
                                                          double* __restrict__ q, double* __restrict__ partial)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
+    pdl_trigger();
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(k);
+    const int i = blockIdx.z;
     double v = 0.0;
-    if (k < o.nk) {
-        const long long c = i * o.plane + (long long)j * o.pitch + k;
-        const double d = o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)];
-        const double s = d * x[c] + offdiag(o, x, i, j, k, c);
-        q[c] = s;
-        v = x[c] * s;
-    }
-    __shared__ double red[4];
-    for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        partial[((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
+    if (k < o.nk)
+        for (int j = blockIdx.y * kRows; j < min((int)(blockIdx.y + 1) * kRows, o.nj); j++) {
+            const long long c = i * o.plane + (long long)j * o.pitch + k;
+            const double d = o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)];
+            const double s = d * x[c] + offdiag(o, x, i, j, k, c);
+            q[c] = s;
+            v += x[c] * s;
+        }
+    block_partial(v, partial);
 }
 
-// r = rhs - S x in FP64 (the true residual), partial sums of (r num1(i))^2, the squared
-// norm of the A-form residual
+// x += alpha d and r -= alpha q with alpha = s[0] / s[1], r rounded to FP32 for the
+// preconditioner and the partial sums of (r num1(i))^2, the squared norm of the A-form
+// residual.  REFINE: x only (the true residual follows)
+template <bool REFINE>
+__global__ void __launch_bounds__(128) mg_update_kernel(int nk, int nj, int pitch, long long plane,
+                                                        const double* s, const double* __restrict__ d,
+                                                        double* __restrict__ x, const double* __restrict__ q,
+                                                        double* __restrict__ r, float* __restrict__ r32,
+                                                        const double* __restrict__ inv_w, double* __restrict__ partial)
+{
+    pdl_trigger();
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(k);
+    const int i = blockIdx.z;
+    const double alpha = s[0] / s[1];
+    double v = 0.0;
+    if (k < nk)
+        for (int j = blockIdx.y * kRows; j < min((int)(blockIdx.y + 1) * kRows, nj); j++) {
+            const long long c = i * plane + (long long)j * pitch + k;
+            x[c] += alpha * d[c];
+            if (!REFINE) {
+                const double rn = r[c] - alpha * q[c];
+                r[c] = rn;
+                r32[c] = (float)rn;
+                const double a = rn * inv_w[i];
+                v += a * a;
+            }
+        }
+    if (!REFINE) block_partial(v, partial);
+}
+
+// r = rhs - S x in FP64 (the true residual), also rounded to FP32, partial sums of
+// (r num1(i))^2
 __global__ void __launch_bounds__(128) mg_true_residual_kernel(OpView<double> o, const double* __restrict__ x,
                                                                const double* __restrict__ rhs, double* __restrict__ r,
+                                                               float* __restrict__ r32,
                                                                const double* __restrict__ inv_w,
                                                                double* __restrict__ partial)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
+    pdl_trigger();
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(k);
+    const int i = blockIdx.z;
     double v = 0.0;
-    if (k < o.nk) {
-        const long long c = i * o.plane + (long long)j * o.pitch + k;
-        const double d = o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)];
-        const double s = rhs[c] - (d * x[c] + offdiag(o, x, i, j, k, c));
-        r[c] = s;
-        const double a = s * inv_w[i];
-        v = a * a;
-    }
-    __shared__ double red[4];
-    for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        partial[((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
+    if (k < o.nk)
+        for (int j = blockIdx.y * kRows; j < min((int)(blockIdx.y + 1) * kRows, o.nj); j++) {
+            const long long c = i * o.plane + (long long)j * o.pitch + k;
+            const double d = o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)];
+            const double s = rhs[c] - (d * x[c] + offdiag(o, x, i, j, k, c));
+            r[c] = s;
+            r32[c] = (float)s;
+            const double a = s * inv_w[i];
+            v += a * a;
+        }
+    block_partial(v, partial);
 }
 
-// per-block partial sums of a.b; of (a num1(i))^2 when b is null (the squared norm of the
-// corresponding A-form vector); of a when both b and inv_w are null
+// per-block partial sums of a.b (b the FP32 preconditioned residual); of (a num1(i))^2 when b
+// is null (the squared norm of the corresponding A-form vector); of a when both are null
 __global__ void __launch_bounds__(128) mg_dot_kernel(int nk, int nj, int pitch, long long plane,
-                                                     const double* __restrict__ a, const double* __restrict__ b,
+                                                     const double* __restrict__ a, const float* __restrict__ b,
                                                      const double* __restrict__ inv_w, double* __restrict__ partial)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
+    pdl_trigger();
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(k);
+    const int i = blockIdx.z;
     double v = 0.0;
-    if (k < nk) {
-        const long long c = i * plane + (long long)j * pitch + k;
-        if (b) v = a[c] * b[c];
-        else if (inv_w) { const double s = a[c] * inv_w[i]; v = s * s; }
-        else v = a[c];
-    }
-    __shared__ double red[4];
-    for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        partial[((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
+    if (k < nk)
+        for (int j = blockIdx.y * kRows; j < min((int)(blockIdx.y + 1) * kRows, nj); j++) {
+            const long long c = i * plane + (long long)j * pitch + k;
+            if (b) v += a[c] * (double)b[c];
+            else if (inv_w) { const double t = a[c] * inv_w[i]; v += t * t; }
+            else v += a[c];
+        }
+    block_partial(v, partial);
 }
 
-// fixed-order sum of n partials into out[slot] (one block of 1024 threads)
+// fixed-order sum of n partials into out[slot] (one block of 1024 threads); next_rz: also the
+// iteration's start, out[0] = out[2] (r.z of the iteration before)
 __global__ void __launch_bounds__(1024) mg_sum_kernel(const double* __restrict__ partial, long long n,
-                                                      double* __restrict__ out, int slot)
+                                                      double* __restrict__ out, int slot, int next_rz)
 {
+    pdl_trigger();
+    int first = threadIdx.x;
+    pdl_wait(first);
     double v = 0.0;
-    for (long long q = threadIdx.x; q < n; q += blockDim.x) v += partial[q];
+#pragma unroll 8
+    for (long long q = first; q < n; q += 1024) v += partial[q];
     __shared__ double red[32];
     for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
@@ -171,30 +206,26 @@ __global__ void __launch_bounds__(1024) mg_sum_kernel(const double* __restrict__
     if (threadIdx.x < 32) {
         double w = red[threadIdx.x];
         for (int off = 16; off >= 1; off >>= 1) w += __shfl_xor_sync(0xffffffffu, w, off);
-        if (threadIdx.x == 0) out[slot] = w;
+        if (threadIdx.x == 0) {
+            out[slot] = w;
+            if (next_rz) out[0] = out[2];
+        }
     }
 }
 
-// y += a x  (a read from device memory: a = s[num] / s[den] * sign)
-__global__ void mg_axpy_kernel(long long n, const double* __restrict__ s, int num, int den, double sign,
-                               const double* __restrict__ x, double* __restrict__ y)
+// d = z + (s[num] / s[den]) d, z the FP32 preconditioned residual
+__global__ void mg_xpby_kernel(long long n, const double* s, int num, int den,
+                               const float* __restrict__ z, double* __restrict__ d)
 {
-    const double a = sign * s[num] / s[den];
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        y[q] += a * x[q];
-}
-
-// d = z + (s[num] / s[den]) d
-__global__ void mg_xpby_kernel(long long n, const double* __restrict__ s, int num, int den,
-                               const double* __restrict__ z, double* __restrict__ d)
-{
+    pdl_trigger();
+    int first = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(first);
     const double b = s[num] / s[den];
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        d[q] = z[q] + b * d[q];
+    for (long long q = first; q < n; q += (long long)gridDim.x * blockDim.x)
+        d[q] = (double)z[q] + b * d[q];
 }
 
-__global__ void mg_copy_scalar_kernel(double* s, int dst, int src) { s[dst] = s[src]; }
-
+// FP64 residual to FP32 (f32 given) and FP32 preconditioned residual to FP64, at the start
 __global__ void mg_to_f32_kernel(long long n, const double* __restrict__ a, float* __restrict__ b)
 {
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
@@ -221,15 +252,8 @@ __global__ void __launch_bounds__(128) mg_sub_mean_kernel(int nk, int pitch, lon
 // column solved exactly with the horizontal neighbours fixed.  The seam neighbour of the
 // columns k = 0 and k = nk-1 is read from `seam` (the two seam planes before the
 // half-sweep), because with an odd nk both ends have the same colour.
-//
-// A CTA takes 32 columns of one row j with four warps: warp q forms the right-hand sides
-// (the horizontal neighbours fixed) of levels q, q+4, ... of all 32 columns and stages them
-// in shared memory with the elimination factors, so the independent loads of a column run
-// four ways in parallel; then warp 0 runs the two sequential recurrences of its 32 columns
-// out of shared memory.  Element (i, column t) of an array is at [i * 32 + t].
-__device__ __forceinline__ float smooth_rhs(const OpView<float>& o, const float* __restrict__ f,
-                                            const float* __restrict__ e, const float* __restrict__ seam,
-                                            int i, int j, int k, int kc, long long c)
+__device__ __forceinline__ float smooth_rhs(const OpView<float>& o, const float* __restrict__ f, const float* e,
+                                            const float* seam, int i, int j, int k, int kc, long long c)
 {
     const int ij = i * o.nj + j;
     float s = f[c];
@@ -243,49 +267,101 @@ __device__ __forceinline__ float smooth_rhs(const OpView<float>& o, const float*
     return s;
 }
 
-__global__ void __launch_bounds__(128) mg_smooth_split_kernel(OpView<float> o, const float* __restrict__ tm,
-                                                              const float* __restrict__ tc, const float* __restrict__ f,
-                                                              float* __restrict__ e, const float* __restrict__ seam,
-                                                              int colour)
+// A CTA takes 32 columns of one row j.  Its kSmoothWarps warps form the right-hand sides (the
+// horizontal neighbours fixed), level by level, and stage them in shared memory; then warp 0
+// runs the two recurrences of its 32 columns from there, kSmoothChunk levels' operands loaded
+// ahead of the chain (a multiply-add and a product per level).  The elimination factors
+// depend on the row and the column class only, so they are staged once per CTA, before the
+// kernel before this one has finished.  The half-sweep also leaves the seam planes for the
+// next one in seam_out: the columns it relaxed, or what seam_in held.
+// FIRST: the first half-sweep from zero, which reads no e (the right-hand side is f) and
+// takes the seam planes as zero, so that nothing has to clear e.
+// Four warps, the factors per column in shared memory (30 KB per CTA instead of 10), the
+// operands of one level at a time, a launch before each half-sweep that copies the seam
+// planes, stored residuals and separate vector kernels: 71.3 ms per solve of 61x361x721, now
+// 48.1; 38x31x45 5.9 -> 3.1 ms, 33x223x149 16.8 -> 9.2 (the same iteration counts).
+constexpr int kSmoothWarps = 8, kSmoothChunk = 8;
+template <bool FIRST>
+__global__ void __launch_bounds__(32 * kSmoothWarps) mg_smooth_split_kernel(
+    OpView<float> o, const float* __restrict__ tm, const float* __restrict__ tc, const float* __restrict__ f,
+    float* e, const float* seam_in, float* seam_out, int colour)
 {
-    extern __shared__ float sm[];   // rhs, forward factor m_i, coupling c_{i-1}, backward factor: [4][ni][32]
+    extern __shared__ float sm[];   // rhs [ni][32]; factors m, coupling below, back factor: [ni][3] each
+    pdl_trigger();
     const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
     const int j = blockIdx.y;
-    const int k = 2 * (blockIdx.x * 32 + lane) + ((colour + j) & 1);
+    const int par = (colour + j) & 1;
+    int k = 2 * (blockIdx.x * 32 + lane) + par;
     const bool valid = k < o.nk;
-    const int ni = o.ni;
+    const int ni = o.ni, planes = o.ni * o.nj;
     float* rhs = sm;
     float* fm = sm + ni * 32;
-    float* fc = sm + 2 * ni * 32;
-    float* bc = sm + 3 * ni * 32;
+    float* fc = fm + ni * 3;
+    float* bc = fc + ni * 3;
+    for (int t = threadIdx.x; t < ni * 3; t += 32 * kSmoothWarps) {
+        const int i = t / 3, w = t - 3 * i, at = (i * o.nj + j) * 3 + w;
+        fm[t] = tm[at];
+        fc[t] = (i > 0) ? o.ci[at - o.nj * 3] : 0.0f;
+        bc[t] = tc[at];
+    }
+    pdl_wait(k);
     const int kc = valid ? kclass(k, o.nk) : 1;
     const long long c0 = (long long)j * o.pitch + k;
     if (valid) {
-#pragma unroll 2
-        for (int i = q; i < ni; i += 4) {
-            const int ij = i * o.nj + j;
-            rhs[i * 32 + lane] = smooth_rhs(o, f, e, seam, i, j, k, kc, i * o.plane + c0);
-            fm[i * 32 + lane] = tm[ij * 3 + kc];
-            fc[i * 32 + lane] = (i > 0) ? o.ci[(ij - o.nj) * 3 + kc] : 0.0f;
-            bc[i * 32 + lane] = tc[ij * 3 + kc];
+#pragma unroll 4
+        for (int i = q; i < ni; i += kSmoothWarps) {
+            const long long c = i * o.plane + c0;
+            rhs[i * 32 + lane] = FIRST ? f[c] : smooth_rhs(o, f, e, seam_in, i, j, k, kc, c);
         }
     }
     __syncthreads();
+    if (q == 1 && blockIdx.x == 0) {
+        // the seam planes whose columns the other colour has
+        const bool first_kept = par != 0, last_kept = ((o.nk - 1) & 1) != par;
+        for (int i = lane; i < ni; i += 32) {
+            const int ij = i * o.nj + j;
+            if (first_kept) seam_out[ij] = FIRST ? 0.0f : seam_in[ij];
+            if (last_kept) seam_out[planes + ij] = FIRST ? 0.0f : seam_in[planes + ij];
+        }
+    }
     if (q != 0 || !valid) return;
+    float* mine = rhs + lane;
     // forward elimination: y_i = (rhs_i - c_{i-1} y_{i-1}) m_i
     float y = 0.0f;
-    for (int i = 0; i < ni; i++) {
-        float s = rhs[i * 32 + lane];
-        if (i > 0) s -= fc[i * 32 + lane] * y;
-        y = s * fm[i * 32 + lane];
-        rhs[i * 32 + lane] = y;
+    for (int i0 = 0; i0 < ni; i0 += kSmoothChunk) {
+        float r[kSmoothChunk], m[kSmoothChunk], a[kSmoothChunk];
+#pragma unroll
+        for (int u = 0; u < kSmoothChunk; u++) {
+            const int i = min(i0 + u, ni - 1);
+            r[u] = mine[i * 32]; m[u] = fm[i * 3 + kc]; a[u] = fc[i * 3 + kc];
+        }
+#pragma unroll
+        for (int u = 0; u < kSmoothChunk; u++)
+            if (i0 + u < ni) {
+                y = (r[u] - a[u] * y) * m[u];
+                r[u] = y;
+            }
+#pragma unroll
+        for (int u = 0; u < kSmoothChunk; u++)
+            if (i0 + u < ni) mine[(i0 + u) * 32] = r[u];
     }
-    // back substitution: x_i = y_i - c'_i x_{i+1}
-    float x = y;
-    e[(ni - 1) * o.plane + c0] = x;
-    for (int i = ni - 2; i >= 0; i--) {
-        x = rhs[i * 32 + lane] - bc[i * 32 + lane] * x;
-        e[i * o.plane + c0] = x;
+    // back substitution: x_i = y_i - c'_i x_{i+1}; the seam planes' columns for the next half-sweep
+    float* seam = (k == 0) ? seam_out + j : (k == o.nk - 1) ? seam_out + planes + j : nullptr;
+    float x = 0.0f;
+    for (int i0 = ni - 1; i0 >= 0; i0 -= kSmoothChunk) {
+        float r[kSmoothChunk], b[kSmoothChunk];
+#pragma unroll
+        for (int u = 0; u < kSmoothChunk; u++) {
+            const int i = max(i0 - u, 0);
+            r[u] = mine[i * 32]; b[u] = (i == ni - 1) ? 0.0f : bc[i * 3 + kc];
+        }
+#pragma unroll
+        for (int u = 0; u < kSmoothChunk; u++)
+            if (i0 - u >= 0) {
+                x = r[u] - b[u] * x;
+                e[(i0 - u) * o.plane + c0] = x;
+                if (seam) seam[(i0 - u) * o.nj] = x;
+            }
     }
 }
 
@@ -332,21 +408,27 @@ __global__ void mg_seam_copy_kernel(int ni, int nj, int nk, int pitch, long long
     seam[(long long)ni * nj + q] = e[c + nk - 1];
 }
 
-// coarse f = sum of the fine residuals of the 2 x 2 (j, k) aggregate
-__global__ void __launch_bounds__(128) mg_restrict_kernel(int nk_f, int nj_f, int pitch_f, long long plane_f,
-                                                          const float* __restrict__ r, int nk_c, int pitch_c,
+// coarse f = sum of the fine residuals f - S e of the 2 x 2 (j, k) aggregate, which are not
+// stored
+__global__ void __launch_bounds__(128) mg_restrict_kernel(OpView<float> o, const float* __restrict__ e,
+                                                          const float* __restrict__ f, int nk_c, int pitch_c,
                                                           long long plane_c, float* __restrict__ fc)
 {
-    const int K = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_trigger();
+    int K = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(K);
     const int J = blockIdx.y, i = blockIdx.z;
     if (K >= nk_c) return;
     const int j0 = 2 * J, k0 = 2 * K;
-    const long long b = i * plane_f;
-    float s = r[b + (long long)j0 * pitch_f + k0];
-    if (k0 + 1 < nk_f) s += r[b + (long long)j0 * pitch_f + k0 + 1];
-    if (j0 + 1 < nj_f) {
-        s += r[b + (long long)(j0 + 1) * pitch_f + k0];
-        if (k0 + 1 < nk_f) s += r[b + (long long)(j0 + 1) * pitch_f + k0 + 1];
+    auto residual = [&](int j, int k) {
+        const long long c = i * o.plane + (long long)j * o.pitch + k;
+        return f[c] - (o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)] * e[c] + offdiag(o, e, i, j, k, c));
+    };
+    float s = residual(j0, k0);
+    if (k0 + 1 < o.nk) s += residual(j0, k0 + 1);
+    if (j0 + 1 < o.nj) {
+        s += residual(j0 + 1, k0);
+        if (k0 + 1 < o.nk) s += residual(j0 + 1, k0 + 1);
     }
     fc[i * plane_c + (long long)J * pitch_c + K] = s;
 }
@@ -354,12 +436,21 @@ __global__ void __launch_bounds__(128) mg_restrict_kernel(int nk_f, int nj_f, in
 // fine e += scale * coarse e of the aggregate.  A piecewise-constant prolongation
 // under-corrects smooth errors; a constant scale keeps the V-cycle symmetric.
 __global__ void __launch_bounds__(128) mg_prolong_kernel(int nk_f, int pitch_f, long long plane_f, float* __restrict__ e,
-                                                         int pitch_c, long long plane_c, const float* __restrict__ ec)
+                                                         int pitch_c, long long plane_c, const float* __restrict__ ec,
+                                                         float* __restrict__ seam)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_trigger();
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(k);
     const int j = blockIdx.y, i = blockIdx.z;
     if (k >= nk_f) return;
-    e[i * plane_f + (long long)j * pitch_f + k] += ATHAD_MG_CSCALE * ec[i * plane_c + (long long)(j >> 1) * pitch_c + (k >> 1)];
+    const long long c = i * plane_f + (long long)j * pitch_f + k;
+    const float v = e[c] + ATHAD_MG_CSCALE * ec[i * plane_c + (long long)(j >> 1) * pitch_c + (k >> 1)];
+    e[c] = v;
+    // the seam planes of the post-smoother's first half-sweep
+    const int ij = i * gridDim.y + j;
+    if (k == 0) seam[ij] = v;
+    if (k == nk_f - 1) seam[gridDim.z * gridDim.y + ij] = v;
 }
 
 // right-hand side of S: rhs_c = -src_c / num1(i) at every interior cell
@@ -403,21 +494,21 @@ struct MGSolver {
     OpView<double> op64{};
     double* coef64 = nullptr;
     double* inv_w = nullptr;                       // num1(i) per interior level
-    double *x = nullptr, *r = nullptr, *z = nullptr, *d = nullptr, *q = nullptr, *rhs = nullptr;
+    double *x = nullptr, *r = nullptr, *d = nullptr, *q = nullptr, *rhs = nullptr;
     double* partial = nullptr;
     double* scal = nullptr;                        // device scalars
     float* seam = nullptr;
     long long nblocks = 0;
     char* mem = nullptr;
     size_t bytes = 0;
-    cudaGraphExec_t iter_graph[2] = {nullptr, nullptr};   // one CG iteration (plain, refined)
+    cudaGraphExec_t iter_graph[3] = {nullptr, nullptr, nullptr};   // a CG step (plain, refined), a direction
     double* h = nullptr;                                  // pinned copy of the device scalars
 };
 
 void mg_free(MGSolver* s)
 {
     if (!s) return;
-    for (int g = 0; g < 2; g++)
+    for (int g = 0; g < 3; g++)
         if (s->iter_graph[g]) cudaGraphExecDestroy(s->iter_graph[g]);
     if (s->h) cudaFreeHost(s->h);
     cudaFree(s->mem);
@@ -570,12 +661,12 @@ MGSolver* mg_build(athad_ctx* ctx, std::string& err)
     const MGLevel& L0 = s->L[0];
     const size_t off_c64 = add((size_t)ni * nj * (3 * 3 + 2) * sizeof(double));
     const size_t off_w = add(ni * sizeof(double));
-    size_t off_v[6];
-    for (int v = 0; v < 6; v++) off_v[v] = add(L0.n * sizeof(double));
-    s->nblocks = (long long)((L0.nk + 127) / 128) * L0.nj * L0.ni;
+    size_t off_v[5];
+    for (int v = 0; v < 5; v++) off_v[v] = add(L0.n * sizeof(double));
+    s->nblocks = (long long)((L0.nk + 127) / 128) * ((L0.nj + kRows - 1) / kRows) * L0.ni;
     const size_t off_p = add(s->nblocks * sizeof(double));
     const size_t off_s = add(64 * sizeof(double));
-    const size_t off_seam = add((size_t)2 * ni * nj * sizeof(float));
+    const size_t off_seam = add((size_t)4 * ni * nj * sizeof(float));
     if (cudaMalloc((void**)&s->mem, bytes) != cudaSuccess) {
         cudaGetLastError(); delete s; err = "pressure_solve: out of device memory"; return nullptr;
     }
@@ -611,8 +702,8 @@ MGSolver* mg_build(athad_ctx* ctx, std::string& err)
                    s->coef64 + 3 * m3, s->coef64 + 3 * m3 + m1};
         s->inv_w = (double*)(s->mem + off_w);
         if (ok) ok = cudaMemcpy(s->inv_w, inv_w.data(), ni * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess;
-        double** vec[6] = {&s->x, &s->r, &s->z, &s->d, &s->q, &s->rhs};
-        for (int v = 0; v < 6; v++) *vec[v] = (double*)(s->mem + off_v[v]);
+        double** vec[5] = {&s->x, &s->r, &s->d, &s->q, &s->rhs};
+        for (int v = 0; v < 5; v++) *vec[v] = (double*)(s->mem + off_v[v]);
         s->partial = (double*)(s->mem + off_p);
         s->scal = (double*)(s->mem + off_s);
         s->seam = (float*)(s->mem + off_seam);
@@ -627,84 +718,109 @@ MGSolver* mg_build(athad_ctx* ctx, std::string& err)
 namespace {
 
 inline dim3 cells_grid(int nk, int nj, int ni) { return dim3((nk + 127) / 128, nj, ni); }
+inline dim3 rows_grid(const MGLevel& L) { return dim3((L.nk + 127) / 128, (L.nj + kRows - 1) / kRows, L.ni); }
 
-void smooth(const MGLevel& L, float* seam, int colour, cudaStream_t st)
+// the staged right-hand sides and factors of a smoother CTA; columns of up to 299 levels
+inline size_t smooth_smem(const MGLevel& L) { return (size_t)(32 + 9) * L.ni * sizeof(float); }
+inline bool smooth_fits(const MGLevel& L) { return smooth_smem(L) <= 48 * 1024; }
+
+// one half-sweep of level L; `half` counts the half-sweeps of a sequence (the seam planes
+// alternate between two buffers), from_zero: L.e is zero and need not be stored so
+void smooth(MGSolver* s, const MGLevel& L, int colour, int half, bool from_zero, cudaStream_t st)
 {
-    mg_seam_copy_kernel<<<(L.ni * L.nj + 255) / 256, 256, 0, st>>>(L.ni, L.nj, L.nk, L.pitch, L.plane, L.e, seam);
-    const int half = (L.nk + 1) / 2;
-    const size_t smem = (size_t)4 * 32 * L.ni * sizeof(float);
-    if (smem <= 48 * 1024)   // columns of up to 96 levels in shared memory
-        mg_smooth_split_kernel<<<dim3((half + 31) / 32, L.nj), 128, smem, st>>>(L.op, L.tm, L.tc, L.f, L.e, seam,
-                                                                              colour);
-    else
-        mg_smooth_kernel<<<dim3((half + 127) / 128, L.nj), 128, 0, st>>>(L.op, L.tm, L.tc, L.f, L.e, seam,
-                                                                       L.r, colour);
+    float* seam[2] = {s->seam, s->seam + 2 * (size_t)s->L[0].ni * s->L[0].nj};
+    float* in = seam[half & 1];
+    float* out = seam[(half + 1) & 1];
+    const int nh = (L.nk + 1) / 2;
+    if (smooth_fits(L)) {
+        const dim3 grid((nh + 31) / 32, L.nj), block(32 * kSmoothWarps);
+        if (from_zero)
+            launch_dependent(mg_smooth_split_kernel<true>, grid, block, smooth_smem(L), st, L.op, (const float*)L.tm,
+                             (const float*)L.tc, (const float*)L.f, L.e, (const float*)in, out, colour);
+        else
+            launch_dependent(mg_smooth_split_kernel<false>, grid, block, smooth_smem(L), st, L.op, (const float*)L.tm,
+                             (const float*)L.tc, (const float*)L.f, L.e, (const float*)in, out, colour);
+        return;
+    }
+    if (from_zero) cudaMemsetAsync(L.e, 0, L.n * sizeof(float), st);
+    mg_seam_copy_kernel<<<(L.ni * L.nj + 255) / 256, 256, 0, st>>>(L.ni, L.nj, L.nk, L.pitch, L.plane, L.e, in);
+    mg_smooth_kernel<<<dim3((nh + 127) / 128, L.nj), 128, 0, st>>>(L.op, L.tm, L.tc, L.f, L.e, in, L.r, colour);
 }
 
 // one V-cycle on level l: L[l].e ~= S_l^-1 L[l].f, starting from zero
 void vcycle(MGSolver* s, int l, cudaStream_t st)
 {
     MGLevel& L = s->L[l];
-    cudaMemsetAsync(L.e, 0, L.n * sizeof(float), st);
+    int half = 0;
     if (l == s->nlev - 1) {
-        for (int it = 0; it < ATHAD_MG_COARSE_SWEEPS; it++) { smooth(L, s->seam, 0, st); smooth(L, s->seam, 1, st); }
-        for (int it = 0; it < ATHAD_MG_COARSE_SWEEPS; it++) { smooth(L, s->seam, 1, st); smooth(L, s->seam, 0, st); }
+        for (int it = 0; it < 2 * ATHAD_MG_COARSE_SWEEPS; it++, half++) smooth(s, L, it & 1, half, it == 0, st);
+        for (int it = 0; it < 2 * ATHAD_MG_COARSE_SWEEPS; it++, half++) smooth(s, L, 1 - (it & 1), half, false, st);
         return;
     }
-    for (int it = 0; it < ATHAD_MG_NU; it++) { smooth(L, s->seam, 0, st); smooth(L, s->seam, 1, st); }
-    mg_residual_kernel<<<cells_grid(L.nk, L.nj, L.ni), 128, 0, st>>>(L.op, L.e, L.f, L.r);
+    for (int it = 0; it < 2 * ATHAD_MG_NU; it++, half++) smooth(s, L, it & 1, half, it == 0, st);
     MGLevel& C = s->L[l + 1];
-    mg_restrict_kernel<<<cells_grid(C.nk, C.nj, C.ni), 128, 0, st>>>(L.nk, L.nj, L.pitch, L.plane, L.r, C.nk,
-                                                                       C.pitch, C.plane, C.f);
+    launch_dependent(mg_restrict_kernel, cells_grid(C.nk, C.nj, C.ni), dim3(128), 0, st, L.op, (const float*)L.e,
+                     (const float*)L.f, C.nk, C.pitch, C.plane, C.f);
     vcycle(s, l + 1, st);
-    mg_prolong_kernel<<<cells_grid(L.nk, L.nj, L.ni), 128, 0, st>>>(L.nk, L.pitch, L.plane, L.e, C.pitch, C.plane, C.e);
-    for (int it = 0; it < ATHAD_MG_NU; it++) { smooth(L, s->seam, 1, st); smooth(L, s->seam, 0, st); }
+    launch_dependent(mg_prolong_kernel, cells_grid(L.nk, L.nj, L.ni), dim3(128), 0, st, L.nk, L.pitch, L.plane, L.e,
+                     C.pitch, C.plane, (const float*)C.e, s->seam);
+    for (int it = 0; it < 2 * ATHAD_MG_NU; it++) smooth(s, L, 1 - (it & 1), it, false, st);
 }
 
-// z = M^-1 r (FP32 V-cycle)
-void precondition(MGSolver* s, cudaStream_t st)
+void sum(MGSolver* s, int slot, bool next_rz, cudaStream_t st)
 {
-    const MGLevel& L0 = s->L[0];
-    mg_to_f32_kernel<<<148 * 8, 256, 0, st>>>(L0.n, s->r, s->L[0].f);
-    vcycle(s, 0, st);
-    mg_to_f64_kernel<<<148 * 8, 256, 0, st>>>(L0.n, s->L[0].e, s->z);
+    launch_dependent(mg_sum_kernel, dim3(1), dim3(1024), 0, st, (const double*)s->partial, s->nblocks, s->scal, slot,
+                     next_rz ? 1 : 0);
 }
 
-void dot(MGSolver* s, const double* a, const double* b, int slot, cudaStream_t st)
+void dot(MGSolver* s, const double* a, const float* b, const double* inv_w, int slot, cudaStream_t st)
 {
     const MGLevel& L0 = s->L[0];
-    mg_dot_kernel<<<cells_grid(L0.nk, L0.nj, L0.ni), 128, 0, st>>>(L0.nk, L0.nj, L0.pitch, L0.plane, a, b, s->inv_w,
-                                                                   s->partial);
-    mg_sum_kernel<<<1, 1024, 0, st>>>(s->partial, s->nblocks, s->scal, slot);
+    launch_dependent(mg_dot_kernel, rows_grid(L0), dim3(128), 0, st, L0.nk, L0.nj, L0.pitch, L0.plane, a, b, inv_w,
+                     s->partial);
+    sum(s, slot, false, st);
 }
 
 // true residual r = rhs - S x with its A-form norm into scal[3]
 void true_residual(MGSolver* s, cudaStream_t st)
 {
     const MGLevel& L0 = s->L[0];
-    mg_true_residual_kernel<<<cells_grid(L0.nk, L0.nj, L0.ni), 128, 0, st>>>(s->op64, s->x, s->rhs, s->r, s->inv_w,
-                                                                             s->partial);
-    mg_sum_kernel<<<1, 1024, 0, st>>>(s->partial, s->nblocks, s->scal, 3);
+    launch_dependent(mg_true_residual_kernel, rows_grid(L0), dim3(128), 0, st, s->op64, (const double*)s->x,
+                     (const double*)s->rhs, s->r, L0.f, (const double*)s->inv_w, s->partial);
+    sum(s, 3, false, st);
 }
 
-// One conjugate-gradient iteration, all scalars on the device: q = S d, alpha = rz / d.q,
-// x += alpha d, r -= alpha q, the residual norm (recursive, or the true residual when
-// `refine`) copied to the pinned host scalars, z = M^-1 r, beta = r.z / rz, d = z + beta d.
-void enqueue_cg_iteration(MGSolver* s, bool refine, cudaStream_t st)
+// The first half of a conjugate-gradient iteration, all scalars on the device: q = S d,
+// alpha = rz / d.q, x += alpha d, r -= alpha q, the residual norm (recursive, or the true
+// residual when `refine`) copied to the pinned host scalars.
+void enqueue_step(MGSolver* s, bool refine, cudaStream_t st)
 {
     const MGLevel& L0 = s->L[0];
-    const long long n = L0.n;
-    mg_apply64_kernel<<<cells_grid(L0.nk, L0.nj, L0.ni), 128, 0, st>>>(s->op64, s->d, s->q, s->partial);
-    mg_sum_kernel<<<1, 1024, 0, st>>>(s->partial, s->nblocks, s->scal, 1);
-    mg_axpy_kernel<<<148 * 8, 256, 0, st>>>(n, s->scal, 0, 1, 1.0, s->d, s->x);
-    mg_axpy_kernel<<<148 * 8, 256, 0, st>>>(n, s->scal, 0, 1, -1.0, s->q, s->r);
-    if (refine) true_residual(s, st);
-    else dot(s, s->r, nullptr, 3, st);
+    launch_dependent(mg_apply64_kernel, rows_grid(L0), dim3(128), 0, st, s->op64, (const double*)s->d, s->q, s->partial);
+    sum(s, 1, true, st);
+    if (refine) {
+        launch_dependent(mg_update_kernel<true>, rows_grid(L0), dim3(128), 0, st, L0.nk, L0.nj, L0.pitch, L0.plane,
+                         (const double*)s->scal, (const double*)s->d, s->x, (const double*)s->q, s->r, L0.f,
+                         (const double*)s->inv_w, s->partial);
+        true_residual(s, st);
+    } else {
+        launch_dependent(mg_update_kernel<false>, rows_grid(L0), dim3(128), 0, st, L0.nk, L0.nj, L0.pitch, L0.plane,
+                         (const double*)s->scal, (const double*)s->d, s->x, (const double*)s->q, s->r, L0.f,
+                         (const double*)s->inv_w, s->partial);
+        sum(s, 3, false, st);
+    }
     cudaMemcpyAsync(s->h, s->scal, 5 * sizeof(double), cudaMemcpyDeviceToHost, st);
-    precondition(s, st);
-    dot(s, s->r, s->z, 2, st);
-    mg_xpby_kernel<<<148 * 8, 256, 0, st>>>(n, s->scal, 2, 0, s->z, s->d);
-    mg_copy_scalar_kernel<<<1, 1, 0, st>>>(s->scal, 0, 2);
+}
+
+// The second half: z = M^-1 r (FP32 V-cycle on r rounded to FP32, which the first half left in
+// the finest level's right-hand side), beta = r.z / rz, d = z + beta d.
+void enqueue_direction(MGSolver* s, cudaStream_t st)
+{
+    const MGLevel& L0 = s->L[0];
+    vcycle(s, 0, st);
+    dot(s, s->r, L0.e, nullptr, 2, st);
+    launch_dependent(mg_xpby_kernel, dim3(148 * 8), dim3(256), 0, st, L0.n, (const double*)s->scal, 2, 0,
+                     (const float*)L0.e, s->d);
 }
 
 }  // namespace
@@ -749,15 +865,15 @@ extern "C" athad_status athad_pressure_solve(athad_ctx* ctx, double rel_tol, int
     const long long n = L0.n;
     mg_rhs_kernel<<<g0, 128, 0, st>>>(d, ctx->src, L0.nk, L0.pitch, L0.plane, s->inv_w, s->rhs);
     // project onto the range of S: remove the mean
-    mg_dot_kernel<<<g0, 128, 0, st>>>(L0.nk, L0.nj, L0.pitch, L0.plane, s->rhs, nullptr, nullptr, s->partial);
-    mg_sum_kernel<<<1, 1024, 0, st>>>(s->partial, s->nblocks, s->scal, 5);
+    dot(s, s->rhs, nullptr, nullptr, 5, st);
     mg_sub_mean_kernel<<<g0, 128, 0, st>>>(L0.nk, L0.pitch, L0.plane, s->rhs, s->scal, 5, count);
-    dot(s, s->rhs, nullptr, 4, st);                                   // ||b||^2 (A form)
+    dot(s, s->rhs, nullptr, s->inv_w, 4, st);                         // ||b||^2 (A form)
     cudaMemsetAsync(s->x, 0, n * sizeof(double), st);
     cudaMemcpyAsync(s->r, s->rhs, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    precondition(s, st);
-    cudaMemcpyAsync(s->d, s->z, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    dot(s, s->r, s->z, 0, st);                                        // rz
+    mg_to_f32_kernel<<<148 * 8, 256, 0, st>>>(n, s->r, L0.f);
+    vcycle(s, 0, st);
+    mg_to_f64_kernel<<<148 * 8, 256, 0, st>>>(n, L0.e, s->d);          // the first direction is z
+    dot(s, s->r, L0.e, nullptr, 2, st);                               // rz (the first step moves it to slot 0)
     ATHAD_CHECK_LAUNCH(ctx, "pressure_solve setup");
     double h[5] = {0, 0, 0, 0, 0};
     athad_status stt = cuda_check(ctx, cudaMemcpyAsync(h, s->scal, sizeof h, cudaMemcpyDeviceToHost, st), "pressure_solve norm");
@@ -767,12 +883,13 @@ extern "C" athad_status athad_pressure_solve(athad_ctx* ctx, double rel_tol, int
     athad_solve_report rep;
     std::memset(&rep, 0, sizeof rep);
     rep.precond_levels = s->nlev;
-    if (!s->iter_graph[0] && h[4] > 0.0) {   // capture the two iteration variants once
-        for (int g = 0; g < 2 && stt == ATHAD_OK; g++) {
+    if (!s->iter_graph[0] && h[4] > 0.0) {   // capture the two steps and the direction once
+        for (int g = 0; g < 3 && stt == ATHAD_OK; g++) {
             cudaGraph_t graph = nullptr;
             stt = cuda_check(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture");
             if (stt != ATHAD_OK) break;
-            enqueue_cg_iteration(s, g == 1, st);
+            if (g < 2) enqueue_step(s, g == 1, st);
+            else enqueue_direction(s, st);
             stt = cuda_check(ctx, cudaStreamEndCapture(st, &graph), "end capture");
             if (stt == ATHAD_OK) stt = cuda_check(ctx, cudaGraphInstantiate(&s->iter_graph[g], graph, 0), "instantiate");
             if (graph) cudaGraphDestroy(graph);
@@ -782,7 +899,9 @@ extern "C" athad_status athad_pressure_solve(athad_ctx* ctx, double rel_tol, int
     int it = 0;
     for (it = 1; it <= max_iter && h[4] > 0.0 && stt == ATHAD_OK; it++) {
         const bool refine = (it % 8 == 0);
-        stt = cuda_check(ctx, cudaGraphLaunch(s->iter_graph[refine ? 1 : 0], st), "pressure_solve iteration");
+        // the direction is formed only when another step follows
+        if (it > 1) stt = cuda_check(ctx, cudaGraphLaunch(s->iter_graph[2], st), "pressure_solve direction");
+        if (stt == ATHAD_OK) stt = cuda_check(ctx, cudaGraphLaunch(s->iter_graph[refine ? 1 : 0], st), "pressure_solve step");
         if (stt == ATHAD_OK) stt = cuda_check(ctx, cudaStreamSynchronize(st), "pressure_solve");
         if (stt != ATHAD_OK) break;
         res = std::sqrt(s->h[3] / h[4]);
@@ -801,8 +920,7 @@ extern "C" athad_status athad_pressure_solve(athad_ctx* ctx, double rel_tol, int
     }
     if (stt != ATHAD_OK) { cudaEventDestroy(t0); cudaEventDestroy(t1); return stt; }
     // zero-mean solution into p_dyn, boundary cells by the reference's boundary conditions
-    mg_dot_kernel<<<g0, 128, 0, st>>>(L0.nk, L0.nj, L0.pitch, L0.plane, s->x, nullptr, nullptr, s->partial);
-    mg_sum_kernel<<<1, 1024, 0, st>>>(s->partial, s->nblocks, s->scal, 6);
+    dot(s, s->x, nullptr, nullptr, 6, st);
     mg_sub_mean_kernel<<<g0, 128, 0, st>>>(L0.nk, L0.pitch, L0.plane, s->x, s->scal, 6, count);
     mg_store_kernel<<<g0, 128, 0, st>>>(d, s->x, L0.nk, L0.pitch, L0.plane, ctx->field[ATHAD_P_DYN]);
     launch_poisson_bcs(pa, st);
