@@ -75,19 +75,25 @@ __device__ __forceinline__ T offdiag(const OpView<T>& o, const T* __restrict__ x
     return s;
 }
 
-// rows of one block's partial sum: the vector kernels take 128 longitudes of kRows rows, so
-// the one block that adds the partials has a quarter of them
+// The vector kernels take 128 longitudes of kRows rows per block, with one partial sum per
+// row (the order of the sums is part of the solve's rounding: CG carries a difference in the
+// last bits of its scalars into the solution's error).
 constexpr int kRows = 4;
 
-// the sum of v over the block's 128 threads, in a fixed order, into partial[block]
-__device__ __forceinline__ void block_partial(double v, double* __restrict__ partial)
+// the sums of v[0 .. kRows) over the block's 128 threads, in a fixed order, into the rows'
+// partials; nj rows per level
+__device__ __forceinline__ void block_partials(double (&v)[kRows], int nj, double* __restrict__ partial)
 {
-    __shared__ double red[4];
-    for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __shared__ double red[kRows][4];
+#pragma unroll
+    for (int r = 0; r < kRows; r++) {
+        for (int off = 16; off >= 1; off >>= 1) v[r] += __shfl_xor_sync(0xffffffffu, v[r], off);
+        if ((threadIdx.x & 31) == 0) red[r][threadIdx.x >> 5] = v[r];
+    }
     __syncthreads();
-    if (threadIdx.x == 0)
-        partial[((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
+    const int r = threadIdx.x, j = blockIdx.y * kRows + r;
+    if (r < kRows && j < nj)
+        partial[((long long)blockIdx.z * nj + j) * gridDim.x + blockIdx.x] = (red[r][0] + red[r][1]) + (red[r][2] + red[r][3]);
 }
 
 // q = S x in FP64, with per-block partial sums of x.q
@@ -98,16 +104,20 @@ __global__ void __launch_bounds__(128) mg_apply64_kernel(OpView<double> o, const
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait(k);
     const int i = blockIdx.z;
-    double v = 0.0;
-    if (k < o.nk)
-        for (int j = blockIdx.y * kRows; j < min((int)(blockIdx.y + 1) * kRows, o.nj); j++) {
+    double v[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; r++) {
+        const int j = blockIdx.y * kRows + r;
+        v[r] = 0.0;
+        if (k < o.nk && j < o.nj) {
             const long long c = i * o.plane + (long long)j * o.pitch + k;
             const double d = o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)];
             const double s = d * x[c] + offdiag(o, x, i, j, k, c);
             q[c] = s;
-            v += x[c] * s;
+            v[r] = x[c] * s;
         }
-    block_partial(v, partial);
+    }
+    block_partials(v, o.nj, partial);
 }
 
 // x += alpha d and r -= alpha q with alpha = s[0] / s[1], r rounded to FP32 for the
@@ -125,9 +135,12 @@ __global__ void __launch_bounds__(128) mg_update_kernel(int nk, int nj, int pitc
     pdl_wait(k);
     const int i = blockIdx.z;
     const double alpha = s[0] / s[1];
-    double v = 0.0;
-    if (k < nk)
-        for (int j = blockIdx.y * kRows; j < min((int)(blockIdx.y + 1) * kRows, nj); j++) {
+    double v[kRows];
+#pragma unroll
+    for (int u = 0; u < kRows; u++) {
+        const int j = blockIdx.y * kRows + u;
+        v[u] = 0.0;
+        if (k < nk && j < nj) {
             const long long c = i * plane + (long long)j * pitch + k;
             x[c] += alpha * d[c];
             if (!REFINE) {
@@ -135,14 +148,15 @@ __global__ void __launch_bounds__(128) mg_update_kernel(int nk, int nj, int pitc
                 r[c] = rn;
                 r32[c] = (float)rn;
                 const double a = rn * inv_w[i];
-                v += a * a;
+                v[u] = a * a;
             }
         }
-    if (!REFINE) block_partial(v, partial);
+    }
+    if (!REFINE) block_partials(v, nj, partial);
 }
 
-// r = rhs - S x in FP64 (the true residual), also rounded to FP32, partial sums of
-// (r num1(i))^2
+// r = rhs - S x in FP64 (the true residual), also rounded to FP32 (r32, may be null), partial
+// sums of (r num1(i))^2
 __global__ void __launch_bounds__(128) mg_true_residual_kernel(OpView<double> o, const double* __restrict__ x,
                                                                const double* __restrict__ rhs, double* __restrict__ r,
                                                                float* __restrict__ r32,
@@ -153,18 +167,22 @@ __global__ void __launch_bounds__(128) mg_true_residual_kernel(OpView<double> o,
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait(k);
     const int i = blockIdx.z;
-    double v = 0.0;
-    if (k < o.nk)
-        for (int j = blockIdx.y * kRows; j < min((int)(blockIdx.y + 1) * kRows, o.nj); j++) {
+    double v[kRows];
+#pragma unroll
+    for (int u = 0; u < kRows; u++) {
+        const int j = blockIdx.y * kRows + u;
+        v[u] = 0.0;
+        if (k < o.nk && j < o.nj) {
             const long long c = i * o.plane + (long long)j * o.pitch + k;
             const double d = o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)];
             const double s = rhs[c] - (d * x[c] + offdiag(o, x, i, j, k, c));
             r[c] = s;
-            r32[c] = (float)s;
+            if (r32) r32[c] = (float)s;
             const double a = s * inv_w[i];
-            v += a * a;
+            v[u] = a * a;
         }
-    block_partial(v, partial);
+    }
+    block_partials(v, o.nj, partial);
 }
 
 // per-block partial sums of a.b (b the FP32 preconditioned residual); of (a num1(i))^2 when b
@@ -177,15 +195,19 @@ __global__ void __launch_bounds__(128) mg_dot_kernel(int nk, int nj, int pitch, 
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait(k);
     const int i = blockIdx.z;
-    double v = 0.0;
-    if (k < nk)
-        for (int j = blockIdx.y * kRows; j < min((int)(blockIdx.y + 1) * kRows, nj); j++) {
+    double v[kRows];
+#pragma unroll
+    for (int u = 0; u < kRows; u++) {
+        const int j = blockIdx.y * kRows + u;
+        v[u] = 0.0;
+        if (k < nk && j < nj) {
             const long long c = i * plane + (long long)j * pitch + k;
-            if (b) v += a[c] * (double)b[c];
-            else if (inv_w) { const double t = a[c] * inv_w[i]; v += t * t; }
-            else v += a[c];
+            if (b) v[u] = a[c] * (double)b[c];
+            else if (inv_w) { const double t = a[c] * inv_w[i]; v[u] = t * t; }
+            else v[u] = a[c];
         }
-    block_partial(v, partial);
+    }
+    block_partials(v, nj, partial);
 }
 
 // fixed-order sum of n partials into out[slot] (one block of 1024 threads); next_rz: also the
@@ -197,7 +219,7 @@ __global__ void __launch_bounds__(1024) mg_sum_kernel(const double* __restrict__
     int first = threadIdx.x;
     pdl_wait(first);
     double v = 0.0;
-#pragma unroll 8
+#pragma unroll 16
     for (long long q = first; q < n; q += 1024) v += partial[q];
     __shared__ double red[32];
     for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -267,26 +289,28 @@ __device__ __forceinline__ float smooth_rhs(const OpView<float>& o, const float*
     return s;
 }
 
-// A CTA takes 32 columns of one row j.  Its kSmoothWarps warps form the right-hand sides (the
-// horizontal neighbours fixed), level by level, and stage them in shared memory; then warp 0
-// runs the two recurrences of its 32 columns from there, kSmoothChunk levels' operands loaded
-// ahead of the chain (a multiply-add and a product per level).  The elimination factors
+// A CTA takes 32 columns of one row j.  Its warps form the right-hand sides (the horizontal
+// neighbours fixed), level by level, and stage them in shared memory; then warp 0 runs the
+// two recurrences of its 32 columns from there, kSmoothChunk levels' operands loaded ahead of
+// the chain (a multiply-add and a product per level).  The couplings and elimination factors
 // depend on the row and the column class only, so they are staged once per CTA, before the
 // kernel before this one has finished.  The half-sweep also leaves the seam planes for the
 // next one in seam_out: the columns it relaxed, or what seam_in held.
 // FIRST: the first half-sweep from zero, which reads no e (the right-hand side is f) and
 // takes the seam planes as zero, so that nothing has to clear e.
-// Four warps, the factors per column in shared memory (30 KB per CTA instead of 10), the
-// operands of one level at a time, a launch before each half-sweep that copies the seam
-// planes, stored residuals and separate vector kernels: 71.3 ms per solve of 61x361x721, now
-// 48.1; 38x31x45 5.9 -> 3.1 ms, 33x223x149 16.8 -> 9.2 (the same iteration counts).
-constexpr int kSmoothWarps = 8, kSmoothChunk = 8;
-template <bool FIRST>
+// With the couplings read from global memory per cell, the factors per column in shared
+// memory, the operands of one level at a time, a launch before each half-sweep that copies the
+// seam planes, stored residuals and separate vector kernels a solve of 61x361x721 took 71.3
+// ms, now 39.6; 38x31x45 5.9 -> 2.9, 33x223x149 16.8 -> 8.9 (the same bits).  Rows
+// split by the parity of k (half the lines per half-sweep): 49.1 against 48.1 before the
+// couplings were staged.
+constexpr int kSmoothChunk = 8;
+template <bool FIRST, int kSmoothWarps>
 __global__ void __launch_bounds__(32 * kSmoothWarps) mg_smooth_split_kernel(
     OpView<float> o, const float* __restrict__ tm, const float* __restrict__ tc, const float* __restrict__ f,
     float* e, const float* seam_in, float* seam_out, int colour)
 {
-    extern __shared__ float sm[];   // rhs [ni][32]; factors m, coupling below, back factor: [ni][3] each
+    extern __shared__ float sm[];   // rhs [ni][32]; factors m, coupling below, back factor: [ni][3] each; couplings
     pdl_trigger();
     const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
     const int j = blockIdx.y;
@@ -298,20 +322,44 @@ __global__ void __launch_bounds__(32 * kSmoothWarps) mg_smooth_split_kernel(
     float* fm = sm + ni * 32;
     float* fc = fm + ni * 3;
     float* bc = fc + ni * 3;
+    float* js = bc + ni * 3;        // coupling to row j - 1, to row j + 1: [ni][3] each
+    float* jn = js + ni * 3;
+    float* kk = jn + ni * 3;        // coupling along k, across the seam: [ni] each
+    float* ks = kk + ni;
     for (int t = threadIdx.x; t < ni * 3; t += 32 * kSmoothWarps) {
         const int i = t / 3, w = t - 3 * i, at = (i * o.nj + j) * 3 + w;
         fm[t] = tm[at];
         fc[t] = (i > 0) ? o.ci[at - o.nj * 3] : 0.0f;
         bc[t] = tc[at];
+        if (!FIRST) {
+            js[t] = (j > 0) ? o.cj[at - 3] : 0.0f;
+            jn[t] = (j < o.nj - 1) ? o.cj[at] : 0.0f;
+            if (w == 0) { kk[i] = o.ck[i * o.nj + j]; ks[i] = o.cs[i * o.nj + j]; }
+        }
     }
+    __syncthreads();
     pdl_wait(k);
     const int kc = valid ? kclass(k, o.nk) : 1;
     const long long c0 = (long long)j * o.pitch + k;
     if (valid) {
+        // rows and columns outside the level are not read
+        const int up = (j > 0) ? o.pitch : 0, dn = (j < o.nj - 1) ? o.pitch : 0;
+        const int west = (k > 0) ? 1 : 0, east = (k < o.nk - 1) ? 1 : 0;
 #pragma unroll 4
         for (int i = q; i < ni; i += kSmoothWarps) {
             const long long c = i * o.plane + c0;
-            rhs[i * 32 + lane] = FIRST ? f[c] : smooth_rhs(o, f, e, seam_in, i, j, k, kc, c);
+            float s = f[c];
+            if (!FIRST) {
+                const float ej = e[c - up], en = e[c + dn], ew = e[c - west], ee = e[c + east];
+                if (up) s -= js[i * 3 + kc] * ej;
+                if (dn) s -= jn[i * 3 + kc] * en;
+                const float ckv = kk[i];
+                if (west) s -= ckv * ew;
+                if (east) s -= ckv * ee;
+                if (!west) s -= ks[i] * seam_in[planes + i * o.nj + j];       // plane k = nk-1
+                else if (!east) s -= ks[i] * seam_in[i * o.nj + j];           // plane k = 0
+            }
+            rhs[i * 32 + lane] = s;
         }
     }
     __syncthreads();
@@ -420,9 +468,23 @@ __global__ void __launch_bounds__(128) mg_restrict_kernel(OpView<float> o, const
     const int J = blockIdx.y, i = blockIdx.z;
     if (K >= nk_c) return;
     const int j0 = 2 * J, k0 = 2 * K;
+    // the roundings spelled out: CG carries a difference in the preconditioner's last bits into
+    // the solution's error (to 5e-9 of p at a 1e-10 residual on small grids)
     auto residual = [&](int j, int k) {
+        const int kc = kclass(k, o.nk), ij = i * o.nj + j;
         const long long c = i * o.plane + (long long)j * o.pitch + k;
-        return f[c] - (o.diag[(i * o.nj + j) * 3 + kclass(k, o.nk)] * e[c] + offdiag(o, e, i, j, k, c));
+        float t = 0.0f;
+        if (i > 0) t = fmaf(o.ci[(ij - o.nj) * 3 + kc], e[c - o.plane], t);
+        if (i < o.ni - 1) t = fmaf(o.ci[ij * 3 + kc], e[c + o.plane], t);
+        if (j > 0) t = fmaf(o.cj[(ij - 1) * 3 + kc], e[c - o.pitch], t);
+        if (j < o.nj - 1) t = fmaf(o.cj[ij * 3 + kc], e[c + o.pitch], t);
+        const float ckv = o.ck[ij];
+        if (k > 0) t = fmaf(ckv, e[c - 1], t);
+        if (k < o.nk - 1) t = fmaf(ckv, e[c + 1], t);
+        if (k == 0) t = fmaf(o.cs[ij], e[c + (o.nk - 1)], t);
+        else if (k == o.nk - 1) t = fmaf(o.cs[ij], e[c - (o.nk - 1)], t);
+        const float dg = o.diag[ij * 3 + kc];
+        return __fsub_rn(f[c], __fadd_rn(__fmul_rn(dg, e[c]), t));
     };
     float s = residual(j0, k0);
     if (k0 + 1 < o.nk) s += residual(j0, k0 + 1);
@@ -435,22 +497,34 @@ __global__ void __launch_bounds__(128) mg_restrict_kernel(OpView<float> o, const
 
 // fine e += scale * coarse e of the aggregate.  A piecewise-constant prolongation
 // under-corrects smooth errors; a constant scale keeps the V-cycle symmetric.
-__global__ void __launch_bounds__(128) mg_prolong_kernel(int nk_f, int pitch_f, long long plane_f, float* __restrict__ e,
-                                                         int pitch_c, long long plane_c, const float* __restrict__ ec,
-                                                         float* __restrict__ seam)
+// A thread takes the two longitudes of one aggregate (an 8-byte access; the rows are 128-byte
+// aligned and padded) in kRows rows: 68 us with a thread per cell on the finest level of
+// 61x361x721.
+__global__ void __launch_bounds__(128) mg_prolong_kernel(int nk_f, int nj_f, int pitch_f, long long plane_f,
+                                                         float* __restrict__ e, int pitch_c, long long plane_c,
+                                                         const float* __restrict__ ec, float* __restrict__ seam)
 {
     pdl_trigger();
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    pdl_wait(k);
-    const int j = blockIdx.y, i = blockIdx.z;
-    if (k >= nk_f) return;
-    const long long c = i * plane_f + (long long)j * pitch_f + k;
-    const float v = e[c] + ATHAD_MG_CSCALE * ec[i * plane_c + (long long)(j >> 1) * pitch_c + (k >> 1)];
-    e[c] = v;
-    // the seam planes of the post-smoother's first half-sweep
-    const int ij = i * gridDim.y + j;
-    if (k == 0) seam[ij] = v;
-    if (k == nk_f - 1) seam[gridDim.z * gridDim.y + ij] = v;
+    int K = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(K);
+    const int i = blockIdx.z;
+    if (2 * K >= nk_f) return;
+    const bool two = 2 * K + 1 < nk_f;
+    const int planes = gridDim.z * nj_f;
+#pragma unroll
+    for (int r = 0; r < kRows; r++) {
+        const int j = blockIdx.y * kRows + r;
+        if (j >= nj_f) break;
+        float* at = e + i * plane_f + (long long)j * pitch_f + 2 * K;
+        const float c = ec[i * plane_c + (long long)(j >> 1) * pitch_c + K];
+        float2 v = *reinterpret_cast<float2*>(at);
+        v.x = fmaf(ATHAD_MG_CSCALE, c, v.x);
+        if (two) v.y = fmaf(ATHAD_MG_CSCALE, c, v.y);
+        *reinterpret_cast<float2*>(at) = v;
+        // the seam planes of the post-smoother's first half-sweep
+        if (K == 0) seam[i * nj_f + j] = v.x;
+        if (2 * K + 2 >= nk_f) seam[planes + i * nj_f + j] = two ? v.y : v.x;
+    }
 }
 
 // right-hand side of S: rhs_c = -src_c / num1(i) at every interior cell
@@ -663,7 +737,7 @@ MGSolver* mg_build(athad_ctx* ctx, std::string& err)
     const size_t off_w = add(ni * sizeof(double));
     size_t off_v[5];
     for (int v = 0; v < 5; v++) off_v[v] = add(L0.n * sizeof(double));
-    s->nblocks = (long long)((L0.nk + 127) / 128) * ((L0.nj + kRows - 1) / kRows) * L0.ni;
+    s->nblocks = (long long)((L0.nk + 127) / 128) * L0.nj * L0.ni;
     const size_t off_p = add(s->nblocks * sizeof(double));
     const size_t off_s = add(64 * sizeof(double));
     const size_t off_seam = add((size_t)4 * ni * nj * sizeof(float));
@@ -720,9 +794,15 @@ namespace {
 inline dim3 cells_grid(int nk, int nj, int ni) { return dim3((nk + 127) / 128, nj, ni); }
 inline dim3 rows_grid(const MGLevel& L) { return dim3((L.nk + 127) / 128, (L.nj + kRows - 1) / kRows, L.ni); }
 
-// the staged right-hand sides and factors of a smoother CTA; columns of up to 299 levels
-inline size_t smooth_smem(const MGLevel& L) { return (size_t)(32 + 9) * L.ni * sizeof(float); }
+// the staged right-hand sides and factors of a smoother CTA; columns of up to 250 levels
+inline size_t smooth_smem(const MGLevel& L) { return (size_t)(32 + 17) * L.ni * sizeof(float); }
 inline bool smooth_fits(const MGLevel& L) { return smooth_smem(L) <= 48 * 1024; }
+
+// Warps of a smoother CTA.  Only its first warp has work in the recurrences, so where the
+// CTAs fill the SMs several times over (the fine levels) four warps keep more columns in them
+// (solve of 61x361x721: 39.8 ms with 4, 43.4 with 8, 45.9 with 2); where they do not, eight
+// shorten the staging (33x223x149: 8.6 ms with 8, 9.0 with 16).
+constexpr int kWarpsMany = 4, kWarpsFew = 8, kManySmooth = 148 * 8;
 
 // one half-sweep of level L; `half` counts the half-sweeps of a sequence (the seam planes
 // alternate between two buffers), from_zero: L.e is zero and need not be stored so
@@ -733,13 +813,16 @@ void smooth(MGSolver* s, const MGLevel& L, int colour, int half, bool from_zero,
     float* out = seam[(half + 1) & 1];
     const int nh = (L.nk + 1) / 2;
     if (smooth_fits(L)) {
-        const dim3 grid((nh + 31) / 32, L.nj), block(32 * kSmoothWarps);
-        if (from_zero)
-            launch_dependent(mg_smooth_split_kernel<true>, grid, block, smooth_smem(L), st, L.op, (const float*)L.tm,
+        const dim3 grid((nh + 31) / 32, L.nj);
+        const bool many = (long long)grid.x * grid.y >= kManySmooth;
+        auto launch = [&](auto kernel, int warps) {
+            launch_dependent(kernel, grid, dim3(32 * warps), smooth_smem(L), st, L.op, (const float*)L.tm,
                              (const float*)L.tc, (const float*)L.f, L.e, (const float*)in, out, colour);
-        else
-            launch_dependent(mg_smooth_split_kernel<false>, grid, block, smooth_smem(L), st, L.op, (const float*)L.tm,
-                             (const float*)L.tc, (const float*)L.f, L.e, (const float*)in, out, colour);
+        };
+        if (from_zero && many) launch(mg_smooth_split_kernel<true, kWarpsMany>, kWarpsMany);
+        else if (from_zero) launch(mg_smooth_split_kernel<true, kWarpsFew>, kWarpsFew);
+        else if (many) launch(mg_smooth_split_kernel<false, kWarpsMany>, kWarpsMany);
+        else launch(mg_smooth_split_kernel<false, kWarpsFew>, kWarpsFew);
         return;
     }
     if (from_zero) cudaMemsetAsync(L.e, 0, L.n * sizeof(float), st);
@@ -762,8 +845,8 @@ void vcycle(MGSolver* s, int l, cudaStream_t st)
     launch_dependent(mg_restrict_kernel, cells_grid(C.nk, C.nj, C.ni), dim3(128), 0, st, L.op, (const float*)L.e,
                      (const float*)L.f, C.nk, C.pitch, C.plane, C.f);
     vcycle(s, l + 1, st);
-    launch_dependent(mg_prolong_kernel, cells_grid(L.nk, L.nj, L.ni), dim3(128), 0, st, L.nk, L.pitch, L.plane, L.e,
-                     C.pitch, C.plane, (const float*)C.e, s->seam);
+    launch_dependent(mg_prolong_kernel, dim3((C.nk + 127) / 128, (L.nj + kRows - 1) / kRows, L.ni), dim3(128), 0, st, L.nk,
+                     L.nj, L.pitch, L.plane, L.e, C.pitch, C.plane, (const float*)C.e, s->seam);
     for (int it = 0; it < 2 * ATHAD_MG_NU; it++) smooth(s, L, 1 - (it & 1), it, false, st);
 }
 
@@ -781,12 +864,12 @@ void dot(MGSolver* s, const double* a, const float* b, const double* inv_w, int 
     sum(s, slot, false, st);
 }
 
-// true residual r = rhs - S x with its A-form norm into scal[3]
-void true_residual(MGSolver* s, cudaStream_t st)
+// true residual rhs - S x into r (and r32) with its A-form norm into scal[3]
+void true_residual(MGSolver* s, double* r, float* r32, cudaStream_t st)
 {
     const MGLevel& L0 = s->L[0];
     launch_dependent(mg_true_residual_kernel, rows_grid(L0), dim3(128), 0, st, s->op64, (const double*)s->x,
-                     (const double*)s->rhs, s->r, L0.f, (const double*)s->inv_w, s->partial);
+                     (const double*)s->rhs, r, r32, (const double*)s->inv_w, s->partial);
     sum(s, 3, false, st);
 }
 
@@ -802,7 +885,7 @@ void enqueue_step(MGSolver* s, bool refine, cudaStream_t st)
         launch_dependent(mg_update_kernel<true>, rows_grid(L0), dim3(128), 0, st, L0.nk, L0.nj, L0.pitch, L0.plane,
                          (const double*)s->scal, (const double*)s->d, s->x, (const double*)s->q, s->r, L0.f,
                          (const double*)s->inv_w, s->partial);
-        true_residual(s, st);
+        true_residual(s, s->r, L0.f, st);
     } else {
         launch_dependent(mg_update_kernel<false>, rows_grid(L0), dim3(128), 0, st, L0.nk, L0.nj, L0.pitch, L0.plane,
                          (const double*)s->scal, (const double*)s->d, s->x, (const double*)s->q, s->r, L0.f,
@@ -897,25 +980,33 @@ extern "C" athad_status athad_pressure_solve(athad_ctx* ctx, double rel_tol, int
     }
     double res = (h[4] > 0.0) ? 1.0 : 0.0;
     int it = 0;
+    bool have_direction = true;
     for (it = 1; it <= max_iter && h[4] > 0.0 && stt == ATHAD_OK; it++) {
         const bool refine = (it % 8 == 0);
         // the direction is formed only when another step follows
-        if (it > 1) stt = cuda_check(ctx, cudaGraphLaunch(s->iter_graph[2], st), "pressure_solve direction");
+        if (!have_direction) stt = cuda_check(ctx, cudaGraphLaunch(s->iter_graph[2], st), "pressure_solve direction");
         if (stt == ATHAD_OK) stt = cuda_check(ctx, cudaGraphLaunch(s->iter_graph[refine ? 1 : 0], st), "pressure_solve step");
+        have_direction = false;
         if (stt == ATHAD_OK) stt = cuda_check(ctx, cudaStreamSynchronize(st), "pressure_solve");
         if (stt != ATHAD_OK) break;
         res = std::sqrt(s->h[3] / h[4]);
         if (it <= 64) rep.history[it - 1] = res;
         if (res <= rel_tol) {
             if (refine) break;
-            // confirm with the true residual before stopping
-            true_residual(s, st);
+            // confirm with the true residual before stopping; where it is larger, the next
+            // direction still comes from the recursive one and the true one replaces it
+            true_residual(s, s->q, nullptr, st);
             cudaMemcpyAsync(s->h, s->scal, 5 * sizeof(double), cudaMemcpyDeviceToHost, st);
             stt = cuda_check(ctx, cudaStreamSynchronize(st), "pressure_solve");
             if (stt != ATHAD_OK) break;
             res = std::sqrt(s->h[3] / h[4]);
             if (it <= 64) rep.history[it - 1] = res;
             if (res <= rel_tol) break;
+            stt = cuda_check(ctx, cudaGraphLaunch(s->iter_graph[2], st), "pressure_solve direction");
+            if (stt == ATHAD_OK)
+                stt = cuda_check(ctx, cudaMemcpyAsync(s->r, s->q, n * sizeof(double), cudaMemcpyDeviceToDevice, st),
+                                 "pressure_solve residual");
+            have_direction = true;
         }
     }
     if (stt != ATHAD_OK) { cudaEventDestroy(t0); cudaEventDestroy(t1); return stt; }
