@@ -50,57 +50,6 @@ __host__ __device__ void evaporate_where_impossible(const ColumnArgs& a, long lo
     a.S_g[c] = 0.0; a.S_c_c[c] = 0.0;
 }
 
-// The Newton step's saturation curves (thermo.cuh: SaturationH2O.h:68-120, 168-178,
-// 230-255) with the reciprocals they divide by formed once: 1/T per Newton step, shared by
-// the saturation and sublimation curves and the derivative factor, and 1/p per cell.  A
-// product by a reciprocal instead of a quotient moves a result by at most an ulp or two.
-__host__ __device__ __forceinline__ double p_sat_r(double T, double invT)
-{
-    if (T >= T_CRIT) return NO_SATURATION;
-    if (T <= 0.0) return 0.0;
-    const double theta = 1.0 - T * (1.0 / T_CRIT);
-    const double sq = sqrt(theta);
-    const double t15 = theta * sq;
-    const double t3 = theta * theta * theta;
-    const double t35 = t3 * sq;
-    const double t4 = t3 * theta;
-    const double t75 = t4 * t3 * sq;
-    const double sum = -7.85951783 * theta + 1.84408259 * t15 + -11.7866497 * t3
-                     + 22.6807411 * t35 + -15.9618719 * t4 + 1.80122502 * t75;
-    return 220640.0 * exp((T_CRIT * invT) * sum);
-}
-__host__ __device__ __forceinline__ double p_subl_r(double T, double invT)
-{
-    if (T <= 0.0) return 0.0;
-    const double lt = log(T * (1.0 / T_TRIPLE));
-    // theta^(1/300): the exponent is within 0.004 for T of 82 to 907 K, where the series to
-    // the fifth power is exact to less than an ulp (x^6 / 720 < 6e-18)
-    const double x = 0.333333333e-2 * lt;
-    const double r = (fabs(x) < 0.004)
-        ? 1.0 + x * (1.0 + x * (0.5 + x * (1.0 / 6.0 + x * (1.0 / 24.0 + x * (1.0 / 120.0))))) : exp(x);
-    const double sum = -0.212144006e2 * r + 0.273203819e2 * exp(0.120666667e1 * lt)
-                     + -0.610598130e1 * exp(0.170333333e1 * lt);
-    return 6.11657 * exp(sum * (T_TRIPLE * invT));
-}
-// saturation mass fraction and its derivative factor (dq_sat/dT = A L / (R_H2O T^2)) from one
-// division.  The Newton step issues its instructions at 70 % of the rate (no loads to wait
-// for), so its count is its time: this, the shared cp and the 1/T of the heat capacities take
-// it from 12 divisions to 6 (704 -> 610 us for the kernel, 527 -> 479 M warp instructions;
-// most cells, four of five, take 3 to 5 steps, and the ice curve is needed in nearly all of
-// them because transport leaves traces of ice everywhere)
-struct SatValue { double q, A; };
-__host__ __device__ __forceinline__ SatValue sat_value(double E, double p, double inv_p, double M_other)
-{
-    if (E == NO_SATURATION) return {1.0, 0.0};
-    if (!(p > 0.0)) return {0.0, 0.0};
-    if (E >= p) return {1.0, 0.0};
-    const double x = E * inv_p;
-    const double num = x * M_H2O;
-    const double den = num + (1.0 - x) * M_other;
-    if (!(den > 0.0)) return {1.0, 0.0};
-    const double r = 1.0 / den;
-    return {num * r, num * M_other * (r * r)};
-}
 // The mixture heat capacity of the Newton step (MixtureAtm.h:123-178) with the three
 // Shomate polynomials sharing t, t^2, t^3 and 1/t^2, and products by the reciprocal molar
 // masses: one division instead of six.  Split in two: the specific heats of the three

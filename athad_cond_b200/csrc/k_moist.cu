@@ -244,15 +244,23 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
             const double p_b = p->F[ATHAD_P_STAT][cb];
             const double qsb = QSC(i_base);
             const double L_b = (T_b >= t_0) ? p->lv : p->ls;
-            const double th_p = T_b * pow(p->p_0 / p_b, kappa) * exp(L_b * qsb / (p->cp_l * T_b));
+            const double th_p = T_b * exp(kappa * log(p->p_0 / p_b) + L_b * qsb / (p->cp_l * T_b));
             int became = 0, i_top = i_base;
             double cape = 0.0;
+            // the next level's values are loaded while this level computes
+            double Tn = 0.0, Pn = 0.0, Cn = 0.0;
+            if (i_base + 1 < im) { Tn = p->F[ATHAD_T][cb + plane_s]; Pn = p->F[ATHAD_P_STAT][cb + plane_s]; Cn = p->F[ATHAD_C][cb + plane_s]; }
             for (int i = i_base + 1; i < im; i++) {
-                const long long c = IDX(i, j, k);
-                const double T_e = p->F[ATHAD_T][c] * t_0;
-                const double p_e = p->F[ATHAD_P_STAT][c];
+                const double T_i = Tn, p_e = Pn, C_i = Cn;
+                if (i + 1 < im) {
+                    const long long cn = IDX(i + 1, j, k);
+                    Tn = p->F[ATHAD_T][cn]; Pn = p->F[ATHAD_P_STAT][cn]; Cn = p->F[ATHAD_C][cn];
+                }
+                const double T_e = T_i * t_0;
                 const double L_e = (T_e >= t_0) ? p->lv : p->ls;
-                const double th_e = T_e * pow(p->p_0 / p_e, kappa) * exp(L_e * QSC(i) / (p->cp_l * T_e));
+                const double qs_e = safe_q_sat(X, saturation_pressure_auto(T_i * t_0 + MC_T_ADD_U), p_e, C_i);
+                // (p_0 / p_e)^kappa exp(L q / (cp T)) as one exponential
+                const double th_e = T_e * exp(kappa * log(p->p_0 / p_e) + L_e * qs_e / (p->cp_l * T_e));
                 if (th_p - th_e > 0.0) {
                     became = 1;
                     i_top = i;
@@ -537,22 +545,35 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 }
                 double cu = 0.0;
                 if (fabs(Mu) > MC_COEFF_RECURR) {
+                    // Two condensation steps, a chain of transcendentals and quotients that
+                    // nothing overlaps: the quotients by T, p and the mixture masses are formed
+                    // once, and the step's share dq / (1 + G) from one division.
                     double T_u = su * p->s_0 / p->cp_l;
-                    const double p_u = cur.P;
+                    const double p_u = cur.P, inv_p = 1.0 / p_u;
+                    const double M_ref = M_nonwater(cur.C, X.co2_0, X.M_bg);
+                    const double M_o_u = M_nonwater(cur.C, cur.CO2, p->M_bg);
                     double dcond_tot = 0.0;
                     for (int it = 0; it < 2; ++it) {
-                        const double E_s = saturation_pressure_auto(T_u);
-                        const double q_sat_u = safe_q_sat(X, E_s, p_u, cur.C);
-                        const double dq = qvu - q_sat_u;
+                        const double inv_T = 1.0 / T_u;
+                        const double E_s = (T_u >= T_CRIT) ? NO_SATURATION
+                                         : (T_u >= T_TRIPLE) ? p_sat_r(T_u, inv_T) : p_subl_r(T_u, inv_T);
+                        const double dq = qvu - sat_value(E_s, p_u, inv_p, M_ref).q;
                         if (dq <= 0.0) break;
-                        const double L_u = (T_u >= t_0) ? p->lv : p->ls;
-                        const double M_o_u = M_nonwater(cur.C, cur.CO2, p->M_bg);
-                        const double dqsdT = dqsat_dT_from(E_s, latent_heat_auto(T_u), T_u, p_u, M_o_u);
-                        const double G = (L_u / p->cp_l) * dqsdT;
-                        const double dcond = dq / (1.0 + G);
+                        const double L_cp = ((T_u >= t_0) ? p->lv : p->ls) / p->cp_l;
+                        // G = L / cp_l dq_sat/dT = N / D (sat_deriv_factor_at, dqsat_dT_from)
+                        double N = 0.0, D = 1.0;
+                        if (T_u > 0.0 && E_s != NO_SATURATION && p_u > 0.0 && !(E_s >= p_u)) {
+                            const double x = E_s * inv_p;
+                            const double den = x * M_H2O + (1.0 - x) * M_o_u;
+                            if (den > 0.0) {
+                                D = den * den;
+                                N = L_cp * (x * M_H2O * M_o_u) * latent_heat_auto(T_u) * ((inv_T * inv_T) * (1.0 / R_H2O));
+                            }
+                        }
+                        const double dcond = dq * D / (D + N);
                         qvu -= dcond;
                         qcu += dcond;
-                        T_u += (L_u / p->cp_l) * dcond;
+                        T_u += L_cp * dcond;
                         dcond_tot += dcond;
                     }
                     su = p->cp_l * T_u / p->s_0;
@@ -678,8 +699,10 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 } else {
                     double edd;
                     if (precip_i > 0.0) {
-                        const double P_16 = pow(precip_i, 1.0 / 6.0);
-                        const double P_49 = pow(precip_i, 4.0 / 9.0);
+                        // powers 1/6 and 4/9 from cube roots (within two ulp of pow)
+                        const double P_13 = cbrt(precip_i);
+                        const double P_16 = sqrt(P_13);
+                        const double P_49 = P_13 * cbrt(P_13);
                         edd = MC_A_EV * (1.0 + MC_B_EV * P_16) * sub_rn(q_sat, qvd) * P_49;
                     } else {
                         edd = 0.0;
