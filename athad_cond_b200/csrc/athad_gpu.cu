@@ -679,6 +679,8 @@ void athad::mixed_args(athad_ctx* ctx, const athad_step_scalars* s, RK4MArgs& a)
     a.write_diag = s->write_diagnostics & 1;
     a.store_n = s->store_n_level ? 1 : 0;
     for (int n = 0; n < kNY; n++) a.Yn_store[n] = ctx->field[ATHAD_TN + n];
+    static_assert(ATHAD_P_SNOW == ATHAD_P_RAIN + 1 && ATHAD_P_SNOWN == ATHAD_P_RAINN + 1, "stage 4 copies both");
+    a.rain = F[ATHAD_P_RAIN]; a.rain_n = F[ATHAD_P_RAINN];
 }
 
 extern "C" {
@@ -699,7 +701,7 @@ static athad_status rk4_step_mixed(athad_ctx* ctx, const athad_step_scalars* s)
         launch_rk4m_stage(stage, a, ctx->stream);
         ATHAD_CHECK_LAUNCH(ctx, "rk4 mixed stage");
     }
-    return s->store_n_level ? store_precip_n_level(ctx, ctx->stream) : ATHAD_OK;
+    return ATHAD_OK;
 }
 
 static PoissonArgs poisson_args(athad_ctx* ctx, int total_iter_count)

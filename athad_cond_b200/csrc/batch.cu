@@ -1,21 +1,28 @@
 // batch.cu - ensembles of contexts advanced together (athad_batch_* of include/athad_gpu.h).
 //
 // A batch owns no field memory: its members are ordinary mixed-precision contexts, each
-// with its own grid and parameters.  One batched model iteration enqueues each member's
-// column physics at that member's own cadence (pressure sweep every 4th iteration,
-// saturation adjustment + moist convection + densities every 2nd) on a few side streams
-// forked from the batch's stream and joined back to it, so that the small kernels of
-// different members run side by side (a member's column kernels fill only part of the
-// GPU: one thread per column, or latency-bound recurrences), then on the batch's stream the
-// level mean of all members in one launch, the four RK4 stages of all members as one
-// persistent launch each (k_rk4m.cu), with the time-level copy fused into stage 4, and a
-// tiny launch that advances the members' device-side iteration counters.
+// with its own grid and parameters.  One batched model iteration forks a few side streams
+// (lanes) from the batch's stream, enqueues each member's iteration on one of them - the
+// column physics at the member's own cadence (pressure sweep every 4th iteration, saturation
+// adjustment + moist convection + densities every 2nd), the level mean, the four RK4 stages
+// with the time-level copy fused into the last - and joins the lanes in a tiny launch that
+// advances the members' device-side iteration counters.
+//
+// The members depend on one another nowhere, so a lane never waits for another: a member's
+// column kernels, which fill only part of the GPU (one thread per column, latency-bound
+// recurrences), run beside other members' RK4 stages, which are bound by memory traffic.
+// One persistent launch per stage over the tiles of all members, behind a join of all
+// column physics, was 1.56 times slower per point than the single-grid stage kernels (a
+// member's arguments in shared memory, neighbouring planes read at unrelated times).  Four
+// iterations, persistent -> lanes: six members of 0.4 to 2.4 M points 19.1 -> 13.8 ms,
+// twelve of 27x99x151 15.3 -> 11.4, six of 15x61x109 2.37 -> 1.69, 32 of 11x21x41 2.68 ->
+// 2.57, one of 31x125x257 3.91 -> 3.06.
 //
 // Step scalars live on the device: every member's buoyancy ramp min(1, n / ramp_iters) is
-// formed inside the stage kernels from its iteration counter, so one captured CUDA graph
-// of an iteration stays valid from step to step.  Graphs are keyed by what changes the
-// launch list: each member's cadence (pressure sweep? column physics?), its pressure
-// ceiling (above 300 iterations) and the tile shape; a batch replays at most a handful.
+// in its step record, kept with its iteration counter, so one captured CUDA graph of an
+// iteration stays valid from step to step.  Graphs are keyed by what changes the launch
+// list: each member's cadence (pressure sweep? column physics?), its pressure ceiling (above
+// 300 iterations) and the tile shape; a batch replays at most a handful.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -27,17 +34,25 @@
 
 namespace athad {
 
+// the buoyancy prefactor of a member's iteration, ramp min(1, iter / ramp_iters)
+__host__ __device__ inline float batch_buoyancy(const BatchStep& st)
+{
+    const double x = (double)st.iter / (double)st.ramp_iters;
+    const double ramp = (x < 1.0) ? x : 1.0;
+    return (float)(ramp * st.g * st.dt / st.u_0);
+}
+
 __global__ void batch_advance_kernel(BatchStep* step, int n)
 {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m < n && step[m].active) step[m].iter += 1;
+    if (m >= n || !step[m].active) return;
+    step[m].iter += 1;
+    step[m].buoy_pref = batch_buoyancy(step[m]);
 }
 
 }  // namespace athad
 
 namespace {
-
-constexpr int kMaxShapes = 8;
 
 struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
@@ -45,28 +60,23 @@ struct GraphEntry {
 
 }  // namespace
 
-constexpr int kSideStreams = 8;   // concurrent column-physics lanes of a batched iteration
+// Lanes of a batched iteration.  Four iterations with 4, 8, 16, 32 lanes: 32 members of
+// 11x21x41 3.73, 2.53, 2.00, 1.76 ms; 16 of 15x61x109 4.52, 4.14, 3.81, 3.80; twelve of
+// 27x99x151 11.6, 11.2, 10.9, 11.0.
+constexpr int kSideStreams = 32;
 
 struct athad_batch {
     std::vector<athad_ctx*> m;
-    std::vector<cudaStream_t> side;     // member q's column physics runs on side[q % size]
+    std::vector<cudaStream_t> side;     // member q's iteration runs on side[q % size]
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> join;
+    std::vector<RK4MArgs> args;         // the members' stage arguments (stage buffer A in Yout, B in Ybnd)
     std::vector<int32_t> iter;          // host mirror of each member's next iteration number
     std::vector<uint8_t> active;
-    athad_batch_step step{};
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
-    char* dev = nullptr;                // device tables, one allocation
-    RK4MArgs* d_args = nullptr;
-    BatchStep* d_step = nullptr;
-    int* d_tiles = nullptr;             // [shapes][n+1]
-    LevelMeanMember* d_lm = nullptr;
-    int n_shapes = 0;
-    int shape = 0;
-    int grid[kMaxShapes] = {};
-    int total_tiles[kMaxShapes] = {};
-    int total_levels = 0, max_jm = 0;
+    BatchStep* d_step = nullptr;        // [n] step records on the device
+    int shape = 0;                      // tile shape of the RK4 stages
     std::map<std::vector<uint8_t>, GraphEntry> graphs;
     std::string err;
 };
@@ -91,59 +101,73 @@ static void drop_graphs(athad_batch* b)
     b->graphs.clear();
 }
 
-// Enqueue one iteration of every active member on b->stream (also used under capture).
-static athad_status enqueue_iteration(athad_batch* b)
+// A member's column physics at its cadence, on its context's stream.
+static athad_status enqueue_columns(athad_ctx* c, int it)
 {
-    const int n = (int)b->m.size();
-    const int ns = (int)b->side.size();
-    athad_status sf = bcuda(b, cudaEventRecord(b->fork, b->stream), "batch fork");
-    for (int q = 0; q < ns && sf == ATHAD_OK; q++) sf = bcuda(b, cudaStreamWaitEvent(b->side[q], b->fork, 0), "batch fork");
-    if (sf != ATHAD_OK) return sf;
+    athad_status s = ATHAD_OK;
+    if (it % 4 == 0) s = athad_pressure_sweep(c, 1, it);
+    if (s == ATHAD_OK && it % 2 == 0) {
+        s = athad_saturation_adjust(c);
+        if (s == ATHAD_OK) s = athad_moist_convection(c, it);
+        if (s == ATHAD_OK) s = athad_densities(c, 0);
+    }
+    return s;
+}
+
+// The level mean (single-grid kernels) and an RK4 stage of member q on its context's stream.
+static athad_status enqueue_level_mean(athad_ctx* c)
+{
+    launch_level_mean(c->L.d, c->field[ATHAD_T], c->sin_w, c->prof[ATHAD_PROF_T_REF_LEVEL], c->row_sum, c->stream, nullptr);
+    return cuda_check(c, cudaGetLastError(), "batch level mean");
+}
+
+static athad_status enqueue_stage(athad_batch* b, int q, int stage, int shape)
+{
+    athad_ctx* c = b->m[q];
+    RK4MArgs& a = b->args[q];
+    for (int f = 0; f < kMixedGroups; f++) {
+        a.Yin[f] = (stage == 3) ? c->mB[f] : c->mA[f];
+        a.Yout[f] = (stage == 1 || stage == 3) ? c->mA[f] : c->mB[f];
+    }
+    launch_rk4m_member_stage(stage, shape, a, b->d_step + q, c->stream);
+    return cuda_check(c, cudaGetLastError(), "batch rk4 stage");
+}
+
+// Runs enqueue(q) for every active member with its context's stream on the member's lane,
+// between a fork of the lanes from b->stream and their join to it (also under capture).
+template <class F> static athad_status on_lanes(athad_batch* b, F enqueue)
+{
+    const int n = (int)b->m.size(), ns = (int)b->side.size();
+    athad_status s = bcuda(b, cudaEventRecord(b->fork, b->stream), "batch fork");
+    for (int q = 0; q < ns && s == ATHAD_OK; q++) s = bcuda(b, cudaStreamWaitEvent(b->side[q], b->fork, 0), "batch fork");
+    if (s != ATHAD_OK) return s;
     for (int q = 0; q < n; q++) {
         if (!b->active[q]) continue;
         athad_ctx* c = b->m[q];
         cudaStream_t saved = c->stream;
         c->stream = b->side[q % ns];
-        const int it = b->iter[q];
-        athad_status s = ATHAD_OK;
-        if (it % 4 == 0) s = athad_pressure_sweep(c, 1, it);
-        if (s == ATHAD_OK && it % 2 == 0) {
-            s = athad_saturation_adjust(c);
-            if (s == ATHAD_OK) s = athad_moist_convection(c, it);
-            if (s == ATHAD_OK) s = athad_densities(c, 0);
-        }
+        s = enqueue(q);
         c->stream = saved;
         if (s != ATHAD_OK) return bfail(b, s, std::string("member ") + std::to_string(q) + ": " + c->err);
     }
-    for (int q = 0; q < ns; q++) {   // join: the batched kernels below read every member's state
-        athad_status sj = bcuda(b, cudaEventRecord(b->join[q], b->side[q]), "batch join");
-        if (sj == ATHAD_OK) sj = bcuda(b, cudaStreamWaitEvent(b->stream, b->join[q], 0), "batch join");
-        if (sj != ATHAD_OK) return sj;
+    for (int q = 0; q < ns && s == ATHAD_OK; q++) {
+        s = bcuda(b, cudaEventRecord(b->join[q], b->side[q]), "batch join");
+        if (s == ATHAD_OK) s = bcuda(b, cudaStreamWaitEvent(b->stream, b->join[q], 0), "batch join");
     }
-    launch_batch_level_mean(b->d_lm, n, b->total_levels, b->max_jm, b->d_step, b->stream);
-    athad_status s = bcuda(b, cudaGetLastError(), "batch level mean");
+    return s;
+}
+
+// Enqueue one iteration of every active member on b->stream (also used under capture).
+static athad_status enqueue_iteration(athad_batch* b)
+{
+    const int n = (int)b->m.size();
+    athad_status s = on_lanes(b, [b](int q) {
+        athad_status r = enqueue_columns(b->m[q], b->iter[q]);
+        if (r == ATHAD_OK) r = enqueue_level_mean(b->m[q]);
+        for (int stage = 1; stage <= 4 && r == ATHAD_OK; stage++) r = enqueue_stage(b, q, stage, b->shape);
+        return r;
+    });
     if (s != ATHAD_OK) return s;
-    BatchTables T;
-    T.args = b->d_args;
-    T.step = b->d_step;
-    T.tile_start = b->d_tiles + (size_t)b->shape * (n + 1);
-    T.n = n;
-    T.total_tiles = b->total_tiles[b->shape];
-    for (int stage = 1; stage <= 4; stage++) {
-        launch_rk4m_batch_stage(stage, b->shape, T, b->grid[b->shape], b->stream);
-        s = bcuda(b, cudaGetLastError(), "batch rk4 stage");
-        if (s != ATHAD_OK) return s;
-    }
-    // the time-level copy's precipitation fluxes (UtilsAtm.h:41-42); the stage kernel wrote
-    // the eleven prognostic fields' level n
-    for (int q = 0; q < n; q++) {
-        if (!b->active[q]) continue;
-        athad_ctx* c = b->m[q];
-        s = bcuda(b, cudaMemcpyAsync(c->field[ATHAD_P_RAINN], c->field[ATHAD_P_RAIN],
-                                     2 * c->L.field_elems * sizeof(double), cudaMemcpyDeviceToDevice,
-                                     b->stream), "batch precipitation level n");
-        if (s != ATHAD_OK) return s;
-    }
     batch_advance_kernel<<<(n + 127) / 128, 128, 0, b->stream>>>(b->d_step, n);
     return bcuda(b, cudaGetLastError(), "batch advance");
 }
@@ -198,85 +222,37 @@ athad_status athad_batch_create(athad_ctx* const* members, int32_t n_members, co
     b->iter.resize(n_members);
     b->active.assign(n_members, 1);
     for (int q = 0; q < n_members; q++) b->iter[q] = first_iter ? first_iter[q] : 1;
-    b->step = *step;
     const int n = n_members;
-    b->n_shapes = std::min(batch_shape_count(), kMaxShapes);
 
-    // host tables
-    std::vector<RK4MArgs> args(n);
+    b->args.resize(n);
     std::vector<BatchStep> steps(n);
-    std::vector<LevelMeanMember> lm(n);
-    std::vector<int> tiles((size_t)b->n_shapes * (n + 1));
-    int level0 = 0;
     for (int q = 0; q < n; q++) {
         athad_ctx* c = members[q];
-        athad_step_scalars sc{step->dt, step->diffusion_ramp, 1.0, 0, 0};
-        mixed_args(c, &sc, args[q]);
-        for (int f = 0; f < kMixedGroups; f++) {
-            args[q].Yout[f] = c->mA[f];      // stage buffer A
-            args[q].Ybnd[f] = c->mB[f];      // stage buffer B
-        }
-        for (int f = 0; f < kNY; f++) args[q].Yn_store[f] = c->field[ATHAD_TN + f];
-        args[q].store_n = 1;
+        RK4MArgs& a = b->args[q];
+        // the time-level copy fused; the buoyancy ramp of the scalars is not used (MEMBER kernels)
+        const athad_step_scalars sc{step->dt, step->diffusion_ramp, 1.0, 0, 1};
+        mixed_args(c, &sc, a);
+        for (int f = 0; f < kMixedGroups; f++) a.Ybnd[f] = c->mB[f];
         BatchStep& s = steps[q];
         std::memset(&s, 0, sizeof s);
-        s.half_dt_f = (float)(0.5 * step->dt);
-        s.dt_f = (float)step->dt;
-        s.diffusion_ramp = (float)step->diffusion_ramp;
-        s.drag_pref = args[q].drag_pref;
-        s.half_dt = 0.5 * step->dt;
-        s.dt_sixth = step->dt / 6.0;
         s.g = c->p.g; s.dt = step->dt; s.u_0 = c->p.u_0;
         s.iter = b->iter[q];
         s.ramp_iters = step->buoyancy_ramp_iters;
-        s.write_diag = 0;
         s.active = 1;
-        lm[q].d = c->L.d;
-        lm[q].t = c->field[ATHAD_T];
-        lm[q].sin_w = c->sin_w;
-        lm[q].out = c->prof[ATHAD_PROF_T_REF_LEVEL];
-        lm[q].level0 = level0;
-        level0 += c->L.d.im;
-        b->max_jm = std::max(b->max_jm, c->L.d.jm);
+        s.buoy_pref = batch_buoyancy(s);
     }
-    b->total_levels = level0;
-    for (int sh = 0; sh < b->n_shapes; sh++) {
-        const BatchShape S = batch_shape_info(sh);
-        int acc = 0;
-        for (int q = 0; q < n; q++) {
-            tiles[(size_t)sh * (n + 1) + q] = acc;
-            const Dims& d = members[q]->L.d;
-            acc += d.im * ((d.jm + S.by - 1) / S.by) * ((d.km + S.bx - 1) / S.bx);
-        }
-        tiles[(size_t)sh * (n + 1) + n] = acc;
-        b->total_tiles[sh] = acc;
-        b->grid[sh] = batch_shape_grid(sh);
-    }
-    b->shape = 0;
 
-    // device tables
-    const size_t a_bytes = round_up(sizeof(RK4MArgs) * n, 256);
-    const size_t s_bytes = round_up(sizeof(BatchStep) * n, 256);
-    const size_t t_bytes = round_up(sizeof(int) * tiles.size(), 256);
-    const size_t l_bytes = round_up(sizeof(LevelMeanMember) * n, 256);
     athad_status st = ATHAD_OK;
     if (cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking) != cudaSuccess) {
         cudaGetLastError(); delete b; return ATHAD_ERR_CUDA;
     }
     b->stream = b->own_stream;
-    if (cudaMalloc((void**)&b->dev, a_bytes + s_bytes + t_bytes + l_bytes) != cudaSuccess) {
+    if (cudaMalloc((void**)&b->d_step, sizeof(BatchStep) * n) != cudaSuccess) {
         cudaGetLastError(); cudaStreamDestroy(b->own_stream); delete b; return ATHAD_ERR_OOM;
     }
-    b->d_args = (RK4MArgs*)b->dev;
-    b->d_step = (BatchStep*)(b->dev + a_bytes);
-    b->d_tiles = (int*)(b->dev + a_bytes + s_bytes);
-    b->d_lm = (LevelMeanMember*)(b->dev + a_bytes + s_bytes + t_bytes);
-    st = bcuda(b, cudaMemcpyAsync(b->d_args, args.data(), sizeof(RK4MArgs) * n, cudaMemcpyHostToDevice, b->stream), "args");
-    if (st == ATHAD_OK) st = bcuda(b, cudaMemcpyAsync(b->d_step, steps.data(), sizeof(BatchStep) * n, cudaMemcpyHostToDevice, b->stream), "steps");
-    if (st == ATHAD_OK) st = bcuda(b, cudaMemcpyAsync(b->d_tiles, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice, b->stream), "tiles");
-    if (st == ATHAD_OK) st = bcuda(b, cudaMemcpyAsync(b->d_lm, lm.data(), sizeof(LevelMeanMember) * n, cudaMemcpyHostToDevice, b->stream), "levels");
+    st = bcuda(b, cudaMemcpyAsync(b->d_step, steps.data(), sizeof(BatchStep) * n, cudaMemcpyHostToDevice, b->stream), "steps");
     if (st == ATHAD_OK) st = bcuda(b, cudaStreamSynchronize(b->stream), "batch create sync");
-    // the side streams and events of the column-physics fork/join
+    // the side streams and events of the lanes' fork/join
     if (st == ATHAD_OK) st = bcuda(b, cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "batch events");
     const int ns = std::min(n, kSideStreams);
     for (int q = 0; q < ns && st == ATHAD_OK; q++) {
@@ -291,7 +267,7 @@ athad_status athad_batch_create(athad_ctx* const* members, int32_t n_members, co
         for (cudaStream_t s : b->side) cudaStreamDestroy(s);
         for (cudaEvent_t e : b->join) cudaEventDestroy(e);
         if (b->fork) cudaEventDestroy(b->fork);
-        cudaFree(b->dev); cudaStreamDestroy(b->own_stream); delete b;
+        cudaFree(b->d_step); cudaStreamDestroy(b->own_stream); delete b;
         return st;
     }
     *out = b;
@@ -306,7 +282,7 @@ athad_status athad_batch_destroy(athad_batch* b)
     for (cudaStream_t s : b->side) { cudaStreamSynchronize(s); cudaStreamDestroy(s); }
     for (cudaEvent_t e : b->join) cudaEventDestroy(e);
     if (b->fork) cudaEventDestroy(b->fork);
-    cudaFree(b->dev);
+    cudaFree(b->d_step);
     cudaStreamDestroy(b->own_stream);
     delete b;
     return ATHAD_OK;
@@ -388,7 +364,7 @@ int32_t athad_batch_shape_count(void) { return batch_shape_count(); }
 
 athad_status athad_batch_set_shape(athad_batch* b, int32_t shape)
 {
-    if (!b || shape < 0 || shape >= b->n_shapes) return ATHAD_ERR_INVALID;
+    if (!b || shape < 0 || shape >= batch_shape_count()) return ATHAD_ERR_INVALID;
     if (shape != b->shape) drop_graphs(b);
     b->shape = shape;
     return ATHAD_OK;
@@ -397,7 +373,6 @@ athad_status athad_batch_set_shape(athad_batch* b, int32_t shape)
 athad_status athad_batch_autotune(athad_batch* b, int32_t reps, int32_t* best_shape, float* ms_per_shape)
 {
     if (!b || reps < 1) return ATHAD_ERR_INVALID;
-    const int n = (int)b->m.size();
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
         cudaGetLastError(); return bfail(b, ATHAD_ERR_CUDA, "autotune events");
@@ -405,19 +380,21 @@ athad_status athad_batch_autotune(athad_batch* b, int32_t reps, int32_t* best_sh
     float best = 3.4e38f;
     int best_id = b->shape;
     athad_status s = ATHAD_OK;
-    for (int sh = 0; sh < b->n_shapes && s == ATHAD_OK; sh++) {
-        BatchTables T;
-        T.args = b->d_args; T.step = b->d_step;
-        T.tile_start = b->d_tiles + (size_t)sh * (n + 1);
-        T.n = n; T.total_tiles = b->total_tiles[sh];
+    for (int sh = 0; sh < batch_shape_count() && s == ATHAD_OK; sh++) {
         // stages 1-3 write only the members' private FP32 buffers, which the next
         // iteration's stage 1 rewrites, so timing them leaves the model state unchanged
-        for (int stage = 1; stage <= 3; stage++) launch_rk4m_batch_stage(stage, sh, T, b->grid[sh], b->stream);
+        auto stages = [b, sh] {
+            return on_lanes(b, [b, sh](int q) {
+                athad_status r = ATHAD_OK;
+                for (int stage = 1; stage <= 3 && r == ATHAD_OK; stage++) r = enqueue_stage(b, q, stage, sh);
+                return r;
+            });
+        };
+        s = stages();
         cudaEventRecord(e0, b->stream);
-        for (int r = 0; r < reps; r++)
-            for (int stage = 1; stage <= 3; stage++) launch_rk4m_batch_stage(stage, sh, T, b->grid[sh], b->stream);
+        for (int r = 0; r < reps && s == ATHAD_OK; r++) s = stages();
         cudaEventRecord(e1, b->stream);
-        s = bcuda(b, cudaEventSynchronize(e1), "autotune");
+        if (s == ATHAD_OK) s = bcuda(b, cudaEventSynchronize(e1), "autotune");
         float ms = 0.0f;
         if (s == ATHAD_OK) s = bcuda(b, cudaEventElapsedTime(&ms, e0, e1), "autotune time");
         ms /= (float)reps;

@@ -68,7 +68,7 @@ ATHAD_HD long long idx3(const Dims& d, int i, int j, int k)
 // completed and its writes are visible, so stream order holds for every access.  The
 // kernel before it calls pdl_trigger() to let the dependent's CTAs onto the SMs its last
 // wave frees instead of after its completion.  Both are no-ops in a kernel launched
-// without the attribute (the batched RK4 kernels, the kernels shared with other paths).
+// without the attribute (the kernels shared with other paths).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -213,13 +213,16 @@ __device__ __forceinline__ void prefetch_tile(const RK4MArgs& a, int i, int j0, 
     }
 }
 
-// One cell of one stage.  Shared by the single-grid kernel and the batched persistent
-// kernel (k_batch.cu), which reads each member's arguments from shared memory.
+// One cell of one stage.
 template <int STAGE>
-__device__ __forceinline__ void rk4m_cell(const RK4MArgs& a, int i, int j, int k)
+__device__ __forceinline__ void rk4m_cell(const RK4MArgs& a, int i, int j, int k, float buoy_pref)
 {
     const Dims& d = a.d;
     const long long c = idx3(d, i, j, k);
+    if (STAGE == 4 && a.store_n) {   // the copy's precipitation fluxes (UtilsAtm.h:41-42)
+        a.rain_n[c] = __ldg(a.rain + c);
+        a.rain_n[c + d.fstride] = __ldg(a.rain + c + d.fstride);
+    }
     const bool interior = (i > 0 && i < d.im - 1 && j > 0 && j < d.jm - 1 && k > 0 && k < d.km - 1);
     if (!interior) {
         if (STAGE == 1) {   // boundary values into both stage buffers; p_dyn for the stencil
@@ -320,7 +323,7 @@ __device__ __forceinline__ void rk4m_cell(const RK4MArgs& a, int i, int j, int k
             const float t_ijk = y1.z;
             const float coriolis_rad = nontrad * 2.0f * sinthe * w_ijk;
             const float rhs_u = -dpdr_exp - tr_u + diffusion_u
-                + a.buoy_pref * (t_ijk - (float)__ldg(a.t_ref + i))
+                + buoy_pref * (t_ijk - (float)__ldg(a.t_ref + i))
                 + a.force_nd * coriolis_rad;
             k0[0] = rhs_u;
             if (STAGE == 4) a.aux_u[c] = (double)rhs_u + (double)dpdr_exp;
@@ -523,18 +526,14 @@ __device__ __forceinline__ void rk4m_cell(const RK4MArgs& a, int i, int j, int k
 #define ATHAD_RK4M_MIN_BLOCKS_S4 6
 #endif
 
-#ifndef ATHAD_RK4M_BX
-#define ATHAD_RK4M_BX 128        // CTA: BX longitudes x BY rows of one level; 41x181x361: 128 x 1
-#endif                           // 785 us, 64 x 2 804, 32 x 4 832, 64 x 4 857, 32 x 8 901
-#ifndef ATHAD_RK4M_BY
-#define ATHAD_RK4M_BY 1
-#endif
-
-template <int STAGE>
-__global__ void __launch_bounds__(ATHAD_RK4M_BX * ATHAD_RK4M_BY,
-    (STAGE == 1 ? ATHAD_RK4M_MIN_BLOCKS_S1 : STAGE == 4 ? ATHAD_RK4M_MIN_BLOCKS_S4 : ATHAD_RK4M_MIN_BLOCKS)
-    * 128 / (ATHAD_RK4M_BX * ATHAD_RK4M_BY))
-rk4m_stage_kernel(const RK4MArgs a)
+// MEMBER: a batch's member on a lane of its own; its buoyancy prefactor changes from
+// iteration to iteration of a captured graph, so it is read from the member's step record.
+// BX longitudes x BY rows of one level per CTA: 128 x 1 for a single grid (41x181x361: 785 us,
+// 64 x 2 804, 32 x 4 832, 32 x 8 901).
+template <int STAGE, int BX, int BY, bool MEMBER>
+__global__ void __launch_bounds__(BX * BY,
+    (STAGE == 1 ? ATHAD_RK4M_MIN_BLOCKS_S1 : STAGE == 4 ? ATHAD_RK4M_MIN_BLOCKS_S4 : ATHAD_RK4M_MIN_BLOCKS) * 128 / (BX * BY))
+rk4m_stage_kernel(const RK4MArgs a, const BatchStep* step)
 {
     pdl_trigger();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -548,202 +547,42 @@ rk4m_stage_kernel(const RK4MArgs a)
 #else
     const int i = blockIdx.z;
 #endif
-    prefetch_tile<STAGE>(a, i, blockIdx.y * ATHAD_RK4M_BY, blockIdx.x * ATHAD_RK4M_BX, ATHAD_RK4M_BX, ATHAD_RK4M_BY,
-                         threadIdx.y * ATHAD_RK4M_BX + threadIdx.x, ATHAD_RK4M_BX * ATHAD_RK4M_BY);
+    prefetch_tile<STAGE>(a, i, blockIdx.y * BY, blockIdx.x * BX, BX, BY, threadIdx.y * BX + threadIdx.x, BX * BY);
     if (k >= a.d.km || j >= a.d.jm) return;
-    rk4m_cell<STAGE>(a, i, j, k);
+    rk4m_cell<STAGE>(a, i, j, k, MEMBER ? step->buoy_pref : a.buoy_pref);
+}
+
+template <int BX, int BY, bool MEMBER>
+static void launch_stage(int stage, const RK4MArgs& a, const BatchStep* step, cudaStream_t st)
+{
+    const dim3 block(BX, BY, 1);
+    const dim3 grid((a.d.km + BX - 1) / BX, (a.d.jm + BY - 1) / BY, a.d.im);
+    switch (stage) {
+        case 1: launch_dependent(rk4m_stage_kernel<1, BX, BY, MEMBER>, grid, block, 0, st, a, step); break;
+        case 2: launch_dependent(rk4m_stage_kernel<2, BX, BY, MEMBER>, grid, block, 0, st, a, step); break;
+        case 3: launch_dependent(rk4m_stage_kernel<3, BX, BY, MEMBER>, grid, block, 0, st, a, step); break;
+        default: launch_dependent(rk4m_stage_kernel<4, BX, BY, MEMBER>, grid, block, 0, st, a, step); break;
+    }
 }
 
 void launch_rk4m_stage(int stage, const RK4MArgs& a, cudaStream_t st)
 {
-    const dim3 block(ATHAD_RK4M_BX, ATHAD_RK4M_BY, 1);
-    const dim3 grid((a.d.km + ATHAD_RK4M_BX - 1) / ATHAD_RK4M_BX, (a.d.jm + ATHAD_RK4M_BY - 1) / ATHAD_RK4M_BY, a.d.im);
-    switch (stage) {
-        case 1: launch_dependent(rk4m_stage_kernel<1>, grid, block, 0, st, a); break;
-        case 2: launch_dependent(rk4m_stage_kernel<2>, grid, block, 0, st, a); break;
-        case 3: launch_dependent(rk4m_stage_kernel<3>, grid, block, 0, st, a); break;
-        default: launch_dependent(rk4m_stage_kernel<4>, grid, block, 0, st, a); break;
-    }
+    launch_stage<128, 1, false>(stage, a, nullptr, st);
 }
 
-
-// ---------------------------------------------------------------------------------------
-// Batched form: the members of an ensemble advance together, one persistent launch per
-// stage.  The tiles of all members (BX longitudes x BY rows of one level) are numbered
-// member after member; CTA b takes the contiguous range [b*per, (b+1)*per), so it changes
-// member at most a few times.  On a change it copies that member's arguments into shared
-// memory, sets the stage buffers of this stage and the member's step scalars, and runs the
-// same per-cell code as the single-grid kernel.
-template <int STAGE>
-__device__ __forceinline__ void load_member_args(RK4MArgs& sa, const BatchTables& T, int m)
-{
-    const long long* src = reinterpret_cast<const long long*>(T.args + m);
-    long long* dst = reinterpret_cast<long long*>(&sa);
-    const int nthreads = blockDim.x * blockDim.y;
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    __syncthreads();   // every warp is done with the previous member's arguments
-    for (int w = tid; w < (int)(sizeof(RK4MArgs) / sizeof(long long)); w += nthreads) dst[w] = src[w];
-    __syncthreads();
-    if (tid < 3) {   // the table holds buffer A in Yout and buffer B in Ybnd
-        float4* A = sa.Yout[tid];
-        float4* B = sa.Ybnd[tid];
-        sa.Yin[tid] = (STAGE == 3) ? B : A;
-        sa.Yout[tid] = (STAGE == 1 || STAGE == 3) ? A : B;
-        sa.Ybnd[tid] = B;
-    } else if (tid == 32) {
-        const BatchStep& st = T.step[m];
-        sa.half_dt_f = st.half_dt_f; sa.dt_f = st.dt_f; sa.diffusion_ramp = st.diffusion_ramp;
-        sa.drag_pref = st.drag_pref;
-        const double x = (double)st.iter / (double)st.ramp_iters;
-        const double ramp = (x < 1.0) ? x : 1.0;
-        sa.buoy_pref = (float)(ramp * st.g * st.dt / st.u_0);
-        sa.half_dt = st.half_dt; sa.dt_sixth = st.dt_sixth; sa.write_diag = st.write_diag;
-    }
-    __syncthreads();
-}
-
-template <int STAGE, int BX, int BY, int MINB>
-__global__ void __launch_bounds__(BX * BY, MINB) rk4m_batch_kernel(const BatchTables T)
-{
-    __shared__ __align__(16) RK4MArgs sa;
-    const int per = (T.total_tiles + gridDim.x - 1) / gridDim.x;
-    const int t0 = blockIdx.x * per;
-    const int t1 = min(T.total_tiles, t0 + per);
-    if (t0 >= t1) return;
-    // member owning tile t0: the last m with tile_start[m] <= t0 (binary search, uniform)
-    int lo = 0, hi = T.n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(T.tile_start + mid) <= t0) lo = mid; else hi = mid - 1;
-    }
-    int m = lo;
-    load_member_args<STAGE>(sa, T, m);
-    int tstart = __ldg(T.tile_start + m), tend = __ldg(T.tile_start + m + 1);
-    int active = __ldg(&T.step[m].active);
-    int nkx = (sa.d.km + BX - 1) / BX, nkj = nkx * ((sa.d.jm + BY - 1) / BY);
-    for (int t = t0; t < t1; t++) {
-        if (t >= tend) {
-            while (__ldg(T.tile_start + m + 1) <= t) m++;
-            load_member_args<STAGE>(sa, T, m);
-            tstart = __ldg(T.tile_start + m); tend = __ldg(T.tile_start + m + 1);
-            active = __ldg(&T.step[m].active);
-            nkx = (sa.d.km + BX - 1) / BX; nkj = nkx * ((sa.d.jm + BY - 1) / BY);
-        }
-        if (!active) continue;
-        const int local = t - tstart;
-        const int i = local / nkj;
-        const int rem = local - i * nkj;
-        const int jt = rem / nkx;
-        const int k = (rem - jt * nkx) * BX + threadIdx.x;
-        const int j = jt * BY + threadIdx.y;
-        if (k < sa.d.km && j < sa.d.jm) rk4m_cell<STAGE>(sa, i, j, k);
-    }
-}
-
-// Tile shapes the autotuner chooses from: (longitudes, rows, CTAs per SM the register
-// budget is sized for).  A CTA walks its tiles in a row, so rows of one tile share their
-// neighbours in L1: stages 1-3 of six members of 3.4 M cells take 1.93 ms with 32 x 4 at 5
-// CTAs, 1.98 at 6, 2.10 at 7, 2.33 with 128 x 1 at 6, 1.99 with 32 x 8.  The tiles are not
-// prefetched into L2 as the single grid's are: 2.24 ms with prefetch_tile.
-#define ATHAD_BATCH_SHAPES(X) X(0, 32, 4, 5) X(1, 32, 4, 6) X(2, 64, 2, 5) X(3, 32, 8, 3) X(4, 128, 1, 6) \
-    X(5, 32, 4, 4)
-
-template <int BX, int BY, int MINB>
-static void launch_batch_shape(int stage, const BatchTables& T, int grid, cudaStream_t st)
-{
-    const dim3 block(BX, BY, 1);
-    switch (stage) {
-        case 1: rk4m_batch_kernel<1, BX, BY, MINB><<<grid, block, 0, st>>>(T); break;
-        case 2: rk4m_batch_kernel<2, BX, BY, MINB><<<grid, block, 0, st>>>(T); break;
-        case 3: rk4m_batch_kernel<3, BX, BY, MINB><<<grid, block, 0, st>>>(T); break;
-        default: rk4m_batch_kernel<4, BX, BY, MINB><<<grid, block, 0, st>>>(T); break;
-    }
-}
-
-template <int BX, int BY, int MINB>
-static int batch_shape_grid()
-{
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rk4m_batch_kernel<2, BX, BY, MINB>, BX * BY, 0);
-    if (per_sm < 1) per_sm = 1;
-    return sms * per_sm;
-}
-
+// The tile shapes a batch's autotuner chooses from.
 int batch_shape_count() { return 6; }
 
-BatchShape batch_shape_info(int shape)
+void launch_rk4m_member_stage(int stage, int shape, const RK4MArgs& a, const BatchStep* step, cudaStream_t st)
 {
-    BatchShape r{0, 0, 0};
-#define ATHAD_SHAPE_INFO(ID, BX, BY, MINB) if (shape == ID) { r.bx = BX; r.by = BY; r.min_blocks = MINB; }
-    ATHAD_BATCH_SHAPES(ATHAD_SHAPE_INFO)
-#undef ATHAD_SHAPE_INFO
-    return r;
-}
-
-int batch_shape_grid(int shape)
-{
-#define ATHAD_SHAPE_GRID(ID, BX, BY, MINB) if (shape == ID) return batch_shape_grid<BX, BY, MINB>();
-    ATHAD_BATCH_SHAPES(ATHAD_SHAPE_GRID)
-#undef ATHAD_SHAPE_GRID
-    return 0;
-}
-
-void launch_rk4m_batch_stage(int stage, int shape, const BatchTables& T, int grid, cudaStream_t st)
-{
-#define ATHAD_SHAPE_LAUNCH(ID, BX, BY, MINB) if (shape == ID) { launch_batch_shape<BX, BY, MINB>(stage, T, grid, st); return; }
-    ATHAD_BATCH_SHAPES(ATHAD_SHAPE_LAUNCH)
-#undef ATHAD_SHAPE_LAUNCH
-}
-
-// computeLevelMeanTemperature of every member in one launch: one CTA per (member, level),
-// the same row sums and mirror pairing as level_mean_kernel.
-__global__ void __launch_bounds__(256) batch_level_mean_kernel(const LevelMeanMember* __restrict__ M, int n,
-                                                               const BatchStep* __restrict__ step)
-{
-    extern __shared__ double rows[];
-    const int g = blockIdx.x;
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (M[mid].level0 <= g) lo = mid; else hi = mid - 1;
+    switch (shape) {
+        case 0: launch_stage<128, 1, true>(stage, a, step, st); break;
+        case 1: launch_stage<64, 2, true>(stage, a, step, st); break;
+        case 2: launch_stage<32, 4, true>(stage, a, step, st); break;
+        case 3: launch_stage<32, 8, true>(stage, a, step, st); break;
+        case 4: launch_stage<64, 4, true>(stage, a, step, st); break;
+        default: launch_stage<128, 2, true>(stage, a, step, st); break;
     }
-    const LevelMeanMember& mm = M[lo];
-    if (!step[lo].active) return;
-    const Dims d = mm.d;
-    const int i = g - mm.level0;
-    if (i >= d.im) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int j = warp; j < d.jm; j += nwarp) {
-        const double* row = mm.t + idx3(d, i, j, 0);
-        double s = 0.0;
-        for (int k = lane; k < d.km; k += 32) s += __ldg(row + k);
-        for (int off = 16; off >= 1; off >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, off);
-        if (lane == 0) rows[j] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        // explicit roundings: this file compiles with fused multiply-add, the single-grid
-        // level mean without, and both must give the same bits
-        double sum = 0.0, wsum = 0.0;
-        const int half = d.jm / 2;
-        for (int j = 0; j < half; j++) {
-            sum = __dadd_rn(sum, __dmul_rn(mm.sin_w[j], __dadd_rn(rows[j], rows[d.jm - 1 - j])));
-            wsum = __dadd_rn(wsum, __dmul_rn(__dmul_rn(2.0, mm.sin_w[j]), (double)d.km));
-        }
-        if (d.jm & 1) {
-            sum = __dadd_rn(sum, __dmul_rn(mm.sin_w[half], rows[half]));
-            wsum = __dadd_rn(wsum, __dmul_rn(mm.sin_w[half], (double)d.km));
-        }
-        mm.out[i] = (wsum > 0.0) ? sum / wsum : 1.0;
-    }
-}
-
-void launch_batch_level_mean(const LevelMeanMember* M, int n, int total_levels, int max_jm,
-                             const BatchStep* step, cudaStream_t st)
-{
-    batch_level_mean_kernel<<<total_levels, 256, sizeof(double) * max_jm, st>>>(M, n, step);
 }
 
 }  // namespace athad

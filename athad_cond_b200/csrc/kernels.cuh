@@ -103,7 +103,8 @@ struct RK4MArgs {
     float4* Yn32[kMixedGroups];        // FP32 time level n (written by stage 1, read by 2-3)
     float4* K[kMixedGroups];           // FP32 accumulator
     float4* F[kMixedForcing];          // packed forcing: (MC_w, q_t, k_T, t_eq), (q_c, q_cloud, q_ice, q_gr)
-    double* Yn_store[11];       // store_n: stage 4 also writes the new time level n here
+    double* Yn_store[11];       // store_n: stage 4 also writes the new time level n here,
+    const double* rain; double* rain_n;   // and copies rain and, one fstride on, snow
     double* aux_u; double* aux_v; double* aux_w;
     double* prod; double* tke_source; double* dis_source;
     float inv_2dr, inv_2dthe, inv_2dphi, inv_dr, inv_dthe, inv_dphi, inv_dr2, inv_dthe2, inv_dphi2;
@@ -115,34 +116,19 @@ struct RK4MArgs {
 };
 void launch_rk4m_stage(int stage, const RK4MArgs& a, cudaStream_t st);
 
-// Batched mixed-precision step (k_rk4m.cu): per-member step scalars, the device tables the
-// persistent stage kernel reads, and the batched level mean.
+// A batch member's step record on the device (batch.cu): the scalars that change from
+// iteration to iteration of a captured graph.
 struct BatchStep {
-    float half_dt_f, dt_f, diffusion_ramp, drag_pref;
-    double half_dt, dt_sixth;
-    double g, dt, u_0;         // buoyancy prefactor ramp * g * dt / u_0, formed per stage
+    double g, dt, u_0;         // buoyancy prefactor ramp * g * dt / u_0
+    float buoy_pref;           // of iteration iter
     int iter;                  // the member's current iteration number (1-based)
     int ramp_iters;            // buoyancy ramp = min(1, iter / ramp_iters)
-    int write_diag, active;
+    int active;
 };
-struct BatchTables {
-    const RK4MArgs* args;      // [n] per member; stage buffer A in Yout, B in Ybnd
-    const BatchStep* step;     // [n]
-    const int* tile_start;     // [n+1] first tile of each member (for the launch's shape)
-    int n, total_tiles;
-};
-struct BatchShape { int bx, by, min_blocks; };
+// launch_rk4m_stage with the buoyancy prefactor from the member's step record, in one of the
+// tile shapes 0 .. batch_shape_count() - 1
 int batch_shape_count();
-BatchShape batch_shape_info(int shape);
-int batch_shape_grid(int shape);   // persistent grid: SMs x resident CTAs of that shape
-void launch_rk4m_batch_stage(int stage, int shape, const BatchTables& T, int grid, cudaStream_t st);
-struct LevelMeanMember {
-    Dims d;
-    const double* t; const double* sin_w; double* out;
-    int level0;                // first global level index of this member
-};
-void launch_batch_level_mean(const LevelMeanMember* M, int n, int total_levels, int max_jm,
-                             const BatchStep* step, cudaStream_t st);
+void launch_rk4m_member_stage(int stage, int shape, const RK4MArgs& a, const BatchStep* step, cudaStream_t st);
 
 // Per-(i,j) coefficients of the 7-point Poisson operator, PressureSolverAtm.h:236-269,
 // computed on the host once per context.

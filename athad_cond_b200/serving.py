@@ -4,8 +4,8 @@ time, advanced together on one GPU by continuous batching.
 A request is one run: a grid, a condition point (ensemble.draw_condition) and a number of
 model iterations.  The server keeps every admitted run's state resident on the device (one
 mixed-precision GpuAtmosphere each) and advances all of them by one iteration per step
-through one GpuBatch: each run's column physics at its own cadence, the RK4 stages of all
-runs in one persistent launch per stage.  Between steps it
+through one GpuBatch: each run's column physics at its own cadence and its RK4 stages, the
+runs side by side.  Between steps it
   * retires runs that have done their iterations (download of the requested fields, the
     context's memory freed),
   * admits waiting requests in arrival order while a slot is free and the run's device

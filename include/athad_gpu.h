@@ -584,10 +584,10 @@ athad_status athad_get_report(athad_ctx* ctx, athad_report* out);
 
 /* ---- ensembles: batched iteration of many contexts ----------------------------
  * No counterpart in the reference, which runs one grid per process.  A batch advances
- * mixed-precision contexts (members, each with its own grid and parameters) together on
- * one stream: every member's column physics at its own cadence, the level mean of all
- * members in one launch, each RK4 stage of all members in one persistent launch, the
- * time-level copy (storeIntermediateData3D) fused into the last stage.  The members stay
+ * mixed-precision contexts (members, each with its own grid and parameters) together in the
+ * order of one stream: every member's column physics at its own cadence, level mean and RK4
+ * stages, the time-level copy (storeIntermediateData3D) fused into the last, side by side
+ * on streams of the batch that fork from that stream and join it again.  The members stay
  * ordinary contexts: upload/download work on them between batch calls (on the batch's
  * stream order: call athad_batch_synchronize first).  A member's result is bit-for-bit
  * the result of the same iterations run on it alone through athad_rk4_step and friends
@@ -621,7 +621,7 @@ athad_status athad_batch_iteration(athad_batch* b);
 /* The same iteration replayed from a CUDA graph, captured on first use for the current
  * cadence pattern of the members (at most a few per batch). */
 athad_status athad_batch_iteration_graph(athad_batch* b);
-/* Tile shapes of the persistent RK4 kernel; athad_batch_autotune times RK4 stages 1-3 of
+/* Tile shapes of the members' RK4 stage kernels; athad_batch_autotune times RK4 stages 1-3 of
  * the whole batch once per shape (reps repetitions, model state unchanged), keeps the
  * fastest and reports each shape's milliseconds per stage triple. */
 int32_t      athad_batch_shape_count(void);
