@@ -232,6 +232,7 @@ SIGNATURES = {
     "athad_boundary_conditions": (ctypes.c_int, [_P]),
     "athad_post_rk4_filters": (ctypes.c_int, [_P]),
     "athad_damp_wiggles": (ctypes.c_int, [_P, ctypes.c_int]),
+    "athad_damp_wiggles_of": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int), ctypes.c_int32]),
     "athad_turbulence_run": (ctypes.c_int, [_P]),
     "athad_two_cat_ice_scheme": (ctypes.c_int, [_P]),
     "athad_zero_cat_ice_scheme": (ctypes.c_int, [_P]),

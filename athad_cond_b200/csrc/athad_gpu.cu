@@ -911,11 +911,35 @@ athad_status athad_post_rk4_filters(athad_ctx* ctx)
 
 athad_status athad_damp_wiggles(athad_ctx* ctx, athad_field f)
 {
-    if (!ctx || (int)f < 0 || (int)f >= ATHAD_NFIELDS) return fail(ctx, ATHAD_ERR_INVALID, "damp_wiggles: bad argument");
+    return athad_damp_wiggles_of(ctx, &f, 1);
+}
+
+athad_status athad_damp_wiggles_of(athad_ctx* ctx, const athad_field* fields, int32_t n)
+{
+    if (!ctx || n < 0 || (n > 0 && !fields)) return fail(ctx, ATHAD_ERR_INVALID, "damp_wiggles: bad argument");
+    for (int q = 0; q < n; q++)
+        if ((int)fields[q] < 0 || (int)fields[q] >= ATHAD_NFIELDS)
+            return fail(ctx, ATHAD_ERR_INVALID, "damp_wiggles: bad argument");
     if (ctx->L.d.km > 3072) return fail(ctx, ATHAD_ERR_UNSUPPORTED, "damp_wiggles: km > 3072");
-    // the RK4 stage buffer A is free between RK4 steps
-    launch_damp_wiggles(ctx->L.d, ctx->field[f], ctx->stA[0], ctx->stream);
-    ATHAD_CHECK_LAUNCH(ctx, "damp_wiggles");
+    static_assert(kWiggleFields <= kNY, "one RK4 stage buffer per field of a launch");
+    WiggleFields w{};
+    for (int q = 0; q < n; q++) {
+        double* f = ctx->field[fields[q]];
+        bool repeated = false;
+        for (int r = 0; r < w.n; r++) repeated |= (w.f[r] == f);
+        if (w.n == kWiggleFields || repeated) {   // a field named twice is filtered twice
+            launch_damp_wiggles(ctx->L.d, w, ctx->stream);
+            ATHAD_CHECK_LAUNCH(ctx, "damp_wiggles");
+            w.n = 0;
+        }
+        w.f[w.n] = f;
+        w.scratch[w.n] = ctx->stA[w.n];   // the RK4 stage buffers A are free between RK4 steps
+        w.n += 1;
+    }
+    if (w.n > 0) {
+        launch_damp_wiggles(ctx->L.d, w, ctx->stream);
+        ATHAD_CHECK_LAUNCH(ctx, "damp_wiggles");
+    }
     return ATHAD_OK;
 }
 

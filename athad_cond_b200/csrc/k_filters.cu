@@ -85,6 +85,11 @@ __global__ void __launch_bounds__(128) radial_columns_kernel(FilterArgs a)
 // The meridional pass adds the two neighbours first, so the result at row jm-1-j is bit for
 // bit the result at row j of the mirrored field; the reference's left-to-right
 // (v[j-1] - 2 v[j]) + v[j+1] rounds the mirrored rows differently (an ulp at most).
+// The fields of one launch lie side by side in its grid: a field alone ends each launch with
+// SMs that wait for the last CTAs, and a small one does not fill the GPU.  The 23 fields of a
+// moist iteration, one at a time and up to eleven: 21x91x181 262 and 73 us, 41x181x361 483
+// and 396, 61x181x361 607 and 575.  Limiting a launch to what the L2 holds with its scratch
+// is no better (41x181x361, four fields: 417).
 constexpr int kWalk = 8;
 
 // the zonal pass (periodic) of the longitudes k, k + 1 of one row; k is even, and the second
@@ -98,13 +103,16 @@ __device__ __forceinline__ double2 zonal_two(const double* __restrict__ row, int
     return make_double2(x.x + 0.25 * (west - 2.0 * x.x + e0), x.y + 0.25 * (x.x - 2.0 * x.y + east));
 }
 
-__global__ void __launch_bounds__(128) wiggle_kj_kernel(Dims d, const double* __restrict__ src, double* __restrict__ dst)
+__global__ void __launch_bounds__(128) wiggle_kj_kernel(Dims d, const WiggleFields w)
 {
     pdl_trigger();
     int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     pdl_wait(k);
-    const int j0 = blockIdx.y * kWalk, i = blockIdx.z;
+    const int q = blockIdx.z / d.im, i = blockIdx.z - q * d.im;
+    const int j0 = blockIdx.y * kWalk;
     if (k >= d.km) return;
+    const double* __restrict__ src = w.f[q];
+    double* __restrict__ dst = w.scratch[q];
     const int jn = min(j0 + kWalk, d.jm);
     const double* plane = src + idx3(d, i, 0, 0);
     double2 c = zonal_two(plane + (long long)j0 * d.pitch, k, d.km);
@@ -118,13 +126,17 @@ __global__ void __launch_bounds__(128) wiggle_kj_kernel(Dims d, const double* __
     }
 }
 
-__global__ void __launch_bounds__(128) wiggle_i_kernel(Dims d, const double* __restrict__ src, double* __restrict__ dst)
+__global__ void __launch_bounds__(128) wiggle_i_kernel(Dims d, const WiggleFields w)
 {
     pdl_trigger();
     int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     pdl_wait(k);
-    const int j = blockIdx.y, i0 = blockIdx.z * kWalk;
+    const int nz = (d.im + kWalk - 1) / kWalk;
+    const int q = blockIdx.z / nz, i0 = (blockIdx.z - q * nz) * kWalk;
+    const int j = blockIdx.y;
     if (k >= d.km) return;
+    const double* __restrict__ src = w.scratch[q];
+    double* __restrict__ dst = w.f[q];
     const int in = min(i0 + kWalk, d.im);
     auto two = [&](int i) { return *reinterpret_cast<const double2*>(src + idx3(d, i, j, k)); };
     double2 c = two(i0), m = (i0 > 0) ? two(i0 - 1) : c;
@@ -148,13 +160,11 @@ void launch_post_rk4_filters(const FilterArgs& a, cudaStream_t st)
     radial_columns_kernel<<<dim3((d.km + 127) / 128, d.jm, 3), 128, 0, st>>>(a);
 }
 
-void launch_damp_wiggles(const Dims& d, double* f, double* scratch, cudaStream_t st)
+void launch_damp_wiggles(const Dims& d, const WiggleFields& w, cudaStream_t st)
 {
     const unsigned kx = ((d.km + 1) / 2 + 127) / 128;
-    launch_dependent(wiggle_kj_kernel, dim3(kx, (d.jm + kWalk - 1) / kWalk, d.im), dim3(128), 0, st, d, (const double*)f,
-                     scratch);
-    launch_dependent(wiggle_i_kernel, dim3(kx, d.jm, (d.im + kWalk - 1) / kWalk), dim3(128), 0, st, d,
-                     (const double*)scratch, f);
+    launch_dependent(wiggle_kj_kernel, dim3(kx, (d.jm + kWalk - 1) / kWalk, d.im * w.n), dim3(128), 0, st, d, w);
+    launch_dependent(wiggle_i_kernel, dim3(kx, d.jm, (d.im + kWalk - 1) / kWalk * w.n), dim3(128), 0, st, d, w);
 }
 
 }  // namespace athad

@@ -220,7 +220,12 @@ struct FilterArgs {
     const int* polar_passes;    // [jm] zonal passes per row
 };
 void launch_post_rk4_filters(const FilterArgs& a, cudaStream_t st);
-void launch_damp_wiggles(const Dims& d, double* f, double* scratch, cudaStream_t st);
+constexpr int kWiggleFields = 11;
+struct WiggleFields {
+    double* f[kWiggleFields]; double* scratch[kWiggleFields];
+    int n;
+};
+void launch_damp_wiggles(const Dims& d, const WiggleFields& w, cudaStream_t st);
 void launch_repitch(const Dims& d, const double* packed, double* dst, cudaStream_t st);
 
 // TurbulenceAtm::run (k_turb.cu).  Per-level constants built on the host as the reference

@@ -82,14 +82,11 @@ class ModelLoop:
         if it % 2 == 0:
             out["h2o_post_rk4"] = g.water_budget()
             g.SaturationAdjustment_run()
-            for n in MOIST_FIELDS_AFTER_SATADJ:
-                g.damp_wiggles(n)
+            g.damp_wiggles_of(MOIST_FIELDS_AFTER_SATADJ)
             g.ice_scheme()
-            for n in ICE_FLUXES:
-                g.damp_wiggles(n)
+            g.damp_wiggles_of(ICE_FLUXES)
             g.MoistConvection_run(it)
-            for n in CONVECTION_FIELDS:
-                g.damp_wiggles(n)
+            g.damp_wiggles_of(CONVECTION_FIELDS)
             g.moist_caps()
             g.vapour_ceiling()
             out["co2"] = g.co2_column()
@@ -100,8 +97,7 @@ class ModelLoop:
             g.water_vapour_evaporation()
             g.latent_sensible_heat()
             g.turbulence_run()
-            for n in TURBULENCE_FIELDS:
-                g.damp_wiggles(n)
+            g.damp_wiggles_of(TURBULENCE_FIELDS)
         g.boundary_conditions()
         ramp = min(1.0, self.total_iter_count / self.ramp_iters) if self.ramp_iters > 0 else 1.0
         budget = 2 if (self.checkpoint > 0 and it % self.checkpoint == 0) else 0

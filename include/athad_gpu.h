@@ -435,6 +435,8 @@ athad_status athad_post_rk4_filters(athad_ctx* ctx);
  * 429-531: what the moist iteration applies to t, ice, c and cloud after the saturation
  * adjustment (cAtmosphereModel.cpp:1225-1228).  Uses the RK4 stage buffers as scratch. */
 athad_status athad_damp_wiggles(athad_ctx* ctx, athad_field field);
+/* The same on each of n fields, in fewer launches than n calls. */
+athad_status athad_damp_wiggles_of(athad_ctx* ctx, const athad_field* fields, int32_t n);
 /* TurbulenceAtm(*this).run() (TurbulenceAtm.h:62-79; call sites cAtmosphereModel.cpp:614, 1426),
  * flat terrain: compute_vel_star into ATHAD_2D_VEL_STAR, compute_sources with the
  * configured closure (prod, nue, tke_source, dis_source; the floors of tke and dis) and

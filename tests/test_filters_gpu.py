@@ -80,3 +80,19 @@ def test_damp_wiggles_edges(grid):
         g.damp_wiggles("c")
         for n in ("t", "c"):
             assert np.array_equal(g.download(n), o.f[n], equal_nan=True), n
+
+
+@pytest.mark.parametrize("grid", [(4, 5, 5), (9, 17, 131)])
+def test_damp_wiggles_of_many_fields_equals_one_at_a_time(grid):
+    """More fields than one launch takes, one of them named twice: bit for bit the calls in turn."""
+    names = ["t", "ice", "c", "cloud", "u", "v", "w", "t", "gr", "co2", "tke", "dis", "p_stat", "r_humid", "nue"]
+    st = rough(grid, 59)
+    with GpuAtmosphere(*grid, config_params()) as one, GpuAtmosphere(*grid, config_params()) as many:
+        for g in (one, many):
+            g.upload_state(st)
+        for n in names:
+            one.damp_wiggles(n)
+        many.damp_wiggles_of(names)
+        many.damp_wiggles_of([])
+        for n in names:
+            assert np.array_equal(many.download(n), one.download(n)), n
