@@ -96,3 +96,18 @@ def test_damp_wiggles_of_many_fields_equals_one_at_a_time(grid):
         many.damp_wiggles_of([])
         for n in names:
             assert np.array_equal(many.download(n), one.download(n)), n
+
+
+@pytest.mark.parametrize("grid", [(4, 5, 5), (5, 33, 7), (7, 41, 387), (12, 24, 130)])
+def test_post_rk4_filters_edges(grid):
+    """Rows shorter than the passes' halo or longer than one walk of a CTA, every count of
+    passes from 0 to 12, columns that end inside a batch of loads."""
+    st = rough(grid, 61)
+    st["w"][1, 2, 0] = np.inf
+    o = OracleState(st, config_params())
+    o.post_rk4_filters()
+    with GpuAtmosphere(*grid, config_params()) as g:
+        g.upload_state(st)
+        g.post_rk4_filters()
+        for n in ("u", "v", "w"):
+            assert np.array_equal(g.download(n), o.f[n], equal_nan=True), n
