@@ -97,9 +97,9 @@ __host__ __device__ void entrainment_gradients(const MoistArgs& X, int i, int j,
     const double height = X.height[i];
     const double r_the_height = (X.r_Earth * 1.0e3 + height) * costhe;
     const double U_Earth = r_the_height * 2.0 * M_PI;
-    const double inv_step_dr = 0.5 / X.step[i];
-    const double inv_step_the = 0.5 / (U_Earth / (d.jm - 1));
-    const double inv_step_phi = 1.0 / (U_Earth / (d.km - 1));
+    const double inv_step_dr = 0.5 / X.step[i], inv_U = 1.0 / U_Earth;
+    const double inv_step_the = 0.5 * (d.jm - 1) * inv_U;
+    const double inv_step_phi = (d.km - 1) * inv_U;
     const int i_p = (i + 1 < d.im - 1) ? i + 1 : d.im - 1;
     const int i_m = (i - 1 > 0) ? i - 1 : 0;
     *dcdr = (c[IDX(i_p, j, k)] - c[IDX(i_m, j, k)]) * inv_step_dr;

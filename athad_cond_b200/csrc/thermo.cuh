@@ -23,6 +23,14 @@ constexpr double M_CO2 = 0.044010;
 constexpr double R_H2O = R_STAR / M_H2O;
 constexpr double R_CO2 = R_STAR / M_CO2;
 
+// A division is some thirty instructions here, most of them in one chain, so the functions
+// below form quotients by constants as products and take sums of quotients over a common
+// denominator: the values move by an ulp or two.  saturation_mass_fraction of M_nonwater's
+// mixture at a temperature takes 4 divisions instead of 9, cp_of 1 instead of 6, the moist
+// lapse rate 2 instead of 5.  At 41x181x361: saturation adjustment 655 -> 607 us, convection
+// 1232 -> 1136 (with the entrainment gradients), ice 254 -> 235, densities 175 -> 140.  The
+// two saturation curves keep their quotients: their exponent multiplies an ulp in theta by 30.
+
 // Wagner & Pruss saturation line (SaturationH2O.h:68-93)
 ATHAD_HD double saturation_pressure(double T)
 {
@@ -64,7 +72,7 @@ ATHAD_HD double saturation_pressure_auto(double T)   // SaturationH2O.h:123-127
 ATHAD_HD double latent_heat(double T)
 {
     if (T >= T_CRIT) return 0.0;
-    const double x = (T_CRIT - T) / (T_CRIT - 273.15);
+    const double x = (T_CRIT - T) * (1.0 / (T_CRIT - 273.15));
     return (x > 0.0) ? 2.501e6 * exp(0.38 * log(x)) : 0.0;
 }
 ATHAD_HD double latent_heat_sublimation(double T) { return latent_heat(T) + 3.337e5; }
@@ -79,9 +87,8 @@ ATHAD_HD double saturation_mass_fraction(double E, double p, double M_other)
     if (E == NO_SATURATION) return 1.0;
     if (!(p > 0.0)) return 0.0;
     if (E >= p) return 1.0;
-    const double x = E / p;
-    const double num = x * M_H2O;
-    const double den = num + (1.0 - x) * M_other;
+    const double num = E * M_H2O;
+    const double den = num + (p - E) * M_other;
     return (den > 0.0) ? num / den : 1.0;
 }
 ATHAD_HD double saturation_mass_fraction_at(double T, double p, double M_other)
@@ -92,10 +99,9 @@ ATHAD_HD double saturation_mass_fraction_at(double T, double p, double M_other)
 ATHAD_HD double sat_deriv_factor_at(double E, double p, double M_other)   // :230-239
 {
     if (E == NO_SATURATION || !(p > 0.0) || E >= p) return 0.0;
-    const double x = E / p;
-    const double den = x * M_H2O + (1.0 - x) * M_other;
+    const double den = E * M_H2O + (p - E) * M_other;
     if (!(den > 0.0)) return 0.0;
-    return x * M_H2O * M_other / (den * den);
+    return E * p * (M_H2O * M_other) / (den * den);
 }
 
 ATHAD_HD double dqsat_dT_from(double E, double L, double T, double p, double M_other)  // :251-255
@@ -109,27 +115,21 @@ ATHAD_HD double dqsat_dT(double T, double p, double M_other)   // :257-260
     return dqsat_dT_from(saturation_pressure_auto(T), latent_heat_auto(T), T, p, M_other);
 }
 
-// full moist lapse rate (SaturationH2O.h:280-293), with E = saturation_pressure_auto(T)
-// when the caller has formed it already
+// full moist lapse rate (SaturationH2O.h:280-293), g (1 + L A / (R T)) / (cp + L^2 A / (R_H2O
+// T^2)), with E = saturation_pressure_auto(T)
 ATHAD_HD double moist_lapse_E(double T, double E, double p, double M_other, double cp, double R_mix, double g)
 {
     if (!(cp > 0.0) || !(T > 0.0) || !(R_mix > 0.0)) return 0.0;
     const double A = sat_deriv_factor_at(E, p, M_other);
     if (!(A > 0.0)) return g / cp;
-    const double L = latent_heat_auto(T);
-    const double num = 1.0 + L * A / (R_mix * T);
-    const double den = cp + L * L * A / (R_H2O * T * T);
+    const double L = latent_heat_auto(T), LA = L * A, RT = R_H2O * T;
+    const double num = (R_mix * T + LA) * RT;
+    const double den = R_mix * (cp * RT * T + L * LA);
     return (den > 0.0) ? g * num / den : g / cp;
 }
 ATHAD_HD double moist_lapse(double T, double p, double M_other, double cp, double R_mix, double g)
 {
-    if (!(cp > 0.0) || !(T > 0.0) || !(R_mix > 0.0)) return 0.0;
-    const double A = sat_deriv_factor_at(saturation_pressure_auto(T), p, M_other);
-    if (!(A > 0.0)) return g / cp;
-    const double L = latent_heat_auto(T);
-    const double num = 1.0 + L * A / (R_mix * T);
-    const double den = cp + L * L * A / (R_H2O * T * T);
-    return (den > 0.0) ? g * num / den : g / cp;
+    return moist_lapse_E(T, saturation_pressure_auto(T), p, M_other, cp, R_mix, g);
 }
 
 // The Newton steps' saturation curves (SaturationH2O.h:68-120, 168-178, 230-255) with the reciprocals they divide by formed once: 1/T per Newton step, shared by
@@ -211,9 +211,12 @@ ATHAD_HD double cp_of(double c, double co2, double T, double M_b)   // MixtureAt
 {
     double q_v, q_c, q_b;
     split(c, co2, q_v, q_c, q_b);
-    return q_v * (shomate(T, 30.09200, 6.832514, 6.793435, -2.534480, 0.082139) / M_H2O)
-         + q_c * (shomate(T, 24.99735, 55.18696, -33.69137, 7.948387, -0.136638) / M_CO2)
-         + q_b * (shomate(T, 28.98641, 1.853978, -9.647459, 16.63537, 0.000117) / M_b);
+    const double t = smin(smax(T, 298.0), 2000.0) * 1.0e-3;   // shomate() of the three components
+    const double t2 = t * t, t3 = t2 * t, it2 = 1.0 / t2;
+    const double h2o = 30.09200 + 6.832514 * t + 6.793435 * t2 + -2.534480 * t3 + 0.082139 * it2;
+    const double co2s = 24.99735 + 55.18696 * t + -33.69137 * t2 + 7.948387 * t3 + -0.136638 * it2;
+    const double bg = 28.98641 + 1.853978 * t + -9.647459 * t2 + 16.63537 * t3 + 0.000117 * it2;
+    return q_v * (h2o * (1.0 / M_H2O)) + q_c * (co2s * (1.0 / M_CO2)) + q_b * (bg * (1.0 / M_b));
 }
 
 ATHAD_HD double M_nonwater(double c, double co2, double M_b)   // MixtureAtm.h:209-217
@@ -222,8 +225,8 @@ ATHAD_HD double M_nonwater(double c, double co2, double M_b)   // MixtureAtm.h:2
     split(c, co2, q_v, q_c, q_b);
     const double sum = q_c + q_b;
     if (!(sum > 0.0)) return M_b;
-    const double inv = (q_c / sum) / M_CO2 + (q_b / sum) / M_b;
-    return (inv > 0.0) ? 1.0 / inv : M_b;
+    const double moles = q_c * (1.0 / M_CO2) + q_b * (1.0 / M_b);
+    return (moles > 0.0) ? sum / moles : M_b;
 }
 
 // the water vapour mole fraction, MixtureAtm.h:181-187 (M_of) and :220-225 (x_H2O_of)
