@@ -169,3 +169,18 @@ def test_zero_source_returns_zero():
         g.upload_state(st)
         rep = g.pressure_solve(1e-10, 10)
         assert rep["iterations"] == 0 and np.array_equal(g.download("p_dyn"), np.zeros(grid))
+
+
+@pytest.mark.parametrize("grid", [(4, 5, 5), (5, 8, 20), (11, 301, 301), (252, 9, 21), (253, 9, 21)])
+def test_solve_at_the_smoothers_edges(grid):
+    """The smallest grid, an even number of longitudes (seam columns of different colours), rows
+    enough for the smoother's CTAs of four warps, and columns of 250 and 251 levels, the last
+    that its shared memory holds and the first that take one thread each."""
+    st = perturbation(grid, 8, symmetric=False)
+    with GpuAtmosphere(*grid, config_params()) as g:
+        g.upload_state(st)
+        rep = g.pressure_solve(1e-10, 1000)
+        p = g.download("p_dyn")
+    assert rep["converged"] and rep["rel_residual"] <= 1e-10
+    op = operator(*grid)
+    assert relative_residual(op, p, source(op, st["aux_u"], st["aux_v"], st["aux_w"])) <= 1e-9
