@@ -65,8 +65,12 @@ struct State<true> {
     }
 };
 
+// One thread per cell, bound by the round trips of its loads: all of them issued before the
+// first store, and registers for 8 CTAs per SM (FP32 state) or 7.  What the diagnostics add to
+// a step at 41x181x361, mixed / FP64: 88 / 98 us unbounded and with loads after stores; with the
+// loads first, unbounded 107 / 102, 6 CTAs 83 / 84, 7 77 / 80, 8 73 / 84.
 template <bool FP32>
-__global__ void __launch_bounds__(128) rhs_diag_kernel(const RhsDiagArgs a)
+__global__ void __launch_bounds__(128, FP32 ? 8 : 7) rhs_diag_kernel(const RhsDiagArgs a)
 {
     const Dims& d = a.d;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -93,10 +97,17 @@ __global__ void __launch_bounds__(128) rhs_diag_kernel(const RhsDiagArgs a)
     const double coriolis_phi = -2.0 * (costhe * v_ijk + nontrad * sinthe * u_ijk);
 
     if (a.flags & 1) {
+        // every load before the first store, which later loads could not pass
+        y.template load<1>();
+        y.template load<2>();
+        const StarD CL = y.star(5);
+        const StarD IC = y.star(6);
+        const StarD T = y.star(0);
+        const double t_ref_i = a.t_ref[i];
         // acting forces (:447-456)
         a.out[0][c] = 1.0 * a.coeff_Coriolis
             * sqrt((coriolis_rad * coriolis_rad + coriolis_the * coriolis_the + coriolis_phi * coriolis_phi) / 3.0);
-        a.out[1][c] = 1.0 * a.coeff_buoy * (t_ijk - a.t_ref[i]);
+        a.out[1][c] = 1.0 * a.coeff_buoy * (t_ijk - t_ref_i);
         const double pt = dpdthe * inv_rm, pp = dpdphi * inv_rmsinthe;
         a.out[2][c] = -a.coeff_u_p * sqrt((dpdr * dpdr + pt * pt + pp * pp) / 3.0);
         // latent heat of the advected condensate (:458-488): the thresholds are saturation
@@ -107,10 +118,6 @@ __global__ void __launch_bounds__(128) rhs_diag_kernel(const RhsDiagArgs a)
         const double t_u = t_ijk * a.t_0;
         const double q_rain = (t_u >= thermo::T_CRIT) ? 1.0 : 0.0;
         const double q_ice = 0.0;
-        y.template load<1>();
-        y.template load<2>();
-        const StarD CL = y.star(5);
-        const StarD IC = y.star(6);
         const double q_lat = (c_ijk >= 0.85 * q_rain)
             ? u_ijk * ((CL.ip - CL.im) * a.inv_2dr) + v_ijk * inv_rm * ((CL.jp - CL.jm) * a.inv_2dthe)
               + w_ijk * inv_rmsinthe * ((CL.kp - CL.km) * a.inv_2dphi) : 0.0;
@@ -119,7 +126,6 @@ __global__ void __launch_bounds__(128) rhs_diag_kernel(const RhsDiagArgs a)
               + w_ijk * inv_rmsinthe * ((IC.kp - IC.km) * a.inv_2dphi) : 0.0;
         a.out[3][c] = a.coeff_L * (q_lat + q_lat_ice);
         // sensible heat (:490-491), the meridional second difference in mirror-exact form
-        const StarD T = y.star(0);
         const double d2tdr2 = (T.ip - 2.0 * T.c + T.im) * a.inv_dr2;
         const double dtdr = (T.ip - T.im) * a.inv_2dr;
         const double d2tdthe2 = ((T.jp + T.jm) - 2.0 * T.c) * a.inv_dthe2;

@@ -176,10 +176,7 @@ __device__ __forceinline__ void stage_update(const RK4Args& a, int n, long long 
     if (STAGE == 4 && a.store_n) a.Yn_store[n][c] = out;   // storeIntermediateData3D fused
 }
 
-// One RK4 stage.  The right-hand side is evaluated in the order that keeps the fewest
-// values live (turbulence, momentum, temperature, tracers), each term with the operation
-// order of RHS_Atm_Turb.cpp; stencil values a later phase needs again are re-read, which
-// hits L1.
+// field n of the stage's state; 11 is the pressure
 __device__ __forceinline__ const double* stage_field(const RK4Args& a, int n)
 {
     return (n < 11) ? a.Yin[n] : a.p_dyn;
@@ -190,6 +187,10 @@ __device__ __forceinline__ const double* stage_field(const RK4Args& a, int n)
 #endif
 constexpr int kTracerUnroll64 = ATHAD_RK4_TRACER_UNROLL;
 
+// One RK4 stage.  The right-hand side is evaluated in the order that keeps the fewest
+// values live (turbulence, momentum, temperature, tracers), each term with the operations of
+// RHS_Atm_Turb.cpp; stencil values a later phase needs again are re-read, which
+// hits L1.
 template <int STAGE>
 __global__ void __launch_bounds__(kThreads, ATHAD_RK4_MIN_BLOCKS * 128 / kThreads)
 rk4_stage_kernel(const RK4Args a)
