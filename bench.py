@@ -52,15 +52,15 @@ E2E_DOWN = ["t", "u", "v", "w", "c", "cloud", "ice", "gr", "co2", "tke", "dis", 
 # algorithmic bytes moved per grid point by one RK4 step with the time-level copy fused into
 # stage 4.  FP64 form: 273 fields of 8 B (level mean 1 read; stage 1: 37 reads + 22 writes;
 # stages 2-3: 48 + 22; stage 4: 48 + 14 + the 11 time-level writes).  Mixed form: level mean
-# 8 B, stage 1 296 B read + 176 B written, stages 2-3 176 + 88 B, stage 4 220 + 200 B (the
-# field lists of k_rk4m.cu) = 1428 B.
-RK4_BYTES_PER_POINT = {0: 8 * (1 + 59 + 70 + 70 + 62 + 11), 1: 8 + 472 + 264 + 264 + 332 + 88}
+# 8 B, stage 1 296 B read + 176 B written, stages 2-3 176 + 96 B, stage 4 224 + 200 B (the
+# field lists of k_rk4m.cu) = 1448 B.
+RK4_BYTES_PER_POINT = {0: 8 * (1 + 59 + 70 + 70 + 62 + 11), 1: 8 + 472 + 272 + 272 + 336 + 88}
 # algorithmic bytes per grid point of one pressure call (PressureSolverAtm::run with one
 # sweep): source 24 + 8, sweep 24, ceiling 8
 PRESSURE_BYTES_PER_POINT = 64
 # DRAM bytes (read + write) of one RK4 step (level mean and the four stage launches, the
 # time-level copy fused) measured by ncu (one capture of each form's stage launches): per form, grid
-RK4_TRAFFIC = {("fp64", (41, 181, 361)): 6.680e9, ("mixed", (41, 181, 361)): 3.880e9}
+RK4_TRAFFIC = {("fp64", (41, 181, 361)): 5.731e9, ("mixed", (41, 181, 361)): 4.016e9}
 # fields compared between the two forms after the timed iterations: the 11 prognostics and
 # the diagnosed pressure and densities
 ERR_FIELDS = ["t", "u", "v", "w", "c", "cloud", "ice", "gr", "co2", "tke", "dis",
