@@ -217,9 +217,12 @@ void launch_columns(const RadArgs& a, double omega, cudaStream_t st)
     const dim3 grid((a.d.km + 31) / 32, a.d.jm);
     const size_t mem = 3 * 32 * sizeof(double) * (size_t)a.d.im;
     // columns of up to 288 layers fit the 227 KB of a CTA (with the path sums)
-    if (mem <= 221184) {
+    constexpr size_t kMost = 3 * 32 * sizeof(double) * 288;
+    if (mem <= kMost) {
+        // the kernel's limit is the process's: every caller sets the same one, so that a thread
+        // with lower columns cannot lower it between another's call and its launch
         if (mem > 40960)
-            cudaFuncSetAttribute(mlr_columns_kernel<BLEND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mem);
+            cudaFuncSetAttribute(mlr_columns_kernel<BLEND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
         mlr_columns_kernel<BLEND, true><<<grid, 32 * kWarps, mem, st>>>(a, omega);
     } else {
         mlr_columns_kernel<BLEND, false><<<grid, 32 * kWarps, 0, st>>>(a, omega);

@@ -5,6 +5,8 @@ the reference (test_pin_reference.py).
 Tolerance: 1e-12 of each field's largest magnitude (the sweeps call pow and exp, whose last
 bit differs between CUDA and glibc).  A mirror-symmetric state stays mirror-symmetric.
 """
+import threading
+
 import numpy as np
 import pytest
 
@@ -99,3 +101,36 @@ def test_column_heights_and_ragged_rows(grid):
         for n in ("t", "radiation", "epsilon"):
             assert close(g.download(n), o.f[n]) <= 1e-12, n
         assert close(g.download_2d("albedo"), o.f2["albedo"]) <= 1e-12
+
+
+def test_contexts_of_other_heights_on_other_threads():
+    """Two threads, each with a context of its own, one of 70 and one of 280 layers: every call
+    succeeds and the states are those of the same calls one after the other."""
+    grids, calls = [(70, 5, 5), (280, 5, 5)], 1000
+
+    def run(q, ready=lambda: None):
+        with GpuAtmosphere(*grids[q], config_params()) as g:
+            g.upload_state(state(grids[q], 90 + q))
+            ready()
+            for _ in range(calls):
+                g.radiative_heating(0.05)
+            return {n: g.download(n) for n in ("t", "radiation", "epsilon")}
+
+    want = [run(q) for q in range(2)]
+    together = threading.Barrier(2, timeout=60)
+    errors, got = [], [None, None]
+
+    def work(q):
+        try:
+            got[q] = run(q, together.wait)
+        except Exception as e:   # reported by the test's own thread
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(q,)) for q in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for q in range(2):
+        for n in want[q]:
+            assert np.array_equal(got[q][n], want[q][n]), (grids[q], n)
