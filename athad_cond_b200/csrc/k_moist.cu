@@ -244,7 +244,7 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
             const double p_b = p->F[ATHAD_P_STAT][cb];
             const double qsb = QSC(i_base);
             const double L_b = (T_b >= t_0) ? p->lv : p->ls;
-            const double th_p = T_b * exp(kappa * log(p->p_0 / p_b) + L_b * qsb / (p->cp_l * T_b));
+            const double th_p = T_b * pow(p->p_0 / p_b, kappa) * exp(L_b * qsb / (p->cp_l * T_b));
             int became = 0, i_top = i_base;
             double cape = 0.0;
             // the next level's values are loaded while this level computes
@@ -259,8 +259,7 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 const double T_e = T_i * t_0;
                 const double L_e = (T_e >= t_0) ? p->lv : p->ls;
                 const double qs_e = safe_q_sat(X, saturation_pressure_auto(T_i * t_0 + MC_T_ADD_U), p_e, C_i);
-                // (p_0 / p_e)^kappa exp(L q / (cp T)) as one exponential
-                const double th_e = T_e * exp(kappa * log(p->p_0 / p_e) + L_e * qs_e / (p->cp_l * T_e));
+                const double th_e = T_e * pow(p->p_0 / p_e, kappa) * exp(L_e * qs_e / (p->cp_l * T_e));
                 if (th_p - th_e > 0.0) {
                     became = 1;
                     i_top = i;

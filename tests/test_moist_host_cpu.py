@@ -119,3 +119,20 @@ def test_host_column_code_with_non_finite_inputs(host_lib):
     f = host_run(host_lib, o)
     o.moist_convection(2)
     assert_close(f, o, "non-finite")
+
+
+@pytest.mark.parametrize("pressure", [-0.0])
+def test_host_column_code_at_vanishing_pressures(host_lib, pressure):
+    """A negative zero, whose ratios are infinite, in single cells of convecting columns."""
+    grid = (11, 21, 41)
+    st = convective_state(grid, seed=59)
+    rng = np.random.default_rng(59)
+    for n in ("u", "v", "E_u", "M_u"):
+        st[n] = rng.normal(size=grid)
+    p = st["p_stat"].copy()
+    p[tuple(rng.integers(1, s - 1, 40) for s in grid)] = pressure
+    st["p_stat"] = p
+    o = OracleState(st, config_params())
+    f = host_run(host_lib, o)
+    o.moist_convection(2)
+    assert_close(f, o, pressure)
