@@ -29,6 +29,24 @@ ATHAD_HD bool is_finite_bits(double v)
     return (b & 0x7FF0000000000000ULL) != 0x7FF0000000000000ULL;
 }
 
+// a / b where y, the reciprocal of b or a product of reciprocals that is within some ulps of it,
+// is at hand: the product a y corrected by its remainder (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).  It is
+// the rounded quotient (always, with y the rounded reciprocal), where a division takes some
+// thirty instructions.  quot_finite: a, b and the quotient finite and b not zero.  quot: where
+// the correction is not finite (b zero or infinite, an infinite a) the product stands, which is
+// the quotient there.
+ATHAD_HD double quot_finite(double a, double b, double y)
+{
+    const double q = a * y;
+    return fma(fma(-q, b, a), y, q);
+}
+ATHAD_HD double quot(double a, double b, double y)
+{
+    const double v = quot_finite(a, b, y);
+    return is_finite_bits(v) ? v : a * y;
+}
+
 // safe_clamp of RungeKutta_Atm_Turb.cpp:76-81
 ATHAD_HD double safe_clamp(double v, double lo, double hi)
 {

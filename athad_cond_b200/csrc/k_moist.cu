@@ -545,7 +545,7 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 double cu = 0.0;
                 if (fabs(Mu) > MC_COEFF_RECURR) {
                     // Two condensation steps, a chain of transcendentals and quotients that
-                    // nothing overlaps: the quotients by T, p and the mixture masses are formed
+                    // nothing overlaps: the quotient by p and the mixture masses are formed
                     // once, and the step's share dq / (1 + G) from one division.
                     double T_u = su * p->s_0 / p->cp_l;
                     const double p_u = cur.P, inv_p = 1.0 / p_u;
@@ -553,20 +553,18 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                     const double M_o_u = M_nonwater(cur.C, cur.CO2, p->M_bg);
                     double dcond_tot = 0.0;
                     for (int it = 0; it < 2; ++it) {
-                        const double inv_T = 1.0 / T_u;
-                        const double E_s = (T_u >= T_CRIT) ? NO_SATURATION
-                                         : (T_u >= T_TRIPLE) ? p_sat_r(T_u, inv_T) : p_subl_r(T_u, inv_T);
-                        const double dq = qvu - sat_value(E_s, p_u, inv_p, M_ref).q;
+                        const double E_s = saturation_pressure_auto(T_u);
+                        const double dq = qvu - saturation_mass_fraction(E_s, p_u, M_ref);
                         if (dq <= 0.0) break;
                         const double L_cp = ((T_u >= t_0) ? p->lv : p->ls) / p->cp_l;
                         // G = L / cp_l dq_sat/dT = N / D (sat_deriv_factor_at, dqsat_dT_from)
                         double N = 0.0, D = 1.0;
                         if (T_u > 0.0 && E_s != NO_SATURATION && p_u > 0.0 && !(E_s >= p_u)) {
-                            const double x = E_s * inv_p;
+                            const double x = quot(E_s, p_u, inv_p);
                             const double den = x * M_H2O + (1.0 - x) * M_o_u;
                             if (den > 0.0) {
-                                D = den * den;
-                                N = L_cp * (x * M_H2O * M_o_u) * latent_heat_auto(T_u) * ((inv_T * inv_T) * (1.0 / R_H2O));
+                                D = den * den * (R_H2O * T_u * T_u);
+                                N = L_cp * (x * M_H2O * M_o_u) * latent_heat_auto(T_u);
                             }
                         }
                         const double dcond = dq * D / (D + N);

@@ -121,9 +121,10 @@ def test_host_column_code_with_non_finite_inputs(host_lib):
     assert_close(f, o, "non-finite")
 
 
-@pytest.mark.parametrize("pressure", [-0.0])
+@pytest.mark.parametrize("pressure", [1e-320, -0.0])
 def test_host_column_code_at_vanishing_pressures(host_lib, pressure):
-    """A negative zero, whose ratios are infinite, in single cells of convecting columns."""
+    """A denormal pressure, whose reciprocal is infinite, and a negative zero, whose ratios are
+    infinite, in single cells of convecting columns."""
     grid = (11, 21, 41)
     st = convective_state(grid, seed=59)
     rng = np.random.default_rng(59)
