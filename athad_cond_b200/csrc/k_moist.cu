@@ -475,7 +475,9 @@ __host__ __device__ void mc_column(const MoistArgs& X, int j, int k)
                 if (t_u >= t_0) p->F[ATHAD_G_P][c] = (ip == 1) ? 0.0 : K_p * qcu_c;
                 else p->F[ATHAD_G_P][c] = 0.0;
             }
-            i_eu = ib + 1;   // levels from here on hold theirs (the base only moves down)
+            // levels from here on hold theirs for the next pass, which takes them where it is
+            // deep too (a shallow pass leaves zeros)
+            i_eu = deep ? ib + 1 : im;
             p->F[ATHAD_M_U][IDX(il, j, k)] = 0.0;
         }
         if (interior) cloud_base_update(X, j, k, i_deep_beg, i_lfs, &i_base);
