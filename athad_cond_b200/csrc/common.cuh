@@ -99,6 +99,11 @@ __device__ __forceinline__ void pdl_wait(int& index)
     pdl_wait();
     asm volatile("" : "+r"(index));
 }
+__device__ __forceinline__ void pdl_wait(int& index, int& other)   // where some addresses are formed from `other` alone
+{
+    pdl_wait(index);
+    asm volatile("" : "+r"(other));
+}
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

@@ -148,7 +148,7 @@ __device__ __forceinline__ double2 zonal_two(const double* __restrict__ row, int
     const double2 x = *reinterpret_cast<const double2*>(row + k);
     const double west = row[k == 0 ? km - 1 : k - 1];
     const double east = (k + 1 >= km) ? 0.0 : row[k + 2 >= km ? 0 : k + 2];
-    const double e0 = (k + 1 >= km) ? row[0] : x.y;
+    const double e0 = (k + 1 >= km) ? row[k + 1 - km] : x.y;   // row[0], addressed from k (pdl_wait)
     return make_double2(x.x + 0.25 * (west - 2.0 * x.x + e0), x.y + 0.25 * (x.x - 2.0 * x.y + east));
 }
 

@@ -207,14 +207,14 @@ rk4_stage_kernel(const RK4Args a)
     pdl_trigger();
     const Dims& d = a.d;
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    pdl_wait(k);
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     // the even stages walk the radial planes from the top down (ATHAD_RK4_SERPENTINE, kernels.cuh)
 #if ATHAD_RK4_SERPENTINE
-    const int i = (STAGE % 2 == 0) ? d.im - 1 - (int)blockIdx.z : (int)blockIdx.z;
+    int i = (STAGE % 2 == 0) ? d.im - 1 - (int)blockIdx.z : (int)blockIdx.z;
 #else
-    const int i = blockIdx.z;
+    int i = blockIdx.z;
 #endif
+    pdl_wait(k, i);   // i alone addresses t_ref, which the launch before stage 1 writes
     if (k >= d.km || j >= d.jm) return;
     const long long c = idx3(d, i, j, k);
     const bool interior = (i > 0 && i < d.im - 1 && j > 0 && j < d.jm - 1 && k > 0 && k < d.km - 1);

@@ -537,16 +537,16 @@ rk4m_stage_kernel(const RK4MArgs a, const BatchStep* step)
 {
     pdl_trigger();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    pdl_wait(k);
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     // the even stages walk the radial planes from the top down, so that each stage starts
     // on the planes its predecessor wrote last (1.036 -> 1.030 ms per step at 41x181x361;
     // a stage's cells are independent, so the order changes no result)
 #if ATHAD_RK4_SERPENTINE
-    const int i = (STAGE % 2 == 0) ? a.d.im - 1 - (int)blockIdx.z : (int)blockIdx.z;
+    int i = (STAGE % 2 == 0) ? a.d.im - 1 - (int)blockIdx.z : (int)blockIdx.z;
 #else
-    const int i = blockIdx.z;
+    int i = blockIdx.z;
 #endif
+    pdl_wait(k, i);   // i alone addresses t_ref, which the launch before stage 1 writes
     prefetch_tile<STAGE>(a, i, blockIdx.y * BY, blockIdx.x * BX, BX, BY, threadIdx.y * BX + threadIdx.x, BX * BY);
     if (k >= a.d.km || j >= a.d.jm) return;
     rk4m_cell<STAGE>(a, i, j, k, MEMBER ? step->buoy_pref : a.buoy_pref);
