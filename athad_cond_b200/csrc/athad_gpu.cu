@@ -725,7 +725,6 @@ athad_status athad_pressure_sweep(athad_ctx* ctx, int32_t n_sweeps, int32_t tota
     if (!ctx || n_sweeps < 0) return fail(ctx, ATHAD_ERR_INVALID, "pressure_sweep: bad argument");
     if (n_sweeps == 0) return ATHAD_OK;
     PoissonArgs a = poisson_args(ctx, total_iter_count);
-    a.aux_lid = 1;
     a.first_sweep = 1;
     if (poisson_sweeps_split(ctx->L.d, n_sweeps)) {
         // RK4 stage buffers: scratch between RK4 steps

@@ -95,15 +95,10 @@ __global__ void __launch_bounds__(256) poisson_src_kernel(PoissonArgs a)
 
 // one colour of the red-black sweep, PressureSolverAtm.h:225-486 (update :475-480); thread
 // kk of row (i, j) takes the kk-th cell of the colour, k = 2 kk + ((i + j + COLOUR) & 1),
-// so every lane of a warp updates a cell
-// ATHAD_POISSON_SRC_FIELD 1: the source formed by its own launch into a scratch field that
-// both colours read; 0: each colour forms its cells' sources from aux_u/v/w.  The pressure
-// call at 41x181x361 inside the model iteration (PDL on, mixed form, 300 iterations):
-// 59.1 us with the source field, 68.8 us forming the sources in the colours (46 registers,
-// 5 CTAs of 256 per SM), 63.7 us at 8 CTAs (spills), 60.0 us at 6.
-#ifndef ATHAD_POISSON_SRC_FIELD
-#define ATHAD_POISSON_SRC_FIELD 1
-#endif
+// so every lane of a warp updates a cell.  The source comes from its own launch, in a scratch
+// field that both colours read: the pressure call at 41x181x361 inside the model iteration (PDL
+// on, mixed form, 300 iterations) takes 59.1 us so, 60.0 to 68.8 with the sources formed in the
+// colours from aux_u/v/w.
 #ifndef ATHAD_POISSON_MIN_BLOCKS
 #define ATHAD_POISSON_MIN_BLOCKS 1
 #endif
@@ -117,15 +112,11 @@ __global__ void __launch_bounds__(256, ATHAD_POISSON_MIN_BLOCKS) poisson_colour_
     const int i = blockIdx.z;
     const int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((i + j + COLOUR) & 1);
     const bool fluid = !(k < 1 || k >= d.km - 1 || j < 1 || j >= d.jm - 1 || i < 1 || i >= d.im - 1);
-    bool clamped = false, beyond = false;
+    bool beyond = false;
     if (fluid) {
         const long long c = idx3(d, i, j, k);
         const PoiIJ P = a.poi[i * d.jm + j];
-#if ATHAD_POISSON_SRC_FIELD
         const double src = __ldg(a.src + c);
-#else
-        const double src = cell_source(a, P, i, c, clamped);
-#endif
         const long long sI = d.plane, sJ = d.pitch;
         const double* p = a.p;
         const double pip = p[c + sI], pim = p[c - sI];
@@ -138,7 +129,6 @@ __global__ void __launch_bounds__(256, ATHAD_POISSON_MIN_BLOCKS) poisson_colour_
         a.p[c] = v;
         beyond = !(fabs(v) <= a.ceiling);      // non-finite included
     }
-    count_clamped(a, clamped);
     // one atomic per warp that has such a value (rare): the ceiling pass runs only then
     if (__any_sync(0xffffffffu, beyond) && (threadIdx.x & 31) == 0 && a.counters)
         atomicOr(a.counters + 5, 1ull);
@@ -186,12 +176,10 @@ __global__ void __launch_bounds__(128) poisson_bc_kernel(PoissonArgs a)
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long n_planes = 2LL * d.jm * d.km, n_rows = 2LL * d.im * d.km, n_seam = 2LL * d.im * d.jm;
     int i, j, k;
-    bool plane = false;
     if (t < n_planes) {
         const int side = (int)(t / ((long long)d.jm * d.km));
         const int r = (int)(t % ((long long)d.jm * d.km));
         i = side ? d.im - 1 : 0; j = r / d.km; k = r % d.km;
-        plane = true;
     } else if ((t -= n_planes) < n_rows) {
         const int side = (int)(t / ((long long)d.im * d.km));
         const int r = (int)(t % ((long long)d.im * d.km));
@@ -204,11 +192,8 @@ __global__ void __launch_bounds__(128) poisson_bc_kernel(PoissonArgs a)
         return;
     }
     a.p[idx3(d, i, j, k)] = bc_final(d, a.p, i, j, k);
-    if (a.aux_lid && plane && k >= 1 && k < d.km - 1 && j >= 1 && j < d.jm - 1)
-        aux_lid_cell(a, i, j, k);   // the aux radial boundary, PressureSolverAtm.h:106-121
 }
 
-// aux_lid: also the aux radial boundary (a sweep whose source launch wrote it passes 0)
 static void launch_bcs(const PoissonArgs& a, cudaStream_t st)
 {
     const Dims& d = a.d;
@@ -272,20 +257,10 @@ void launch_poisson_sweep(const PoissonArgs& a, cudaStream_t st)
     const dim3 half_grid(((d.km + 1) / 2 + 31) / 32, (d.jm + 7) / 8, d.im);
     // each launch after the first waits for the one before it (pdl_wait) but is scheduled
     // during its tail
-#if ATHAD_POISSON_SRC_FIELD
     poisson_src_kernel<<<grid, block, 0, st>>>(a);
     launch_dependent(poisson_colour_kernel<0>, half_grid, block, 0, st, a);
-#else
-    poisson_colour_kernel<0><<<half_grid, block, 0, st>>>(a);
-#endif
     launch_dependent(poisson_colour_kernel<1>, half_grid, block, 0, st, a);
-#if ATHAD_POISSON_SRC_FIELD
-    PoissonArgs b = a;
-    b.aux_lid = 0;   // the source launch wrote the aux boundary (aux is constant in a sweep)
-    launch_bcs(b, st);
-#else
     launch_bcs(a, st);
-#endif
     // one wave of CTAs, each striding over the grid: when no value reached the ceiling (the
     // usual case) the launch costs one short wave
     const long long quads = (long long)d.im * d.plane / 4;

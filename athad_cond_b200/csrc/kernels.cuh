@@ -148,7 +148,6 @@ struct PoissonArgs {
                                     // launch, [0] the call's total (folded by the ceiling)
     double inv_2dr, inv_2dthe, inv_2dphi;
     int anelastic, metric_div;
-    int aux_lid;                // the boundary passes also write the aux radial boundary
     int first_sweep;            // the ceiling starts the call's count instead of adding
     double ceiling;
 };
