@@ -594,7 +594,8 @@ static athad_status rk4_step_fp64(athad_ctx* ctx, const athad_step_scalars* s)
     a.coeff_MC_vel = p.L_atm / (p.u_0 * p.u_0);
     a.coeff_MC_q = p.L_atm / (p.u_0 * p.c_0);
     a.coeff_MC_t = p.L_atm / (p.u_0 * p.t_0);
-    a.lv = p.lv; a.ls = p.ls; a.inv_pr_turb = 1.0 / p.pr_turb; a.L_atm_over_u0 = p.L_atm / p.u_0;
+    a.lv = p.lv; a.ls = p.ls; a.L_atm = p.L_atm; a.u_0 = p.u_0; a.inv_u_0 = 1.0 / p.u_0;
+    a.pr_turb = p.pr_turb; a.inv_pr_turb = 1.0 / p.pr_turb;
     a.inv_re = 1.0 / p.re_turb;
     a.nue_max = 1000.0 / (p.u_0 * p.L_atm);
     a.nue_air_nd = 1.5e-5 / (p.u_0 * p.L_atm);

@@ -39,7 +39,7 @@ struct RK4Args {
     double inv_2dr, inv_2dthe, inv_2dphi, inv_dr2, inv_dthe2, inv_dphi2;
     double dt, half_dt, dt_sixth, diffusion_ramp, buoyancy_ramp, tke_max_nd, force_nd;
     double coeff_energy_p, coeff_energy, coeff_MC_vel, coeff_MC_q, coeff_MC_t;
-    double lv, ls, inv_pr_turb, L_atm_over_u0;
+    double lv, ls, L_atm, u_0, inv_u_0, pr_turb, inv_pr_turb;
     // launch constants the reference evaluates per cell from the same operands (hoisted,
     // values identical): 1/re_turb, 1000/(u_0 L_atm), 1.5e-5/(u_0 L_atm), the tracer
     // diffusivities, the buoyancy prefactor buoyancy_ramp*1*g*dt/u_0 and the drag

@@ -371,3 +371,27 @@ def test_many_sweeps_bit_exact(grid, n_sweeps, anelastic):
             assert np.array_equal(g.download(n), o.f[n]), n
         r = g.report()
         assert r["poisson_src_cells"] == cells and r["poisson_src_clamped"] == clamped
+
+
+@pytest.mark.parametrize("turb", [Turb.K_EPSILON, Turb.K_OMEGA, Turb.K_OMEGA_SST])
+def test_rk4_step_rounds_as_the_oracle(turb):
+    """The FP64 step forms its quotients from shared reciprocals, corrected to the rounded
+    quotient: every output is the oracle's bit for bit.  The SST closure's dissipation source
+    alone is left out, which takes a power and a hyperbolic tangent of libm's or of CUDA's."""
+    grid = (21, 31, 61)
+    p = config_params()
+    p.turb_model = int(turb)
+    st = make_state(*grid, seed=7)
+    rng = np.random.default_rng(7)
+    for n in ("MC_t", "MC_q", "MC_v", "MC_w", "S_c", "S_r", "S_i", "S_s", "S_g", "S_v"):
+        st[n] = 1e-3 * rng.normal(size=grid)
+    st["nue"] = 1e-3 * np.abs(rng.normal(size=grid))
+    o = OracleState(st, p)
+    o.rk4(dt=4e-5, diffusion_ramp=1.0, buoyancy_ramp=0.5, write_diagnostics=True)
+    names = PROG + ["aux_u", "aux_v", "aux_w", "prod", "tke_source"]
+    if turb != Turb.K_OMEGA_SST:
+        names.append("dis_source")
+    with gpu_with(st, p) as g:
+        g.solveRungeKutta_Atmosphere_Turb(4e-5, 1.0, 0.5, write_diagnostics=True)
+        for n in names:
+            assert np.array_equal(g.download(n), o.f[n]), n
