@@ -88,9 +88,10 @@ __global__ void __launch_bounds__(128) turb_sources_kernel(TurbArgs a)
     const double ddisdr = (D[c + sI] - D[c - sI]) * inv_2dr * exp_rm;
 
     const double nue_max = a.nue_max;
-    // The production rounds as the reference's does; in the closures below a division (some
-    // thirty dependent instructions, most of the kernel's) gives a reciprocal that the quotients
-    // by the same value share: 183 -> 126 us per call at 41x181x361 with the SST closure.
+    // A division is some thirty dependent instructions, most of the kernel's; in the closures
+    // below it gives a reciprocal that the quotients by the same value share, each corrected to
+    // the rounded quotient (quot): 183 -> 123 us per call at 41x181x361 with the SST closure
+    // (119 with the plain products).
     double cnue = (MODEL == ATHAD_TURB_K_EPSILON) ? kCNue * tke * tke / dis : tke / dis;
     cnue = dmin(cnue, nue_max);
     const double der = 0.66667 * (dudr + dvdthe + dwdphi);
@@ -132,24 +133,28 @@ __global__ void __launch_bounds__(128) turb_sources_kernel(TurbArgs a)
     } else {
         // the theta and phi gradients of tke/dis the closures form with 1/rm (:593-596,
         // :722-725)
-        const double inv_the = inv_2dthe / rm, inv_phi = inv_2dphi / (rm * sinthe);
-        const double dtkedthe_neu = (T[c + sJ] - T[c - sJ]) * inv_the;
-        const double ddisdthe_neu = (D[c + sJ] - D[c - sJ]) * inv_the;
-        const double dtkedphi_neu = (T[c + 1] - T[c - 1]) * inv_phi;
-        const double ddisdphi_neu = (D[c + 1] - D[c - 1]) * inv_phi;
+        const double den_the = rm * 2.0 * a.dthe, inv_the = 1.0 / den_the;
+        const double den_phi = rm * sinthe * 2.0 * a.dphi, inv_phi = 1.0 / den_phi;
+        auto by_the = [&](double x) { return quot(x, den_the, inv_the); };
+        auto by_phi = [&](double x) { return quot(x, den_phi, inv_phi); };
+        const double dtkedthe_neu = by_the(T[c + sJ] - T[c - sJ]);
+        const double ddisdthe_neu = by_the(D[c + sJ] - D[c - sJ]);
+        const double dtkedphi_neu = by_phi(T[c + 1] - T[c - 1]);
+        const double ddisdphi_neu = by_phi(D[c + 1] - D[c - 1]);
         const double cross = dtkedr * ddisdr + dtkedthe_neu * ddisdthe_neu + dtkedphi_neu * ddisdphi_neu;
         if (MODEL == ATHAD_TURB_K_OMEGA) {
             const double bet_star = 0.09, gam = 0.52, C_lim = 0.875, bet_0 = 0.0708;
-            const double inv_r = inv_2dr / (rm + 1.0);
-            const double dudr_u = (u[c + sI] - u[c - sI]) * inv_r;
-            const double dvdthe_u = (v[c + sJ] - v[c - sJ]) * inv_the;
-            const double dwdphi_u = (w[c + 1] - w[c - 1]) * inv_phi;
-            const double dudthe_u = (u[c + sJ] - u[c - sJ]) * inv_the;
-            const double dudphi_u = (u[c + 1] - u[c - 1]) * inv_phi;
-            const double dvdr_u = (v[c + sI] - v[c - sI]) * inv_r;
-            const double dwdr_u = (w[c + sI] - w[c - sI]) * inv_r;
-            const double dvdphi_u = (v[c + 1] - v[c - 1]) * inv_phi;
-            const double dwdthe_u = (w[c + sJ] - w[c - sJ]) * inv_the;
+            const double inv_r = 1.0 / (rm + 1.0);
+            auto by_r = [&](double x) { return quot(quot(x, 2.0 * a.dr, inv_2dr), rm + 1.0, inv_r); };
+            const double dudr_u = by_r(u[c + sI] - u[c - sI]);
+            const double dvdthe_u = by_the(v[c + sJ] - v[c - sJ]);
+            const double dwdphi_u = by_phi(w[c + 1] - w[c - 1]);
+            const double dudthe_u = by_the(u[c + sJ] - u[c - sJ]);
+            const double dudphi_u = by_phi(u[c + 1] - u[c - 1]);
+            const double dvdr_u = by_r(v[c + sI] - v[c - sI]);
+            const double dwdr_u = by_r(w[c + sI] - w[c - sI]);
+            const double dvdphi_u = by_phi(v[c + 1] - v[c - 1]);
+            const double dwdthe_u = by_the(w[c + sJ] - w[c - sJ]);
             const double S11 = dudr_u, S22 = dvdthe_u, S33 = dwdphi_u;
             const double S12 = 0.5 * (dudthe_u + dvdr_u);
             const double S13 = 0.5 * (dudphi_u + dwdr_u);
@@ -176,13 +181,14 @@ __global__ void __launch_bounds__(128) turb_sources_kernel(TurbArgs a)
             const double y_phys = dmax(L.height - a.y_mount, 1.0e-6);
             const double y_star = y_phys / a.L_atm;
             const double inv_dis = 1.0 / dis, inv_y = 1.0 / y_star, inv_y_dis = inv_y * inv_dis;
-            const double CD_kw = dmax(2.0 * sig_w2 * inv_dis * cross, 1.0e-20);
-            const double from_wall = sqrt(tke) * ((1.0 / bet_star) * inv_y_dis);
-            const double viscous = 500.0 * nue_air_nd * (inv_y * inv_y_dis);
+            const double CD_kw = dmax(quot(2.0 * sig_w2, dis, inv_dis) * cross, 1.0e-20);
+            const double from_wall = quot(sqrt(tke), bet_star * dis * y_star, (1.0 / bet_star) * inv_y_dis);
+            const double viscous = quot(500.0 * nue_air_nd, y_star * y_star * dis, inv_y * inv_y_dis);
             const double arg1 = dmin(dmax(from_wall, viscous), 4.0 * sig_w2 * tke / (CD_kw * y_star * y_star));
             const double arg2 = dmax(2.0 * from_wall, viscous);
-            const double a1_2 = arg1 * arg1;
-            const double F1 = tanh(a1_2 * a1_2);
+            // arg1^4 with the square's rounding error, as close as pow(arg1, 4); tanh(3^4) is 1
+            const double a1_2 = arg1 * arg1, a1_err = fma(arg1, arg1, -a1_2);
+            const double F1 = (arg1 >= 3.0) ? 1.0 : tanh(fma(a1_2, a1_2, 2.0 * a1_2 * a1_err));
             const double F2 = tanh(arg2 * arg2);
             nue = a1 * tke / dmax(a1 * dis, Omega * F2);
             const double dis_safe = dis, tke_safe = dmax(tke, 1.0e-20);
@@ -190,7 +196,7 @@ __global__ void __launch_bounds__(128) turb_sources_kernel(TurbArgs a)
             const double Y_k = bet_star * tke_safe * dis_safe;
             const double P_w = (F1 * gam1 + (1.0 - F1) * gam2) * P_k * dis_safe / tke_safe;
             const double Y_w = (F1 * bet1 + (1.0 - F1) * bet2) * dis_safe * dis_safe;
-            const double D_w = 2.0 * (1.0 - F1) * sig_w2 * inv_dis * cross;
+            const double D_w = quot(2.0 * (1.0 - F1) * sig_w2, dis, inv_dis) * cross;
             tke_source = P_k - Y_k;
             dis_source = P_w - Y_w + D_w;
         }

@@ -71,3 +71,19 @@ def test_turbulence_run_keeps_mirror_symmetry():
             assert np.array_equal(a, mirror(a, False)), n
         vs = g.download_2d("vel_star")
         assert np.array_equal(vs, vs[::-1, :])
+
+
+def test_eddy_viscosity_of_k_omega_rounds_as_the_oracle():
+    """nue of the k-omega closure is made of quotients and square roots alone: the gradients'
+    quotients, formed from shared reciprocals and corrected, give the oracle's bits."""
+    grid = (21, 31, 61)
+    p = config_params()
+    p.turb_model = int(Turb.K_OMEGA)
+    st = state(grid, 61)
+    o = OracleState(st, p)
+    o.turbulence_run(compat=0)
+    with GpuAtmosphere(*grid, p) as g:
+        g.upload_state(st)
+        g.turbulence_run()
+        for n in ("nue", "tke_source"):
+            assert np.array_equal(g.download(n), o.f[n]), n
