@@ -133,7 +133,9 @@ __global__ void __launch_bounds__(128, 4) ice_columns_kernel(IceArgs a)
             }
             const double step = a.step_f[i];
             const double mass_layer = rh * step;
-            const double dt_snow_dim = step * (1.0 / 0.96), inv_dt = 1.0 / dt_snow_dim;
+            const double dt_snow_dim = quot_finite(step, 0.96, 1.0 / 0.96), inv_dt = 1.0 / dt_snow_dim;
+            auto per_dt = [&](double x) { return quot(x, dt_snow_dim, inv_dt); };
+            const double max_cloud_loss = per_dt(cl), max_ice_loss = per_dt(ic);
             if (!(t_u > t_0) && !(t_u <= kThn)) {
                 N_i = kNi0 * exp(0.2 * (t_0 - t_u));
                 m_i = dmin((rh * ic) / N_i, kMiMax);
@@ -146,9 +148,9 @@ __global__ void __launch_bounds__(128, 4) ice_columns_kernel(IceArgs a)
             } else {
                 S_nuc = 0.0;
             }
-            double S_c_frz = (t_u < kThn) ? cl * inv_dt : 0.0;
+            double S_c_frz = (t_u < kThn) ? max_cloud_loss : 0.0;
             if (cv > q_Ice) S_i_dep = kCiDep * N_i * cbrt(m_i) * (cv - q_Ice);
-            if (cv < q_Ice) S_i_dep = dmax(-ic * inv_dt, (cv - q_Ice) * inv_dt);
+            if (cv < q_Ice) S_i_dep = dmax(-max_ice_loss, per_dt(cv - q_Ice));
             double S_c_au = (cl > kQcCrit) ? kCcAu * (cl - kQcCrit) : 0.0;
             double S_i_au = (ic > 0.0) ? dmax(kCiAu * ic, 0.0) : 0.0;
             double S_d_au = 0.0;
@@ -165,7 +167,7 @@ __global__ void __launch_bounds__(128, 4) ice_columns_kernel(IceArgs a)
                     S_s_melt = kCsMelt * (1.0 + kBsMelt * S526) * (t_u - t_0) * cbrt(Snow);
                     S_s_melt = dmin(S_s_melt, Snow / mass_layer);
                 }
-                S_i_melt = ic * inv_dt;
+                S_i_melt = max_ice_loss;
             }
             double S_agg = 0.0, S_i_cri = 0.0, S_r_cri = 0.0;
             if (t_u <= t_0) {
@@ -191,13 +193,11 @@ __global__ void __launch_bounds__(128, 4) ice_columns_kernel(IceArgs a)
             }
             // the cloud-water and cloud-ice limiters (:413-434)
             const double S_cloud_total = S_c_au + S_ac + S_rim + S_c_frz + S_shed;
-            const double max_cloud_loss = cl * inv_dt;
             if (S_cloud_total > max_cloud_loss && S_cloud_total > 0) {
                 const double fac = max_cloud_loss / S_cloud_total;
                 S_c_au *= fac; S_ac *= fac; S_rim *= fac; S_c_frz *= fac; S_shed *= fac;
             }
             const double S_ice_total = S_i_au + S_d_au + S_agg + S_i_cri + S_i_melt;
-            const double max_ice_loss = ic * inv_dt;
             if (S_ice_total > max_ice_loss && S_ice_total > 0) {
                 const double fac = max_ice_loss / S_ice_total;
                 S_i_au *= fac; S_d_au *= fac; S_agg *= fac; S_i_cri *= fac; S_i_melt *= fac;

@@ -67,3 +67,23 @@ def test_two_cat_ice_scheme_keeps_mirror_symmetry():
         for n in OUT:
             a = g.download(n)
             assert np.array_equal(a, mirror(a, False)), n
+
+
+def test_freezing_of_cloud_water_rounds_as_the_oracle():
+    """Below the homogeneous freezing point, without rain or snow and with too little cloud water
+    to convert, the cloud water's source is -cloud / dt alone: the oracle's bits."""
+    grid = (21, 31, 61)
+    st = make_state(*grid, seed=77)
+    rng = np.random.default_rng(77)
+    st["t"] = (220.0 + 15.0 * rng.random(grid)) / 273.15
+    st["cloud"] = 4e-4 * rng.random(grid)
+    for n in ("ice", "P_rainn", "P_snown", "S_c_c"):
+        st[n] = np.zeros(grid)
+    o = OracleState(st, config_params())
+    with GpuAtmosphere(*grid, config_params()) as g:
+        g.upload_state(st)
+        g.two_cat_ice_scheme()
+        o.two_cat_ice_scheme()
+        inner = (slice(0, -1), slice(1, -1), slice(1, -1))
+        assert (o.f["S_c"][inner] < 0.0).all()
+        assert np.array_equal(g.download("S_c"), o.f["S_c"])
