@@ -1,9 +1,9 @@
 // batch.cu - ensembles of contexts advanced together (athad_batch_* of include/athad_gpu.h).
 //
 // A batch owns no field memory: its members are ordinary mixed-precision contexts, each
-// with its own grid and parameters.  One batched model iteration forks a few side streams
-// (lanes) from the batch's stream, enqueues each member's iteration on one of them - the
-// column physics at the member's own cadence (pressure sweep every 4th iteration, saturation
+// with its own grid and parameters.  One batched model iteration forks up to 32 of the members'
+// own streams (lanes) from the batch's stream, enqueues each member's iteration on one of them -
+// the column physics at the member's own cadence (pressure sweep every 4th iteration, saturation
 // adjustment + moist convection + densities every 2nd), the level mean, the four RK4 stages
 // with the time-level copy fused into the last - and joins the lanes in a tiny launch that
 // advances the members' device-side iteration counters.
@@ -14,9 +14,10 @@
 // One persistent launch per stage over the tiles of all members, behind a join of all
 // column physics, was 1.56 times slower per point than the single-grid stage kernels (a
 // member's arguments in shared memory, neighbouring planes read at unrelated times).  Four
-// iterations, persistent -> lanes: six members of 0.4 to 2.4 M points 19.1 -> 13.8 ms,
-// twelve of 27x99x151 15.3 -> 11.4, six of 15x61x109 2.37 -> 1.69, 32 of 11x21x41 2.68 ->
-// 2.57, one of 31x125x257 3.91 -> 3.06.
+// iterations, persistent -> lanes: the 64 members of the largest ensemble (60.1 M points) 273 ->
+// 128 ms, 64 of 15x61x109 31.9 -> 14.7, 64 of 11x21x41 6.0 -> 3.5, six of 0.4 to 2.4 M points
+// 19.1 -> 13.8, one of 27x99x151 2.44 -> 1.42.  Without a graph, where the host issues each
+// launch: 64 of 15x61x109 33.1 -> 16.0, 64 of 11x21x41 6.9 -> 6.8.
 //
 // Step scalars live on the device: every member's buoyancy ramp min(1, n / ramp_iters) is
 // in its step record, kept with its iteration counter, so one captured CUDA graph of an
@@ -67,7 +68,7 @@ constexpr int kSideStreams = 32;
 
 struct athad_batch {
     std::vector<athad_ctx*> m;
-    std::vector<cudaStream_t> side;     // member q's iteration runs on side[q % size]
+    std::vector<cudaStream_t> side;     // member q's iteration runs on side[q % size], streams of the members
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> join;
     std::vector<RK4MArgs> args;         // the members' stage arguments (stage buffer A in Yout, B in Ybnd)
@@ -134,25 +135,27 @@ static athad_status enqueue_stage(athad_batch* b, int q, int stage, int shape)
 }
 
 // Runs enqueue(q) for every active member with its context's stream on the member's lane,
-// between a fork of the lanes from b->stream and their join to it (also under capture).
+// between a fork of the lanes from b->stream and their join to it (also under capture).  The
+// lanes that have forked join, whatever failed.
 template <class F> static athad_status on_lanes(athad_batch* b, F enqueue)
 {
     const int n = (int)b->m.size(), ns = (int)b->side.size();
     athad_status s = bcuda(b, cudaEventRecord(b->fork, b->stream), "batch fork");
-    for (int q = 0; q < ns && s == ATHAD_OK; q++) s = bcuda(b, cudaStreamWaitEvent(b->side[q], b->fork, 0), "batch fork");
-    if (s != ATHAD_OK) return s;
-    for (int q = 0; q < n; q++) {
+    int forked = 0;
+    for (; forked < ns && s == ATHAD_OK; forked++) s = bcuda(b, cudaStreamWaitEvent(b->side[forked], b->fork, 0), "batch fork");
+    for (int q = 0; q < n && s == ATHAD_OK; q++) {
         if (!b->active[q]) continue;
         athad_ctx* c = b->m[q];
         cudaStream_t saved = c->stream;
         c->stream = b->side[q % ns];
         s = enqueue(q);
         c->stream = saved;
-        if (s != ATHAD_OK) return bfail(b, s, std::string("member ") + std::to_string(q) + ": " + c->err);
+        if (s != ATHAD_OK) bfail(b, s, std::string("member ") + std::to_string(q) + ": " + c->err);
     }
-    for (int q = 0; q < ns && s == ATHAD_OK; q++) {
-        s = bcuda(b, cudaEventRecord(b->join[q], b->side[q]), "batch join");
-        if (s == ATHAD_OK) s = bcuda(b, cudaStreamWaitEvent(b->stream, b->join[q], 0), "batch join");
+    for (int q = 0; q < forked; q++) {
+        cudaError_t e = cudaEventRecord(b->join[q], b->side[q]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->join[q], 0);
+        if (s == ATHAD_OK) s = bcuda(b, e, "batch join");
     }
     return s;
 }
@@ -252,19 +255,18 @@ athad_status athad_batch_create(athad_ctx* const* members, int32_t n_members, co
     }
     st = bcuda(b, cudaMemcpyAsync(b->d_step, steps.data(), sizeof(BatchStep) * n, cudaMemcpyHostToDevice, b->stream), "steps");
     if (st == ATHAD_OK) st = bcuda(b, cudaStreamSynchronize(b->stream), "batch create sync");
-    // the side streams and events of the lanes' fork/join
+    // The lanes are the streams that the first members own (made with each context), and the
+    // events of their fork and join.  Streams of the batch's own cost a batch of 64 members of
+    // 11x21x41 1.2 ms more at creation and 1.3 ms more at its end, and a server makes a batch
+    // whenever its members change.
     if (st == ATHAD_OK) st = bcuda(b, cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "batch events");
     const int ns = std::min(n, kSideStreams);
     for (int q = 0; q < ns && st == ATHAD_OK; q++) {
-        cudaStream_t s = nullptr;
         cudaEvent_t e = nullptr;
-        st = bcuda(b, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "batch side stream");
-        if (st == ATHAD_OK) b->side.push_back(s);
-        if (st == ATHAD_OK) st = bcuda(b, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "batch events");
-        if (st == ATHAD_OK) b->join.push_back(e);
+        st = bcuda(b, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "batch events");
+        if (st == ATHAD_OK) { b->join.push_back(e); b->side.push_back(members[q]->own_stream); }
     }
     if (st != ATHAD_OK) {
-        for (cudaStream_t s : b->side) cudaStreamDestroy(s);
         for (cudaEvent_t e : b->join) cudaEventDestroy(e);
         if (b->fork) cudaEventDestroy(b->fork);
         cudaFree(b->d_step); cudaStreamDestroy(b->own_stream); delete b;
@@ -277,9 +279,8 @@ athad_status athad_batch_create(athad_ctx* const* members, int32_t n_members, co
 athad_status athad_batch_destroy(athad_batch* b)
 {
     if (!b) return ATHAD_ERR_INVALID;
-    cudaStreamSynchronize(b->stream);
+    cudaStreamSynchronize(b->stream);   // the lanes have joined it (the members may be gone)
     drop_graphs(b);
-    for (cudaStream_t s : b->side) { cudaStreamSynchronize(s); cudaStreamDestroy(s); }
     for (cudaEvent_t e : b->join) cudaEventDestroy(e);
     if (b->fork) cudaEventDestroy(b->fork);
     cudaFree(b->d_step);

@@ -190,3 +190,39 @@ def test_configuration4_members_in_the_mix_equal_members_alone():
             assert np.isfinite(mix[n]).all(), (s.grid, n)
             assert np.array_equal(mix[n], a), (s.grid, n)
         g.close()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_more_members_than_lanes_equal_members_alone(graph):
+    """36 members, so that some follow one another on a lane, of several grids and at different
+    iterations of the cadence, one of them inactive: every member's state is that of the same
+    iterations on it alone."""
+    grids = [(4, 5, 5), (11, 21, 41), (9, 13, 20)]
+    n, steps, idle = 36, 24, 33
+    first = [1 + q % 4 for q in range(n)]
+    ms = [member(grids[q % 3], 500 + q % 6) for q in range(n)]
+    with GpuBatch(ms, first_iter=first) as b:
+        b.set_active(idle, False)
+        for _ in range(steps):
+            b.iteration(graph=graph)
+        b.synchronize()
+        assert [b.member_iter(q) for q in range(n)] == [f + (0 if q == idle else steps) for q, f in enumerate(first)]
+    alone = {}
+    for q in range(n):
+        key = (q % 3, 500 + q % 6, first[q], 0 if q == idle else steps)
+        if key not in alone:
+            alone[key] = alone_api(grids[key[0]], *key[1:])
+        for name in CHECK:
+            assert np.array_equal(ms[q].download(name), alone[key][name]), (q, name)
+        ms[q].close()
+
+
+def test_batch_outlives_its_members():
+    """Members closed before their batch: the batch still ends without touching them."""
+    ms = [member(GRIDS[0], 600 + q) for q in range(2)]
+    b = GpuBatch(ms)
+    b.iteration()
+    b.synchronize()
+    for m in ms:
+        m.close()
+    b.close()
