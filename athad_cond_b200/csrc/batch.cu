@@ -55,7 +55,9 @@ __global__ void batch_advance_kernel(BatchStep* step, int n)
 
 namespace {
 
+// a cadence pattern: how often it ran without a graph, then its graph
 struct GraphEntry {
+    int uses = 0;
     cudaGraphExec_t exec = nullptr;
 };
 
@@ -65,6 +67,16 @@ struct GraphEntry {
 // 11x21x41 3.73, 2.53, 2.00, 1.76 ms; 16 of 15x61x109 4.52, 4.14, 3.81, 3.80; twelve of
 // 27x99x151 11.6, 11.2, 10.9, 11.0.
 constexpr int kSideStreams = 32;
+
+// A pattern is captured when it comes for the kCaptureAt-th time.  The graph of an iteration of
+// 33 or more members takes 2 ms to instantiate and 2 to end (60 us a lane each), a batch has three
+// or four of them, and a server drops them whenever its members change: every twenty iterations
+// or so with 64 runs of a thousand.  A replay saves 0.5 ms per iteration of 33 members of
+// 11x21x41.  A batch of them made, run and closed, for kCaptureAt = 1, 2, 4, 8: 4 iterations 15,
+// 8.3, 4.9 and 4.7 ms, 8 iterations 17, 18, 12 and 8.2, 16 iterations 26, 22, 28 and 19, 40
+// iterations 33, 35, 38 and 41, 120 iterations 72, 71, 74 and 99.  Members of 27x99x151 and more
+// keep the GPU busy while the host captures.
+constexpr int kCaptureAt = 8;
 
 struct athad_batch {
     std::vector<athad_ctx*> m;
@@ -173,6 +185,29 @@ static athad_status enqueue_iteration(athad_batch* b)
     if (s != ATHAD_OK) return s;
     batch_advance_kernel<<<(n + 127) / 128, 128, 0, b->stream>>>(b->d_step, n);
     return bcuda(b, cudaGetLastError(), "batch advance");
+}
+
+// Whether a caller captures the batch's stream: a graph cannot be captured then.
+static bool capturing(const athad_batch* b)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(b->stream, &c) != cudaSuccess) { cudaGetLastError(); return false; }
+    return c != cudaStreamCaptureStatusNone;
+}
+
+// What enqueue() puts on b->stream, as a graph.
+template <class F> static athad_status capture(athad_batch* b, F enqueue, cudaGraphExec_t* exec)
+{
+    cudaGraph_t graph = nullptr;
+    athad_status s = bcuda(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+    if (s != ATHAD_OK) return s;
+    s = enqueue();
+    const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
+    if (s == ATHAD_OK) s = bcuda(b, e, "end capture");
+    if (s == ATHAD_OK) s = bcuda(b, cudaGraphInstantiate(exec, graph, 0), "instantiate");
+    if (s != ATHAD_OK) *exec = nullptr;
+    if (graph) cudaGraphDestroy(graph);
+    return s;
 }
 
 static std::vector<uint8_t> graph_key(const athad_batch* b)
@@ -342,21 +377,13 @@ athad_status athad_batch_iteration_graph(athad_batch* b)
     auto it = b->graphs.find(key);
     if (it == b->graphs.end()) {
         if (b->graphs.size() >= 16) drop_graphs(b);
-        cudaGraph_t graph = nullptr;
-        athad_status s = bcuda(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-        if (s != ATHAD_OK) return s;
-        athad_status se = enqueue_iteration(b);
-        cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
-        if (se != ATHAD_OK) { if (graph) cudaGraphDestroy(graph); return se; }
-        s = bcuda(b, ee, "end capture");
-        if (s != ATHAD_OK) return s;
-        GraphEntry g;
-        s = bcuda(b, cudaGraphInstantiate(&g.exec, graph, 0), "instantiate");
-        cudaGraphDestroy(graph);
-        if (s != ATHAD_OK) return s;
-        it = b->graphs.emplace(key, g).first;
+        it = b->graphs.emplace(key, GraphEntry()).first;
     }
-    athad_status s = bcuda(b, cudaGraphLaunch(it->second.exec, b->stream), "graph launch");
+    GraphEntry& g = it->second;
+    if (!g.exec && ++g.uses < kCaptureAt && !capturing(b)) return athad_batch_iteration(b);
+    athad_status s = ATHAD_OK;
+    if (!g.exec) s = capture(b, [b] { return enqueue_iteration(b); }, &g.exec);
+    if (s == ATHAD_OK) s = bcuda(b, cudaGraphLaunch(g.exec, b->stream), "graph launch");
     if (s == ATHAD_OK) advance_host(b);
     return s;
 }

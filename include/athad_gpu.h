@@ -620,8 +620,9 @@ athad_status athad_batch_member_iter(const athad_batch* b, int32_t member, int32
 athad_status athad_batch_set_active(athad_batch* b, int32_t member, int32_t active);
 /* One model iteration of every active member (cadence of cAtmosphereModel.cpp:1156-1509). */
 athad_status athad_batch_iteration(athad_batch* b);
-/* The same iteration replayed from a CUDA graph, captured on first use for the current
- * cadence pattern of the members (at most a few per batch). */
+/* The same iteration replayed from a CUDA graph, captured when the current cadence pattern of
+ * the members (at most a few per batch) comes for the eighth time and launched without one
+ * until then. */
 athad_status athad_batch_iteration_graph(athad_batch* b);
 /* Tile shapes of the members' RK4 stage kernels; athad_batch_autotune times RK4 stages 1-3 of
  * the whole batch once per shape (reps repetitions, model state unchanged), keeps the

@@ -198,7 +198,7 @@ def test_more_members_than_lanes_equal_members_alone(graph):
     iterations of the cadence, one of them inactive: every member's state is that of the same
     iterations on it alone."""
     grids = [(4, 5, 5), (11, 21, 41), (9, 13, 20)]
-    n, steps, idle = 36, 24, 33
+    n, steps, idle = 36, 36, 33   # every pattern of the cadence nine times: the last is a graph's replay
     first = [1 + q % 4 for q in range(n)]
     ms = [member(grids[q % 3], 500 + q % 6) for q in range(n)]
     with GpuBatch(ms, first_iter=first) as b:
