@@ -418,11 +418,18 @@ athad_status athad_batch_autotune(athad_batch* b, int32_t reps, int32_t* best_sh
                 return r;
             });
         };
-        s = stages();
+        // Replays of a graph, as iterations run: launched one by one, the stages of many small
+        // members take the host longer than the GPU, whatever the shape.
+        // A stream that cannot be captured (the legacy one) runs them one by one.
+        cudaGraphExec_t exec = nullptr;
+        if (capture(b, stages, &exec) != ATHAD_OK) cudaGetLastError();
+        auto once = [&] { return exec ? bcuda(b, cudaGraphLaunch(exec, b->stream), "autotune") : stages(); };
+        s = once();
         cudaEventRecord(e0, b->stream);
-        for (int r = 0; r < reps && s == ATHAD_OK; r++) s = stages();
+        for (int r = 0; r < reps && s == ATHAD_OK; r++) s = once();
         cudaEventRecord(e1, b->stream);
         if (s == ATHAD_OK) s = bcuda(b, cudaEventSynchronize(e1), "autotune");
+        if (exec) cudaGraphExecDestroy(exec);
         float ms = 0.0f;
         if (s == ATHAD_OK) s = bcuda(b, cudaEventElapsedTime(&ms, e0, e1), "autotune time");
         ms /= (float)reps;

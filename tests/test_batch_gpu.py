@@ -226,3 +226,23 @@ def test_batch_outlives_its_members():
     for m in ms:
         m.close()
     b.close()
+
+
+def test_autotune_times_the_stages_as_iterations_run_them():
+    """Many small members: three of an iteration's four RK4 stages take no longer than the whole
+    replayed iteration, so that what is compared is the stages and not their launches."""
+    import time
+    ms = [member((5, 9, 17), 700 + q) for q in range(40)]
+    with GpuBatch(ms) as b:
+        _, times = b.autotune(reps=10)
+        for _ in range(36):       # every pattern of the cadence has its graph
+            b.iteration(graph=True)
+        b.synchronize()
+        t0 = time.perf_counter()
+        for _ in range(16):
+            b.iteration(graph=True)
+        b.synchronize()
+        iteration_ms = (time.perf_counter() - t0) / 16 * 1e3
+    for m in ms:
+        m.close()
+    assert min(times) < iteration_ms, (times, iteration_ms)
