@@ -139,7 +139,11 @@ __global__ void __launch_bounds__(128) radial_columns_kernel(FilterArgs a)
 // moist iteration, one at a time and up to eleven: 21x91x181 262 and 73 us, 41x181x361 483
 // and 396, 61x181x361 607 and 575.  Limiting a launch to what the L2 holds with its scratch
 // is no better (41x181x361, four fields: 417).
-constexpr int kWalk = 8;
+// Rows (levels) per thread: on a small grid a walk is the launch's length.  One field with 2, 4
+// and 8: 11x21x41 5.8, 6.7 and 9.7 us (8.1 with the passes as separate cells), 21x91x181 6.3, 7.4
+// and 10.6, 41x181x361 20.9, 16.7 and 18.6; eleven fields of 27x99x151 36.9, 27.5 and 26.5, of
+// 41x181x361 215, 178 and 176.
+constexpr int kWalk = 4;
 
 // the zonal pass (periodic) of the longitudes k, k + 1 of one row; k is even, and the second
 // value is not used where k + 1 = km
