@@ -216,9 +216,16 @@ void launch_columns(const RadArgs& a, double omega, cudaStream_t st)
 {
     const dim3 grid((a.d.km + 31) / 32, a.d.jm);
     const size_t mem = 3 * 32 * sizeof(double) * (size_t)a.d.im;
-    // columns of up to 288 layers fit the 227 KB of a CTA (with the path sums)
-    constexpr size_t kMost = 3 * 32 * sizeof(double) * 288;
-    if (mem <= kMost) {
+    // Columns of up to 288 layers fit the 227 KB of a CTA (with the path sums), and of up to 145
+    // two CTAs fit an SM.  Above that one CTA is left on an SM, seven of its warps wait for the
+    // eighth, and the columns in the fields, of which many CTAs run on an SM, are faster unless
+    // the SMs have no second CTA to run.  Shared memory and fields, us per call: 181 x 361
+    // columns 189 and 329 (61 layers), 774 and 893 (140), 1502 and 992 (150), 2849 and 2486
+    // (288); 91 x 181 42 and 86, 197 and 258, 402 and 279, 761 and 671; 30 x 61 (60 CTAs) 37 and
+    // 56, 79 and 142, 84 and 150, 156 and 375.
+    constexpr size_t kMost = 3 * 32 * sizeof(double) * 288, kTwoPerSM = 3 * 32 * sizeof(double) * 145;
+    const bool few = (size_t)grid.x * grid.y <= 148;
+    if (mem <= (few ? kMost : kTwoPerSM)) {
         // the kernel's limit is the process's: every caller sets the same one, so that a thread
         // with lower columns cannot lower it between another's call and its launch
         if (mem > 40960)

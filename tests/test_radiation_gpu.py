@@ -134,3 +134,17 @@ def test_contexts_of_other_heights_on_other_threads():
     for q in range(2):
         for n in want[q]:
             assert np.array_equal(got[q][n], want[q][n]), (grids[q], n)
+
+
+@pytest.mark.parametrize("grid", [(145, 75, 41), (146, 75, 41), (146, 74, 41), (288, 5, 37), (289, 5, 37)])
+def test_columns_at_the_edges_of_shared_memory(grid):
+    """The tallest columns of which two CTAs fit an SM, the next with more CTAs than SMs and with
+    as many, and the tallest that fit at all, with the next."""
+    st = state(grid, 87)
+    o = OracleState(st, config_params())
+    with GpuAtmosphere(*grid, config_params()) as g:
+        g.upload_state(st)
+        g.radiative_heating(0.05)
+        o.radiative_heating(0.05)
+        for n in ("t", "radiation", "epsilon"):
+            assert close(g.download(n), o.f[n]) <= 1e-12, n
