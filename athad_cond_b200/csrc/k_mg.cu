@@ -556,7 +556,8 @@ __global__ void __launch_bounds__(128) mg_store_kernel(Dims d, const double* __r
 struct MGLevel {
     int ni = 0, nj = 0, nk = 0, pitch = 0;
     long long plane = 0, n = 0;
-    float* e = nullptr; float* f = nullptr; float* r = nullptr;
+    float* e = nullptr; float* f = nullptr;
+    float* r = nullptr;         // the right-hand sides of columns too tall for shared memory
     float* coef = nullptr;      // diag, ci, cj (3 per (i,j)), ck, cs (1 per (i,j)), tm, tc (3 per (i,j))
     OpView<float> op{};
     float* tm = nullptr; float* tc = nullptr;
@@ -592,6 +593,10 @@ void mg_free(MGSolver* s)
 namespace {
 
 inline long long rup(long long v, long long a) { return (v + a - 1) / a * a; }
+
+// the staged right-hand sides and factors of a smoother CTA; columns of up to 250 levels
+inline size_t smooth_smem(const MGLevel& L) { return (size_t)(32 + 17) * L.ni * sizeof(float); }
+inline bool smooth_fits(const MGLevel& L) { return smooth_smem(L) <= 48 * 1024; }
 
 // Galerkin coarsening of a level's coefficients (host, FP64): 2 x 2 aggregates in (j, k)
 void coarsen(int ni, int nj, int nk, const std::vector<double>& D, const std::vector<double>& CI,
@@ -729,7 +734,7 @@ MGSolver* mg_build(athad_ctx* ctx, std::string& err)
         L.n = (long long)L.ni * L.plane;
         off_e[l] = add(L.n * sizeof(float));
         off_f[l] = add(L.n * sizeof(float));
-        off_r[l] = add(L.n * sizeof(float));
+        off_r[l] = add(smooth_fits(L) ? 0 : L.n * sizeof(float));
         off_c[l] = add((size_t)L.ni * L.nj * (3 * 5 + 2) * sizeof(float));
     }
     const MGLevel& L0 = s->L[0];
@@ -750,7 +755,7 @@ MGSolver* mg_build(athad_ctx* ctx, std::string& err)
         MGLevel& L = s->L[l];
         L.e = (float*)(s->mem + off_e[l]);
         L.f = (float*)(s->mem + off_f[l]);
-        L.r = (float*)(s->mem + off_r[l]);
+        L.r = smooth_fits(L) ? nullptr : (float*)(s->mem + off_r[l]);
         L.coef = (float*)(s->mem + off_c[l]);
         const size_t m3 = (size_t)L.ni * L.nj * 3, m1 = (size_t)L.ni * L.nj;
         std::vector<float> buf(m3 * 5 + m1 * 2);
@@ -793,10 +798,6 @@ namespace {
 
 inline dim3 cells_grid(int nk, int nj, int ni) { return dim3((nk + 127) / 128, nj, ni); }
 inline dim3 rows_grid(const MGLevel& L) { return dim3((L.nk + 127) / 128, (L.nj + kRows - 1) / kRows, L.ni); }
-
-// the staged right-hand sides and factors of a smoother CTA; columns of up to 250 levels
-inline size_t smooth_smem(const MGLevel& L) { return (size_t)(32 + 17) * L.ni * sizeof(float); }
-inline bool smooth_fits(const MGLevel& L) { return smooth_smem(L) <= 48 * 1024; }
 
 // Warps of a smoother CTA.  Only its first warp has work in the recurrences, so where the
 // CTAs fill the SMs several times over (the fine levels) four warps keep more columns in them
