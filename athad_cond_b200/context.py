@@ -346,8 +346,8 @@ class GpuAtmosphere:
 class GpuBatch:
     """An ensemble of mixed-precision GpuAtmosphere members advanced together
     (athad_batch_* of include/athad_gpu.h): per iteration, each member's column physics at
-    its own cadence, level mean and RK4 stages, the members side by side on streams of the
-    batch."""
+    its own cadence, level mean and RK4 stages, the members side by side on their own
+    streams."""
 
     def __init__(self, members: list, dt: float = 4e-5, diffusion_ramp: float = 1.0,
                  buoyancy_ramp_iters: int = 300, first_iter: list | None = None):

@@ -22,8 +22,9 @@ namespace athad {
 // ---------------------------------------------------------------------------------------
 // computeLevelMeanTemperature (RungeKutta_Atm_Turb.cpp:24-41).  Row sums first, one warp
 // per (i, j) row over all SMs: a 32-lane strided partial sum reduced by xor butterfly; then
-// one CTA per level stages its row sums in shared memory (jm <= 6144) and one thread adds
-// rows j and jm-1-j before weighting, so the mean of a mirrored field is identical.
+// one CTA per level stages its row sums in shared memory (jm <= 6144), adds rows j and jm-1-j
+// before weighting them, so the mean of a mirrored field is identical, and two lanes add the
+// terms.
 // The same pass counts the non-finite values of t (nonfinite, may be null): a row whose sum
 // is finite holds none, so only rows with a non-finite sum are scanned.
 __global__ void __launch_bounds__(256) level_rows_kernel(Dims d, const double* __restrict__ t,

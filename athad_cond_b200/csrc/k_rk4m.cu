@@ -17,7 +17,7 @@
 // FP32 level n have the same groups; their fourth place of group 0 carries nue and MC_v's
 // source.  Separate FP32 arrays per field made stages 2 and 3 issue-limited: 140 M warp
 // instructions and 205 us each at 41x181x361, now 113 M and 135 us, the step 1042 -> 848 us
-// (785 us with prefetch_tile); the results are the same bits.
+// (809 with prefetch_tile, 785 with each stage's own registers); the results are the same bits.
 //
 // Forcing packing: the reference's RHS reads 15 per-cell forcing fields (p_dyn, nue, t_eq,
 // p_stat, r_humid, S_c..S_v, MC_t..MC_w) in every stage.  Stage 1 reads them in FP64 and

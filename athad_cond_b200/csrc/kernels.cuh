@@ -152,11 +152,10 @@ struct PoissonArgs {
     double ceiling;
 };
 void launch_poisson_prepare(const PoissonArgs& a, cudaStream_t st);   // aux BC + source field
-void launch_poisson_sweep(const PoissonArgs& a, cudaStream_t st);
+void launch_poisson_sweep(const PoissonArgs& a, cudaStream_t st);     // source, colours, BCs, ceiling
 // n_sweeps sweeps with p and the source in two scratch fields (where it pays)
 bool poisson_sweeps_split(const Dims& d, int n_sweeps);
-void launch_poisson_sweeps_split(const PoissonArgs& a, int n_sweeps, double* ps, double* ss, cudaStream_t st);     // colours (with their
-                                                                      // sources) + BCs + ceiling
+void launch_poisson_sweeps_split(const PoissonArgs& a, int n_sweeps, double* ps, double* ss, cudaStream_t st);
 void launch_poisson_bcs(const PoissonArgs& a, cudaStream_t st);       // BCs only
 void launch_project_correct(const PoissonArgs& a, double* u, double* v, double* w, cudaStream_t st);
 

@@ -589,7 +589,7 @@ athad_status athad_get_report(athad_ctx* ctx, athad_report* out);
  * mixed-precision contexts (members, each with its own grid and parameters) together in the
  * order of one stream: every member's column physics at its own cadence, level mean and RK4
  * stages, the time-level copy (storeIntermediateData3D) fused into the last, side by side
- * on streams of the batch that fork from that stream and join it again.  The members stay
+ * on the contexts' own streams, which fork from that stream and join it again.  The members stay
  * ordinary contexts: upload/download work on them between batch calls (on the batch's
  * stream order: call athad_batch_synchronize first).  A member's result is bit-for-bit
  * the result of the same iterations run on it alone through athad_rk4_step and friends

@@ -1,11 +1,13 @@
 """Batched ensembles (athad_batch_*): members of uneven grids advanced together.
 
-The batched kernels run the per-cell code of the single-grid mixed-precision step on every
-member, so each member's result must be bit-for-bit what the same iterations give on that
-member alone: through a batch of one (the serving path of a request run alone), and
-through the single-context entry points with the same scalars (the mixed-precision kernels
-are compiled without fused multiply-add, so both kernels round every operation alike).  Covered: uneven grids, members at different iteration numbers (different
-cadence phases), the CUDA-graph replay, every tile shape of the autotuner, inactive members.
+Each member runs the kernels of the single-grid mixed-precision step side by side with the
+others, on a stream of its own or after another member on one, so its result must be bit-for-bit
+what the same iterations give on that member alone: through a batch of one (the serving path
+of a request run alone), and through the single-context entry points with the same scalars (the
+mixed-precision kernels are compiled without fused multiply-add, so every tile shape rounds
+alike).  Covered: uneven grids, members at different iteration numbers (different cadence
+phases), more members than streams, the CUDA-graph replay, every tile shape of the autotuner,
+inactive members.
 """
 import numpy as np
 import pytest

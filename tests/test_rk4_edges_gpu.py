@@ -1,9 +1,9 @@
 """The RK4 step of both precisions on the smallest grid and on ragged ones.
 
-The stage kernels work on tiles of 128 (FP64: 4 CTAs of 128, mixed: 128 x 1 and a batch's
-five other shapes) with operands staged or prefetched by the tile, so the rows that end
-inside a tile, just after one, and the grids with a single interior cell per column are
-where an index can go wrong.  Tolerances, from the states and forces of one step on the
+The stage kernels work on tiles of 128 cells (FP64 32 x 4, mixed 128 x 1) with operands staged
+or prefetched by the tile, so the rows that end inside a tile, just after one, and the smallest
+grid, with two interior levels, are where an index can go wrong.  A batch's other tile shapes
+are test_batch_gpu.py's.  Tolerances, from the states and forces of one step on the
 grids of test_parity_gpu.py and test_mixed_gpu.py: FP64 1e-12; mixed 1e-8 for the
 prognostic fields and 1e-4 for the acting forces.  The time-level copy is exact.
 """
