@@ -248,10 +248,12 @@ ATHAD_HD double x_H2O_of(double c, double co2, double M_b)
 
 // SaturationH2O::dewPoint (SaturationH2O.h:189-202): bisection of the saturation curve
 // (liquid above the triple point, ice below) on [150 K, T_crit], 60 halvings
-// ln p_sat of saturation_pressure_auto and T d ln p_sat / dT, for the dew point's Newton
-// step: the Wagner-Pruss line above the triple point (ln p = ln p_c + (T_c/T) S(theta)), the
-// IAPWS sublimation curve below it (ln p = ln p_t + sum b_i vartheta^(m_i) / vartheta)
-ATHAD_HD void ln_sat(double T, double& ln_p, double& T_dln_p)
+// f = ln p_sat - ln e of saturation_pressure_auto and T d ln p_sat / dT, for the dew point's
+// Newton step: the Wagner-Pruss line above the triple point (ln p = ln p_c + (T_c/T) S(theta)),
+// the IAPWS sublimation curve below it (ln p = ln p_t + sum b_i vartheta^(m_i) / vartheta).  On
+// the first the pressure is measured from p_c, and the rounding error of ln p_c is added: alone
+// it moves the root by half an ulp.
+ATHAD_HD void ln_sat(double T, double ln_e, double& f, double& T_dln_p)
 {
     if (T >= T_TRIPLE) {
         const double theta = 1.0 - T / T_CRIT;
@@ -262,7 +264,7 @@ ATHAD_HD void ln_sat(double T, double& ln_p, double& T_dln_p)
         const double dS = -7.85951783 + 1.5 * 1.84408259 * sq + 3.0 * -11.7866497 * t2
                         + 3.5 * 22.6807411 * t2 * sq + 4.0 * -15.9618719 * t3 + 7.5 * 1.80122502 * t3 * t3 * sq;
         const double cS = (T_CRIT / T) * S;
-        ln_p = 12.30428769302713 + cS;            // ln 220640
+        f = (cS - (ln_e - 12.30428769302713)) - 7.019913681514128e-16;   // ln 220640
         T_dln_p = -cS - dS;
         return;
     }
@@ -270,7 +272,7 @@ ATHAD_HD void ln_sat(double T, double& ln_p, double& T_dln_p)
     const double lt = log(th), inv_th = 1.0 / th;
     const double a0 = -0.212144006e2 * exp(0.333333333e-2 * lt), a1 = 0.273203819e2 * exp(0.120666667e1 * lt),
                  a2 = -0.610598130e1 * exp(0.170333333e1 * lt);
-    ln_p = 1.8110014818928741 + (a0 + a1 + a2) * inv_th;   // ln 6.11657
+    f = (1.8110014818928741 + (a0 + a1 + a2) * inv_th) - ln_e;   // ln 6.11657
     T_dln_p = ((0.333333333e-2 - 1.0) * a0 + (0.120666667e1 - 1.0) * a1 + (0.170333333e1 - 1.0) * a2) * inv_th;
 }
 
@@ -292,9 +294,8 @@ ATHAD_HD double dew_point(double e)
     double T = 1.0 / (1.0 / T_TRIPLE - (ln_e - 1.8110014818928741) * (461.5 / 2.5e6));
     if (!(T > lo && T < hi)) T = 0.5 * (lo + hi);
     for (int it = 0; it < 60; it++) {
-        double ln_p, TD;
-        ln_sat(T, ln_p, TD);
-        const double f = ln_p - ln_e;
+        double f, TD;
+        ln_sat(T, ln_e, f, TD);
         if (f < 0.0) lo = T; else hi = T;
         double Tn = T - T * f / (TD + f);         // 1/Tn = 1/T + f / (T TD)
         if (fabs(Tn - T) <= 1.0e-12 && Tn >= lo && Tn <= hi) return Tn;   // converged
