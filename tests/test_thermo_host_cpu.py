@@ -18,8 +18,9 @@ import subprocess
 import numpy as np
 import pytest
 
-from thermo_checks import (DEW, check_against_the_oracle_over_the_model_range, check_mixture_and_lapse_known_answers,
-                           check_saturation_known_answers)
+from oracle_binding import lib as oracle_lib
+from thermo_checks import (DEW, DQ_DT, SUBL_P, check_against_the_oracle_over_the_model_range,
+                           check_mixture_and_lapse_known_answers, check_saturation_known_answers)
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
@@ -87,3 +88,15 @@ def test_dew_point_over_liquid_water_is_unbiased(host):
     ulps = (L(got) - T) / L(np.spacing(got))
     assert abs(float(np.mean(ulps))) <= 0.1, float(np.mean(ulps))
     assert float(np.max(np.abs(ulps))) <= 4.0
+
+
+def test_saturation_slope_at_vanishing_pressures(host):
+    """dq_sat/dT where the squares of the pressures underflow: the oracle's values, which are
+    formed from the ratio of the two pressures."""
+    T = np.linspace(14.0, 18.0, 41)
+    p = 10.0 * host(SUBL_P, T)
+    assert (p > 0.0).all() and (p * p == 0.0).any()
+    got = host(DQ_DT, T, p, 0.034)
+    want = np.array([oracle_lib().or_dqsat_dT(t, q, 0.034) for t, q in zip(T, p)])
+    assert np.isfinite(want).all() and (want > 0.0).all()
+    assert (np.abs(got - want) <= 1e-11 * want).all()
