@@ -65,7 +65,8 @@ struct GraphEntry {
 
 // Lanes of a batched iteration.  Four iterations with 4, 8, 16, 32 lanes: 32 members of
 // 11x21x41 3.73, 2.53, 2.00, 1.76 ms; 16 of 15x61x109 4.52, 4.14, 3.81, 3.80; twelve of
-// 27x99x151 11.6, 11.2, 10.9, 11.0.
+// 27x99x151 11.6, 11.2, 10.9, 11.0.  More members than lanes, replayed, with 8, 16, 32 lanes:
+// 64 of 11x21x41 5.01, 4.19, 3.62.
 constexpr int kSideStreams = 32;
 
 // A pattern is captured when it comes for the kCaptureAt-th time.  The graph of an iteration of

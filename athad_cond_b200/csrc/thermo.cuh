@@ -29,9 +29,10 @@ constexpr double R_CO2 = R_STAR / M_CO2;
 // and now: heat capacity 0.70 and 0.70 ulp, molar mass 0.50 and 0.49, mass fraction 0.72 and
 // 0.66).  saturation_mass_fraction of M_nonwater's
 // mixture at a temperature takes 4 divisions instead of 9, cp_of 1 instead of 6, the moist
-// lapse rate 2 instead of 5.  At 41x181x361: saturation adjustment 655 -> 607 us, convection
+// lapse rate 3 instead of 5.  At 41x181x361: saturation adjustment 655 -> 607 us, convection
 // 1232 -> 1136 (with the entrainment gradients, and with product forms of its own that cost
-// accuracy and were taken out again: 1170), ice 254 -> 235, densities 175 -> 140.  The
+// accuracy and were taken out again: 1170), ice 254 -> 235, densities 175 -> 140 (133 -> 135
+// with the derivative factor by E / p again).  The
 // two saturation curves keep their quotients: their exponent multiplies an ulp in theta by 30.
 
 // Wagner & Pruss saturation line (SaturationH2O.h:68-93)
