@@ -188,12 +188,14 @@ static athad_status enqueue_iteration(athad_batch* b)
     return bcuda(b, cudaGetLastError(), "batch advance");
 }
 
-// Whether a caller captures the batch's stream: a graph cannot be captured then.
-static bool capturing(const athad_batch* b)
+// Whether the batch's stream can be captured: not while a caller captures it, and not the legacy
+// stream.
+static bool capturable(const athad_batch* b)
 {
+    if (b->stream == cudaStreamLegacy) return false;
     cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(b->stream, &c) != cudaSuccess) { cudaGetLastError(); return false; }
-    return c != cudaStreamCaptureStatusNone;
+    return c == cudaStreamCaptureStatusNone;
 }
 
 // What enqueue() puts on b->stream, as a graph.
@@ -201,12 +203,12 @@ template <class F> static athad_status capture(athad_batch* b, F enqueue, cudaGr
 {
     cudaGraph_t graph = nullptr;
     athad_status s = bcuda(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-    if (s != ATHAD_OK) return s;
+    if (s != ATHAD_OK) { cudaGetLastError(); return s; }   // the next launch's check must not see it
     s = enqueue();
     const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
     if (s == ATHAD_OK) s = bcuda(b, e, "end capture");
     if (s == ATHAD_OK) s = bcuda(b, cudaGraphInstantiate(exec, graph, 0), "instantiate");
-    if (s != ATHAD_OK) *exec = nullptr;
+    if (s != ATHAD_OK) { cudaGetLastError(); *exec = nullptr; }
     if (graph) cudaGraphDestroy(graph);
     return s;
 }
@@ -381,7 +383,8 @@ athad_status athad_batch_iteration_graph(athad_batch* b)
         it = b->graphs.emplace(key, GraphEntry()).first;
     }
     GraphEntry& g = it->second;
-    if (!g.exec && ++g.uses < kCaptureAt && !capturing(b)) return athad_batch_iteration(b);
+    // a stream that cannot be captured is refused from the first use on
+    if (!g.exec && ++g.uses < kCaptureAt && capturable(b)) return athad_batch_iteration(b);
     athad_status s = ATHAD_OK;
     if (!g.exec) s = capture(b, [b] { return enqueue_iteration(b); }, &g.exec);
     if (s == ATHAD_OK) s = bcuda(b, cudaGraphLaunch(g.exec, b->stream), "graph launch");
@@ -423,7 +426,7 @@ athad_status athad_batch_autotune(athad_batch* b, int32_t reps, int32_t* best_sh
         // members take the host longer than the GPU, whatever the shape.
         // A stream that cannot be captured (the legacy one) runs them one by one.
         cudaGraphExec_t exec = nullptr;
-        if (capture(b, stages, &exec) != ATHAD_OK) cudaGetLastError();
+        (void)capture(b, stages, &exec);
         auto once = [&] { return exec ? bcuda(b, cudaGraphLaunch(exec, b->stream), "autotune") : stages(); };
         s = once();
         cudaEventRecord(e0, b->stream);

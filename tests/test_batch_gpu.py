@@ -248,3 +248,20 @@ def test_autotune_times_the_stages_as_iterations_run_them():
     for m in ms:
         m.close()
     assert min(times) < iteration_ms, (times, iteration_ms)
+
+
+def test_graph_iteration_refuses_a_stream_it_cannot_capture():
+    """The legacy stream cannot be captured: the replayed iteration is refused at its first use
+    already, which runs without a graph on other streams, and no member advances."""
+    from athad_cond_b200 import AthadError
+    m = member(GRIDS[0], 800)
+    with GpuBatch([m]) as b:
+        b.set_stream(1)      # cudaStreamLegacy
+        with pytest.raises(AthadError):
+            b.iteration(graph=True)
+        assert b.member_iter(0) == 1
+        b.set_stream(None)
+        b.iteration(graph=True)
+        b.synchronize()
+        assert b.member_iter(0) == 2
+    m.close()
